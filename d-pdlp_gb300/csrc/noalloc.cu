@@ -11,12 +11,22 @@
 // flag) lives in the file-scope device array below, which every GPU that
 // loads this library holds until the process exits.
 //
-// It is a variant of the fused SpMV of the solver: tiles of kTile non-zeros
-// staged with coalesced loads, the rows starting in a tile folded from shared
-// memory; tiles are cut at fixed non-zero offsets, so no row plan has to be
-// built or stored.  A row that continues past its tile leaves one partial per
-// tile in the scratch array, and a second kernel adds them in tile order, so
-// the result is bitwise reproducible.
+// Tiles are cut at fixed non-zero offsets, so no row plan has to be built or
+// stored: a block loads its tile's columns and values with coalesced loads,
+// gathers x and leaves the products in shared memory; two of its warps look up
+// the rows that start in the tile meanwhile (32 row pointers a step); then a
+// thread adds each short row, and a warp each row (or piece of one) of more
+// than kShort products.  A row that continues past its tile leaves one partial
+// per tile in the scratch array, and a second kernel adds them in a fixed
+// order, so the result is bitwise reproducible.
+//
+// Bound by HBM for short rows and by the gathers of x for long ones.  Before,
+// a thread added each row from global memory, which a warp's longest row held
+// up, and a block's first row came from a 25-step serial search.  Measured,
+// through the entry point: 20M non-zeros with power-law columns 358 -> 166 us,
+// a transport matrix (5,000 entries a row) 1,287 -> 162 us (1.6 TB/s of
+// matrix and vectors), 20k non-zeros 35 -> 34 us, which is launches and the
+// read of the error flag.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -39,90 +49,159 @@ struct Scratch {
   double own[kMaxTiles];
   double in[kMaxTiles];
   int own_row[kMaxTiles];
-  int error;
+  int error[2];  // of this call, and of the next one (cleared by this one)
 };
 
 static __device__ __align__(256) Scratch g_scratch;
 
+constexpr int kShort = 32;  // products of a row that one thread adds
+
+// First r in [0, rows) with ptr[r] >= key, else rows, by a warp: each step
+// keeps the one of 33 parts that the answer is in.
 __device__ __forceinline__ int lower_bound_rows(const int *ptr, int rows, int key) {
-  int lo = 0, hi = rows;  // first r in [0, rows) with ptr[r] >= key, else rows
-  while (lo < hi) {
-    int mid = (lo + hi) >> 1;
-    if (ptr[mid] < key) lo = mid + 1;
-    else hi = mid;
+  const int lane = threadIdx.x & 31;
+  int lo = 0, hi = rows;  // the answer is in [lo, hi]
+  while (hi > lo) {
+    const long n = hi - lo;
+    const int at = lo + (int)(n * (lane + 1) / 33);
+    const unsigned below = __ballot_sync(0xffffffffu, at < hi && ptr[at] < key);
+    // a malformed (unsorted) ptr still ends: the interval shrinks every step
+    const int k = below ? 32 - __clz(below) : 0;  // probes 0 .. k - 1 taken as below
+    const int next_lo = k ? lo + (int)(n * k / 33) + 1 : lo;
+    const int next_hi = k < 32 ? min(hi, lo + (int)(n * (k + 1) / 33)) : hi;
+    lo = min(next_lo, hi);
+    hi = max(next_hi, lo);
   }
   return lo;
+}
+
+// Sum of sp[lo, hi) by a warp, in a fixed order; every lane returns it.
+__device__ __forceinline__ double warp_products(const double *sp, int lo, int hi) {
+  double s0 = 0.0, s1 = 0.0;
+  int i = lo + (int)(threadIdx.x & 31);
+  for (; i + 32 < hi; i += 64) {
+    s0 += sp[i];
+    s1 += sp[i + 32];
+  }
+  if (i < hi) s0 += sp[i];
+  return pdlp::warp_sum(s0 + s1);
 }
 
 __global__ void __launch_bounds__(pdlp::kThreads)
     k_spmv_tiles(int rows, int cols, int nnz, int ntiles, const int *__restrict__ ptr,
                  const int *__restrict__ col, const double *__restrict__ val,
-                 const double *__restrict__ x, double *__restrict__ y, Scratch *s) {
-  __shared__ double sv[kTile];
-  __shared__ double sx[kTile];
+                 const double *__restrict__ x, double *__restrict__ y, Scratch *s, int slot) {
+  constexpr int kPer = kTile / pdlp::kThreads;
+  __shared__ double sp[kTile];
   __shared__ int s_rows[2];
-  const int t = blockIdx.x;
+  const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int k0 = t * kTile;
   const int k1 = min(nnz, k0 + kTile);
   const int len = k1 > k0 ? k1 - k0 : 0;
-  // row pointers are validated over all rows (grid-stride), so a malformed
-  // CSR always raises the flag; every access below stays in bounds either way
-  for (long r = (long)t * pdlp::kThreads + threadIdx.x; r < rows;
-       r += (long)ntiles * pdlp::kThreads)
-    if (ptr[r] > ptr[r + 1]) atomicOr(&s->error, 1);
-  if (threadIdx.x == 0) {
-    if (t == 0 && (ptr[0] != 0 || ptr[rows] != nnz)) atomicOr(&s->error, 1);
-    s_rows[0] = t == 0 ? 0 : lower_bound_rows(ptr, rows, k0);
-    s_rows[1] = t == ntiles - 1 ? rows : lower_bound_rows(ptr, rows, k1);
+  int c[kPer];
+  double v[kPer];
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int i = tid + u * pdlp::kThreads;
+    if (i < len) {
+      c[u] = __ldcs(col + k0 + i);
+      v[u] = __ldcs(val + k0 + i);
+    }
+  }
+  if (warp < 2) {
+    const bool first = warp == 0;
+    int r = first ? 0 : rows;
+    if (first ? t > 0 : t < ntiles - 1) r = lower_bound_rows(ptr, rows, first ? k0 : k1);
+    if (lane == 0) s_rows[warp] = r;
+  }
+  if (tid == 0) {
+    if (t == 0 && (ptr[0] != 0 || ptr[rows] != nnz)) atomicOr(&s->error[slot], 1);
+    if (t == 0) s->error[slot ^ 1] = 0;
     s->own_row[t] = -1;  // set below by the row that runs past k1, if any
   }
-  for (int i = threadIdx.x; i < len; i += pdlp::kThreads) {
-    int c = col[k0 + i];
-    double xv = 0.0;
-    if (c >= 0 && c < cols) xv = x[c];
-    else atomicOr(&s->error, 2);  // bad column: flagged, never dereferenced
-    sv[i] = val[k0 + i];
-    sx[i] = xv;
+  // row pointers are validated over all rows (grid-stride), so a malformed
+  // CSR always raises the flag; every access below stays in bounds either way
+  for (long r = (long)t * pdlp::kThreads + tid; r < rows; r += (long)ntiles * pdlp::kThreads)
+    if (ptr[r] > ptr[r + 1]) atomicOr(&s->error[slot], 1);
+  bool bad = false;
+#pragma unroll
+  for (int u = 0; u < kPer; ++u) {
+    const int i = tid + u * pdlp::kThreads;
+    if (i < len) {
+      const bool in = c[u] >= 0 && c[u] < cols;
+      bad |= !in;  // flagged, never dereferenced
+      sp[i] = v[u] * (in ? __ldg(x + c[u]) : 0.0);
+    }
   }
+  if (bad) atomicOr(&s->error[slot], 2);
   __syncthreads();
   const int rA = s_rows[0], rB = s_rows[1];
   // rows starting in this tile; the one running past k1 leaves its partial
-  for (int r = rA + threadIdx.x; r < rB; r += pdlp::kThreads) {
-    int a = ptr[r], e = ptr[r + 1];
-    if (a > e || a < 0 || e > nnz) continue;  // flagged by the validation loop
-    int lo = max(a, k0) - k0, hi = min(e, k1) - k0;
+  for (int base = rA + 32 * warp; base < rB; base += pdlp::kThreads) {
+    const int r = base + lane;
+    int a = 0, e = 0;
+    bool live = r < rB;
+    if (live) {
+      a = ptr[r];
+      e = ptr[r + 1];
+      live = a <= e && a >= 0 && e <= nnz;  // else flagged by the validation loop
+    }
+    const int lo = max(a, k0) - k0, hi = min(e, k1) - k0;
     double sum = 0.0;
-    for (int i = lo; i < hi; ++i) sum = fma(sv[i], sx[i], sum);
-    if (e > k1) {
-      s->own[t] = sum;
-      s->own_row[t] = r;
-    } else {
-      y[r] = sum;
+    const bool wide = live && hi - lo > kShort;
+    if (live && !wide)
+      for (int i = lo; i < hi; ++i) sum += sp[i];
+    unsigned todo = __ballot_sync(0xffffffffu, wide);
+    while (todo) {
+      const int src = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const double w = warp_products(sp, __shfl_sync(0xffffffffu, lo, src),
+                                     __shfl_sync(0xffffffffu, hi, src));
+      if (lane == src) sum = w;
+    }
+    if (live) {
+      if (e > k1) {
+        s->own[t] = sum;
+        s->own_row[t] = r;
+      } else {
+        y[r] = sum;
+      }
     }
   }
   // partial of the row (started in an earlier tile) that runs into this one
-  if (threadIdx.x == 0) {
-    double inc = 0.0;
-    if (t > 0 && rA > 0) {
-      int end = min(ptr[rA], k1);  // row rA-1 ends where row rA starts
-      for (int i = 0; i < end - k0; ++i) inc = fma(sv[i], sx[i], inc);
-    }
-    s->in[t] = inc;
+  if (warp == pdlp::kThreads / 32 - 1) {
+    double in = 0.0;
+    if (t > 0 && rA > 0) in = warp_products(sp, 0, min(ptr[rA], k1) - k0);  // it ends where rA starts
+    if (lane == 0) s->in[t] = in;
   }
 }
 
 // y[r] for a row crossing tiles: its own partial plus the partials of the
-// tiles it runs into, added in tile order
+// tiles it runs into, in tile order (a warp's lanes take turns over more than
+// 32 of them)
 __global__ void k_spmv_tiles_fix(int ntiles, const int *__restrict__ ptr, double *__restrict__ y,
                                  const Scratch *__restrict__ s) {
-  int t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= ntiles) return;
-  int r = s->own_row[t];
-  if (r < 0) return;
-  double tot = s->own[t];
-  int end = ptr[r + 1];
-  for (int u = t + 1; u < ntiles && (long)u * kTile < end; ++u) tot += s->in[u];
-  y[r] = tot;
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+  int r = -1, count = 0;
+  if (t < ntiles) r = s->own_row[t];
+  if (r >= 0) {
+    const long end = ((long)ptr[r + 1] + kTile - 1) / kTile;  // first tile past the row
+    count = (int)max(0l, min((long)ntiles, end) - (t + 1));
+  }
+  double tot = r >= 0 ? s->own[t] : 0.0;
+  if (count <= 32)
+    for (int u = 1; u <= count; ++u) tot += s->in[t + u];
+  unsigned todo = __ballot_sync(0xffffffffu, count > 32);
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int n = __shfl_sync(0xffffffffu, count, src), from = __shfl_sync(0xffffffffu, t, src);
+    double w = 0.0;
+    for (int u = 1 + lane; u <= n; u += 32) w += s->in[from + u];
+    w = pdlp::warp_sum(w);
+    if (lane == src) tot += w;
+  }
+  if (r >= 0) y[r] = tot;
 }
 
 // Device address of the scratch array, per device.  Only a successful
@@ -130,6 +209,7 @@ __global__ void k_spmv_tiles_fix(int ntiles, const int *__restrict__ ptr, double
 // used) is tried again by the next call.
 constexpr int kMaxDevices = 64;
 Scratch *g_addr[kMaxDevices] = {};
+unsigned g_calls[kMaxDevices] = {};  // the error slot alternates
 std::mutex g_addr_mu;
 
 thread_local std::string g_err;
@@ -167,6 +247,7 @@ extern "C" int pdlp_spmv_noalloc(int rows, int cols, int nnz, const int *row_ptr
     return fail(-2, std::string("no usable CUDA device: ") + cudaGetErrorString(e));
   // set-up, once per device, with that device current
   Scratch *s = nullptr;
+  int slot = 0;
   {
     std::lock_guard<std::mutex> lk(g_addr_mu);
     if (!g_addr[dev]) {
@@ -179,22 +260,30 @@ extern "C" int pdlp_spmv_noalloc(int rows, int cols, int nnz, const int *row_ptr
       g_addr[dev] = (Scratch *)p;
     }
     s = g_addr[dev];
+    slot = (int)(g_calls[dev] & 1u);
   }
   cudaStream_t st = (cudaStream_t)stream;
-  // the error flag must start at zero; every other slot a call reads, the
-  // same call writes first
-  e = cudaMemsetAsync(&s->error, 0, sizeof(int), st);
-  if (e != cudaSuccess) return fail(-2, std::string("memset: ") + cudaGetErrorString(e));
+  // this call's error flag was cleared by the call before it (at first by the
+  // array's initialisation); every other slot a call reads, the same call
+  // writes first
   k_spmv_tiles<<<ntiles, pdlp::kThreads, 0, st>>>(rows, cols, nnz, ntiles, row_ptr, col_ind,
-                                                  vals, x, y, s);
-  k_spmv_tiles_fix<<<(ntiles + pdlp::kThreads - 1) / pdlp::kThreads, pdlp::kThreads, 0, st>>>(
-      ntiles, row_ptr, y, s);
+                                                  vals, x, y, s, slot);
+  if (ntiles > 1)  // no row leaves a single tile
+    k_spmv_tiles_fix<<<(ntiles + pdlp::kThreads - 1) / pdlp::kThreads, pdlp::kThreads, 0, st>>>(
+        ntiles, row_ptr, y, s);
   e = cudaGetLastError();
-  if (e != cudaSuccess) return fail(-2, std::string("launch: ") + cudaGetErrorString(e));
+  if (e != cudaSuccess) {
+    cudaMemsetAsync(s->error, 0, sizeof(s->error), st);  // the kernel that clears it did not run
+    return fail(-2, std::string("launch: ") + cudaGetErrorString(e));
+  }
   int flag = 0;
-  e = cudaMemcpyAsync(&flag, &s->error, sizeof(int), cudaMemcpyDeviceToHost, st);
+  e = cudaMemcpyAsync(&flag, &s->error[slot], sizeof(int), cudaMemcpyDeviceToHost, st);
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return fail(-2, std::string("sync: ") + cudaGetErrorString(e));
+  {
+    std::lock_guard<std::mutex> lk(g_addr_mu);
+    ++g_calls[dev];  // the kernel has run, so the other slot is clear
+  }
   if (flag & 2) return fail(-4, "column index out of range");
   if (flag & 1) return fail(-4, "malformed row pointers");
   return 0;

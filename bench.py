@@ -296,11 +296,8 @@ def run_ours(args, cp, rank, world, local):
     prec = {"fp32": cp.PRECISION_FP32_REFINE, "fp32m": cp.PRECISION_FP32_MATRIX,
             "fp64": cp.PRECISION_FP64}[args.precision]
     dp = cp.DeviceProblem(prob)
-    first_info = {}
     for i in range(args.warmup):
         out = dp.solve(params, precision=prec)
-        if i == 0:
-            first_info = out.info
     if world > 1:
         import torch.distributed as dist
         dist.barrier()
@@ -418,12 +415,8 @@ def run_ours(args, cp, rank, world, local):
                      "timing": timing,
                      "isolated_ms": {"primal_step": round(ms[0], 4), "dual_step": round(ms[1], 4),
                                      "eval_A": round(ms[2], 4), "eval_AT": round(ms[3], 4)}},
-        "spmv_kernels": {"A": ["fused", "pipelined"][out.info["spmv_kernel_A"]],
-                         "A^T": ["fused", "pipelined"][out.info["spmv_kernel_AT"]],
-                         "chosen_by": "timing both on the step kernels at the problem's first "
-                                      "solve (ms per launch: A fused, A pipelined, A^T fused, "
-                                      "A^T pipelined)",
-                         "tune_ms": [round(v, 4) for v in first_info.get("tune_ms", [])]},
+        "spmv_kernels": {"A": ["fused", "pipelined", "strip"][out.info["spmv_kernel_A"]],
+                         "A^T": ["fused", "pipelined", "strip"][out.info["spmv_kernel_AT"]]},
         "solve": {"status": r["status"], "iterations": iters, "power_iterations": pm_iters,
                   "rel_primal": r["relative_primal_residual"],
                   "rel_dual": r["relative_dual_residual"], "rel_gap": r["relative_objective_gap"],

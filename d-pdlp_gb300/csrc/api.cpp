@@ -274,6 +274,7 @@ cupdlpx_result_t *run_solve(const pdlp::DevProblem &P, const pdhg_parameters_t &
                             cudaStream_t st, double *trace, int trace_cap, int *trace_len,
                             pdlp_solve_info_t *info,
                             std::chrono::steady_clock::time_point t0) {
+  pdlp::SolveInFlight in_flight;
   pdlp::Solve<double> s(p, st, P, trace ? trace_cap : 0);
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   if (info) {
@@ -328,9 +329,8 @@ cupdlpx_result_t *run_solve(const pdlp::DevProblem &P, const pdhg_parameters_t &
     info->primal_step_ms = s.live_primal_ms();
     info->dual_step_ms = s.live_dual_ms();
     info->timed_chunks = s.live_samples();
-    info->spmv_kernel_A = s.pipe_A() ? 1 : 0;
-    info->spmv_kernel_AT = s.pipe_AT() ? 1 : 0;
-    for (int i = 0; i < 4; ++i) info->tune_ms[i] = s.tune_ms(i);
+    info->spmv_kernel_A = s.kernel_A();
+    info->spmv_kernel_AT = s.kernel_AT();
   }
   return r;
 }
@@ -339,6 +339,7 @@ cupdlpx_result_t *run_refined(const pdlp::DevProblem &P, const pdhg_parameters_t
                               const pdlp_options_t &o, cudaStream_t st,
                               pdlp_solve_info_t *info,
                               std::chrono::steady_clock::time_point t0) {
+  pdlp::SolveInFlight in_flight;
   pdlp::RefineOptions ro;
   if (o.max_refinements > 0) ro.max_rounds = o.max_refinements;
   ro.inner_eps = o.inner_eps;
@@ -369,7 +370,6 @@ cupdlpx_result_t *run_refined(const pdlp::DevProblem &P, const pdhg_parameters_t
     info->fp64_finish = rep.fp64_finish ? 1 : 0;
     info->spmv_kernel_A = rep.kernel_A;
     info->spmv_kernel_AT = rep.kernel_AT;
-    for (int q = 0; q < 4; ++q) info->tune_ms[q] = rep.tune_ms[q];
     if (rep.timed_chunks > 0) {
       info->primal_step_ms = rep.timed_primal_ms_sum / rep.timed_chunks;
       info->dual_step_ms = rep.timed_dual_ms_sum / rep.timed_chunks;
@@ -642,21 +642,50 @@ int pdlp_gpu_rescale(const lp_problem_t *prob, const pdhg_parameters_t *params, 
     pdlp::Solve<double> s(*params, sg.s, *P, 0);
     s.prepare();
     const pdlp::Dev<double> &d = s.dev();
-    const int n = d.n, m = d.m, nnz = s.A().nnz;
-    auto get = [&](double *dst, const double *src, int cnt) {
-      if (cnt > 0) {
-        PDLP_CUDA(cudaMemcpyAsync(dst, src, (size_t)cnt * 8, cudaMemcpyDeviceToHost, sg.s));
-        PDLP_CUDA(cudaStreamSynchronize(sg.s));
-      }
+    const int n = d.n, m = d.m;
+    auto fetch = [&](auto *dst, const auto *src, size_t cnt) {
+      if (cnt == 0) return;
+      PDLP_CUDA(cudaMemcpyAsync(dst, src, cnt * sizeof(*dst), cudaMemcpyDeviceToHost, sg.s));
+      PDLP_CUDA(cudaStreamSynchronize(sg.s));
     };
-    get(vals, s.A64().val, nnz);
-    get(c, d.c, n);
-    get(lv, d.lv, n);
-    get(uv, d.uv, n);
-    get(lc, d.lc, m);
-    get(uc, d.uc, m);
-    get(con, d.Dr, m);
-    get(var, d.Dc, n);
+    // vectors and values back in the caller's order
+    auto order = [&](const int *perm, int cnt) {
+      std::vector<int> o(cnt);
+      for (int i = 0; i < cnt; ++i) o[i] = i;
+      if (perm) fetch(o.data(), perm, cnt);
+      return o;
+    };
+    const std::vector<int> om = order(P->perm_m, m), on = order(P->perm_n, n);
+    auto get = [&](double *dst, const double *src, const std::vector<int> &o) {
+      std::vector<double> v(o.size());
+      fetch(v.data(), src, v.size());
+      for (size_t i = 0; i < o.size(); ++i) dst[o[i]] = v[i];
+    };
+    const pdlp::DevCsr &M = s.A64();
+    if (M.strip.on) {
+      std::vector<double> v(M.store());
+      fetch(v.data(), M.val, v.size());
+      std::vector<int> front(M.strip.nfront + 1), off(M.strip.nstrip + 1);
+      fetch(front.data(), M.ptr, front.size());
+      fetch(off.data(), M.strip.off, off.size());
+      const int *rp = prob->constraint_matrix_row_pointers;
+      for (int i = 0; i < m; ++i) {
+        const int r = om[i], q = i - M.strip.nfront, lg = M.strip.lg, H = 32 >> lg;
+        for (int k = 0; k < rp[r + 1] - rp[r]; ++k)
+          vals[rp[r] + k] =
+              q < 0 ? v[front[i] + k]
+                    : v[((size_t)off[q / H] + (k >> lg)) * 32 + ((q % H) << lg) + (k & ((1 << lg) - 1))];
+      }
+    } else {
+      fetch(vals, M.val, M.nnz);
+    }
+    get(c, d.c, on);
+    get(lv, d.lv, on);
+    get(uv, d.uv, on);
+    get(lc, d.lc, om);
+    get(uc, d.uc, om);
+    get(con, d.Dr, om);
+    get(var, d.Dc, on);
     *cbr = d.cb;
     *obr = d.ob;
     return 0;
@@ -672,6 +701,7 @@ int pdlp_gpu_power_method(const lp_problem_t *prob, const pdhg_parameters_t *par
   try {
     StreamGuard sg;
     std::unique_ptr<pdlp::DevProblem> P(pdlp::upload_problem(prob, sg.s));
+    pdlp::SolveInFlight in_flight;
     pdlp::Solve<double> s(*params, sg.s, *P, 0);
     s.prepare();
     s.init_step();
@@ -758,6 +788,7 @@ int pdlp_device_problem_time_kernels_prec(pdlp_device_problem_t *dp,
   if (!prepare_params(params, p)) return -1;
   try {
     StreamGuard sg;
+    pdlp::SolveInFlight in_flight;
     if (precision == PDLP_PRECISION_FP32_MATRIX) {
       pdlp::Solve<double, float> s(p, sg.s, *dp->P, 0);
       s.prepare();

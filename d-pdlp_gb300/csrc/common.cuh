@@ -89,6 +89,9 @@ struct Ctl {
   double pm_res;
   int pm_done;
   int pm_iters;
+  // in-loop timing of a resident team: ordinary iterations sampled
+  double live_primal_ns, live_dual_ns;
+  int live_n;
 };
 
 // Host-visible mirror written by the device when a solve finishes.
@@ -173,22 +176,55 @@ __device__ __forceinline__ void block_sum(double (&v)[NF], double *smem /*>= 8*N
   __syncthreads();
 }
 
-// Sum (or max, when IS_MAX) of part[0..n) by one block of kThreads threads,
-// in a fixed order.  Result returned to every thread.
+// Sums (or maxima, for the bits of MAXMASK) of NF fields part[f * n ..
+// f * n + n) by one block of kThreads threads, in a fixed order: four loads
+// and four chains a thread and field (an FP64 add has 62 cycles of latency).
+// smem: 8 * NF doubles.  Result returned to every thread.
+template <int NF, unsigned MAXMASK>
+__device__ __forceinline__ void block_fold_fields(const double *part, int n, double *smem,
+                                                  double (&out)[NF]) {
+  double q[NF][4];
+#pragma unroll
+  for (int f = 0; f < NF; ++f)
+#pragma unroll
+    for (int u = 0; u < 4; ++u) q[f][u] = 0.0;
+#pragma unroll 1
+  for (int i = threadIdx.x; i < n; i += 4 * kThreads)
+#pragma unroll
+    for (int f = 0; f < NF; ++f)
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (i + u * kThreads < n) {
+          const double v = part[(long)f * n + i + u * kThreads];
+          q[f][u] = ((MAXMASK >> f) & 1u) ? fmax(q[f][u], v) : q[f][u] + v;
+        }
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  __syncthreads();
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    const bool mx = (MAXMASK >> f) & 1u;
+    double s = mx ? fmax(fmax(q[f][0], q[f][1]), fmax(q[f][2], q[f][3]))
+                  : (q[f][0] + q[f][1]) + (q[f][2] + q[f][3]);
+    s = mx ? warp_max(s) : warp_sum(s);
+    if (lane == 0) smem[f * (kThreads / 32) + wid] = s;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int f = 0; f < NF; ++f) {
+    double r = 0.0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w)
+      r = ((MAXMASK >> f) & 1u) ? fmax(r, smem[f * (kThreads / 32) + w])
+                                : r + smem[f * (kThreads / 32) + w];
+    out[f] = r;
+  }
+  __syncthreads();
+}
 template <bool IS_MAX>
 __device__ double block_fold(const double *part, int n, double *smem) {
-  double s = 0.0;
-  for (int i = threadIdx.x; i < n; i += kThreads)
-    s = IS_MAX ? fmax(s, part[i]) : s + part[i];
-  s = IS_MAX ? warp_max(s) : warp_sum(s);
-  int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  __syncthreads();
-  if (lane == 0) smem[wid] = s;
-  __syncthreads();
-  double r = 0.0;
-  for (int w = 0; w < kThreads / 32; ++w) r = IS_MAX ? fmax(r, smem[w]) : r + smem[w];
-  __syncthreads();
-  return r;
+  double r[1];
+  block_fold_fields<1, IS_MAX ? 1u : 0u>(part, n, smem, r);
+  return r[0];
 }
 
 inline int grid_for(long n, int per_thread = 1) {

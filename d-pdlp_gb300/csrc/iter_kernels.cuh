@@ -30,10 +30,79 @@ __device__ __forceinline__ void halpern_weight(const Ctl *c, const double *hw, i
   sc[1] = 1.0 - w;
 }
 
-// primal step: x_hat = proj(x - tau (c - A^T y)), x_ref = 2 x_hat - x, Halpern
-// (reference pdlp_core_op.cu:393-418, :445-462, :495-526).  RHO1: the
-// reflection coefficient is 1 (the default), so the reflected point is x_ref
-// itself.
+// One variable of the primal step: x_hat = proj(x - tau (c - A^T y)), x_ref =
+// 2 x_hat - x, Halpern (reference pdlp_core_op.cu:393-418, :445-462,
+// :495-526).  rho1: the reflection coefficient is 1 (the default), so the
+// reflected point is x_ref itself.
+template <class T>
+struct PrimalPre {
+  T xc, c, lv, uv, x0;
+};
+template <class T>
+__device__ __forceinline__ void primal_update(const Dev<T> &d, int j, T s, const PrimalPre<T> &p,
+                                              T tau, T w, T omw, bool major, bool fpe, bool rho1,
+                                              T *xnext, double *acc) {
+  T xc = p.xc;
+  // every contraction is spelled out: the kernels that inline this agree bit
+  // for bit
+  T t = fma(-tau, p.c - s, xc);
+  T xh = clamp_to(t, p.lv, p.uv);
+  if (major) {
+    d.xhat[j] = xh;
+    d.lam[j] = (xh - t) / tau;
+  }
+  T xr = T(2) * xh - xc;
+  d.xref[j] = xr;
+  if (fpe) {
+    T dd = xr - xc;
+    d.dx[j] = dd;
+    acc[0] = fma((double)dd, (double)dd, acc[0]);
+  }
+  T refl = rho1 ? xr : fma((T)d.rho, xr, (T)d.one_minus_rho * xc);
+  xnext[j] = fma(w, refl, omw * p.x0);
+}
+
+// One constraint of the dual step: t = y/sigma - A x_ref, y_hat = sigma (t -
+// proj(t)), Halpern (reference pdlp_core_op.cu:420-443, :528-557)
+template <class T>
+struct DualPre {
+  T yc, lc, uc, y0;
+};
+// t = y/sigma - A x_ref from y, 1/sigma and the row's sum.  FP32: rounded once
+// or twice, as in the epilogues of the kernels whose sums the format keeps (see
+// "FP32 sums" in strip.cuh): once on the pipelined kernel's pairs and, in the
+// iterations that both save x_hat and need dx, dy, on the fused kernel's tiles
+// of 512.
+__device__ __forceinline__ double step_point(double yc, double inv_sigma, double s, bool) {
+  return fma(yc, inv_sigma, -s);
+}
+__device__ __forceinline__ float step_point(float yc, float inv_sigma, float s, bool once) {
+  return once ? fmaf(yc, inv_sigma, -s) : __fsub_rn(__fmul_rn(yc, inv_sigma), s);
+}
+enum Fp32Sums { kFp32Tiles512 = 0, kFp32Tiles = 1, kFp32Pairs = 2 };
+template <class T>
+__device__ __forceinline__ void dual_update(const Dev<T> &d, int i, T s, const DualPre<T> &p,
+                                            T sigma, T inv_sigma, T w, T omw, bool major,
+                                            bool fpe, bool rho1, T *ynext, double *acc) {
+  T yc = p.yc;
+  // the reference divides by sigma; one reciprocal per launch instead
+  // (at most 1 ulp apart; an FP64 division costs ~10 FP64 issue slots)
+  T t = step_point(yc, inv_sigma, s,
+                   d.fp32_sums == kFp32Pairs || (d.fp32_sums == kFp32Tiles512 && fpe && major));
+  T tp = clamp_to(t, -p.uc, -p.lc);
+  T yh = (t - tp) * sigma;
+  if (major) d.yhat[i] = yh;
+  T yr = T(2) * yh - yc;
+  if (fpe) {
+    T dd = yr - yc;
+    d.dy[i] = dd;
+    acc[0] = fma((double)dd, (double)dd, acc[0]);
+  }
+  T refl = rho1 ? yr : fma((T)d.rho, yr, (T)d.one_minus_rho * yc);
+  ynext[i] = fma(w, refl, omw * p.y0);
+}
+
+// primal step over A^T
 template <class T, class M, bool MAJOR, bool FPE, bool RHO1>
 struct PrimalEpi {
   using val_t = M;
@@ -57,9 +126,7 @@ struct PrimalEpi {
     omw = (T)sc[1];
   }
   __device__ M gather(int i) const { return (M)ycur[i]; }
-  struct Pre {
-    T xc, c, lv, uv, x0;
-  };
+  using Pre = PrimalPre<T>;
   // per-row vectors of the pipelined kernel, in Pre order
   using vec_t = T;
   static constexpr int NV = 5;
@@ -84,28 +151,11 @@ struct PrimalEpi {
     row_pre(j, sm, p, acc);
   }
   __device__ void row_pre(int j, M sm, const Pre &p, double *acc) const {
-    T s = (T)sm;
-    T xc = p.xc;
-    T t = xc - tau * (p.c - s);
-    T xh = clamp_to(t, p.lv, p.uv);
-    if (MAJOR) {
-      d.xhat[j] = xh;
-      d.lam[j] = (xh - t) / tau;
-    }
-    T xr = T(2) * xh - xc;
-    d.xref[j] = xr;
-    if (FPE) {
-      T dd = xr - xc;
-      d.dx[j] = dd;
-      acc[0] += (double)dd * (double)dd;
-    }
-    T refl = RHO1 ? xr : (T)d.rho * xr + (T)d.one_minus_rho * xc;
-    xnext[j] = w * refl + omw * p.x0;
+    primal_update(d, j, (T)sm, p, tau, w, omw, MAJOR, FPE, RHO1, xnext, acc);
   }
 };
 
-// dual step: t = y/sigma - A x_ref, y_hat = sigma (t - proj(t)), Halpern
-// (reference pdlp_core_op.cu:420-443, :528-557)
+// dual step over A
 template <class T, class M, bool MAJOR, bool FPE, bool RHO1>
 struct DualEpi {
   using val_t = M;
@@ -130,9 +180,7 @@ struct DualEpi {
     omw = (T)sc[1];
   }
   __device__ M gather(int j) const { return (M)d.xref[j]; }
-  struct Pre {
-    T yc, lc, uc, y0;
-  };
+  using Pre = DualPre<T>;
   using vec_t = T;
   static constexpr int NV = 4;
   __device__ void vecs(const T *(&v)[NV]) const {
@@ -154,33 +202,21 @@ struct DualEpi {
     row_pre(i, sm, p, acc);
   }
   __device__ void row_pre(int i, M sm, const Pre &p, double *acc) const {
-    T s = (T)sm;
-    T yc = p.yc;
-    // the reference divides by sigma; one reciprocal per launch instead
-    // (at most 1 ulp apart; an FP64 division costs ~10 FP64 issue slots)
-    T t = yc * inv_sigma - s;
-    T tp = clamp_to(t, -p.uc, -p.lc);
-    T yh = (t - tp) * sigma;
-    if (MAJOR) d.yhat[i] = yh;
-    T yr = T(2) * yh - yc;
-    if (FPE) {
-      T dd = yr - yc;
-      d.dy[i] = dd;
-      acc[0] += (double)dd * (double)dd;
-    }
-    T refl = RHO1 ? yr : (T)d.rho * yr + (T)d.one_minus_rho * yc;
-    ynext[i] = w * refl + omw * p.y0;
+    dual_update(d, i, (T)sm, p, sigma, inv_sigma, w, omw, MAJOR, FPE, RHO1, ynext, acc);
   }
 };
 
+// The evaluation epilogues below hold the solve's data as D: by value in a
+// kernel's parameters, by reference inside a resident team.
+
 // cross term <A^T dy, dx> of the fixed-point error (pdlp_core_op.cu:658-696)
-template <class T, class M, bool RESTART_ONLY>
+template <class T, class M, bool RESTART_ONLY, class D = Dev<T>>
 struct FpeEpi {
   using val_t = M;
   using acc_t = M;
   static constexpr int NF = 1;
   static constexpr unsigned MAXMASK = 0;
-  Dev<T> d;
+  D d;
   PDLP_NO_BLOCK_SCALARS
   __device__ bool init() {
     if (d.ctl->done) return false;
@@ -188,17 +224,19 @@ struct FpeEpi {
     return true;
   }
   __device__ M gather(int i) const { return (M)d.dy[i]; }
-  __device__ void row(int j, M s, double *acc) const { acc[0] += (double)s * (double)d.dx[j]; }
+  __device__ void row(int j, M s, double *acc) const {
+    acc[0] = fma((double)s, (double)d.dx[j], acc[0]);
+  }
 };
 
 // KKT over A x_hat (utils.cu:503-531 constraint half), FP64 terms
-template <class T, class M, bool LINF>
+template <class T, class M, bool LINF, class D = Dev<T>>
 struct EvalAEpi {
   using val_t = M;
   using acc_t = M;
   static constexpr int NF = 2;
   static constexpr unsigned MAXMASK = LINF ? 1u : 0u;
-  Dev<T> d;
+  D d;
   PDLP_NO_BLOCK_SCALARS
   __device__ bool init() { return !d.ctl->done; }
   __device__ M gather(int j) const { return (M)d.xhat[j]; }
@@ -218,13 +256,13 @@ struct EvalAEpi {
 };
 
 // KKT over A^T y_hat (utils.cu:503-531 variable half, plus objective dots)
-template <class T, class M, bool LINF>
+template <class T, class M, bool LINF, class D = Dev<T>>
 struct EvalATEpi {
   using val_t = M;
   using acc_t = M;
   static constexpr int NF = 3;
   static constexpr unsigned MAXMASK = LINF ? 1u : 0u;
-  Dev<T> d;
+  D d;
   PDLP_NO_BLOCK_SCALARS
   __device__ bool init() { return !d.ctl->done; }
   __device__ M gather(int i) const { return (M)d.yhat[i]; }
@@ -250,13 +288,13 @@ __device__ __forceinline__ double ray_scale(const Ctl *c) {
 }
 
 // primal ray over A (utils.cu:561-572, :588-600)
-template <class T, class M>
+template <class T, class M, class D = Dev<T>>
 struct InfAEpi {
   using val_t = M;
   using acc_t = M;
   static constexpr int NF = 2;
   static constexpr unsigned MAXMASK = 1u;
-  Dev<T> d;
+  D d;
   T sc;
   PDLP_NO_BLOCK_SCALARS
   __device__ bool init() {  // runs twice per solve: a per-thread division is fine
@@ -277,13 +315,13 @@ struct InfAEpi {
 
 // dual ray over A^T (utils.cu:574-586, :602-614; the slack slot holds A^T dy
 // as in the reference call at utils.cu:772-776)
-template <class T, class M>
+template <class T, class M, class D = Dev<T>>
 struct InfATEpi {
   using val_t = M;
   using acc_t = M;
   static constexpr int NF = 3;
   static constexpr unsigned MAXMASK = 2u;
-  Dev<T> d;
+  D d;
   T sc;
   PDLP_NO_BLOCK_SCALARS
   __device__ bool init() {
@@ -311,21 +349,23 @@ struct ReducedCostEpi {
   static constexpr unsigned MAXMASK = 0;
   Dev<T> d;
   double *out;
+  const int *perm;  // where each entry goes (null: its own place)
   PDLP_NO_BLOCK_SCALARS
   __device__ bool init() { return true; }
   __device__ M gather(int i) const { return (M)d.yhat[i]; }
   __device__ void row(int j, M s, double *) const {
-    out[j] = ((double)d.c[j] - (double)s) * d.Dc[j] / d.ob;
+    out[perm ? perm[j] : j] = ((double)d.c[j] - (double)s) * d.Dc[j] / d.ob;
   }
 };
 
 // power method: g = A^T (inv * v)   (utils.cu:127-136)
+template <class D = PowDev>
 struct PowAtEpi {
   using val_t = double;
   using acc_t = double;
   static constexpr int NF = 0;
   static constexpr unsigned MAXMASK = 0;
-  PowDev d;
+  D d;
   const double *v;
   double inv;
   PDLP_NO_BLOCK_SCALARS
@@ -339,12 +379,13 @@ struct PowAtEpi {
 };
 
 // power method: v' = A g, sum q.v', sum v'^2   (utils.cu:138-144)
+template <class D = PowDev>
 struct PowAEpi {
   using val_t = double;
   using acc_t = double;
   static constexpr int NF = 2;
   static constexpr unsigned MAXMASK = 0;
-  PowDev d;
+  D d;
   const double *v;
   double *vnext;
   double inv;
@@ -370,12 +411,11 @@ __device__ __forceinline__ void set_steps(Ctl *c) {
   c->inv_sigma = 1.0 / c->sigma;
 }
 
-// Each matrix of a solve runs every SpMV on one of the two kernels: the
-// pipelined one (M.pipe_on) or the fused one.  The choice is made per matrix
-// by timing both on the step epilogue (Solve::tune_kernels), or forced by
-// PDLP_STEP_KERNEL=pipe / fused; reduction partials are sized for either
-// and folded with the counts of the kernel in use.
-// 1: forced pipelined, 0: forced fused, -1: measured per matrix
+// Every SpMV of a matrix runs on one kernel: the strip kernel (strip.cuh), or
+// on plain CSR the pipelined or the fused one when PDLP_STEP_KERNEL=pipe /
+// fused forces it.  Reduction partials are sized and folded with the counts
+// of the kernel in use.
+// 1: forced pipelined, 0: forced fused, -1: the strip kernel
 int kernel_override();
 
 template <class V>
@@ -384,20 +424,32 @@ inline bool use_pipe(const DevCsrT<V> &M) {
 }
 template <class V>
 inline size_t spmv_partials(const DevCsrT<V> &M) {
+  if (M.strip.on)
+    return (size_t)(M.strip.unit_parts ? M.strip.nitem + M.strip.nstrip : M.strip.grid);
   return use_pipe(M) ? (size_t)M.pipe.grid : (size_t)M.plan.nblk;
 }
 template <class V>
 inline size_t spmv_long_rows(const DevCsrT<V> &M) {
+  if (M.strip.on) return (size_t)M.strip.nlong;
   return use_pipe(M) ? (size_t)M.pipe.nlong : (size_t)M.plan.nlong;
 }
 // partial buffers large enough for either kernel
 template <class V>
 inline size_t spmv_partials_max(const DevCsrT<V> &M) {
+  if (M.strip.on)
+    return (size_t)(M.strip.unit_parts ? M.strip.nitem + M.strip.nstrip : M.strip.grid);
   return (size_t)(M.pipe.grid > M.plan.nblk ? M.pipe.grid : M.plan.nblk);
 }
 template <class V>
 inline size_t spmv_long_rows_max(const DevCsrT<V> &M) {
+  if (M.strip.on) return (size_t)M.strip.nlong;
   return (size_t)(M.pipe.nlong > M.plan.nlong ? M.pipe.nlong : M.plan.nlong);
+}
+
+// A and A^T do not fit in the 129 MB L2 beside the vectors
+template <class V>
+inline bool strip_streams(const DevCsrT<V> &M) {
+  return 2.0 * M.strip.store * (4 + sizeof(V)) > 100e6;
 }
 
 template <class Epi>
@@ -410,6 +462,28 @@ void set_pipe_smem() {
 template <class Epi, class V>
 void launch_spmv(const DevCsrT<V> &M, const Epi &epi, double *part, double *lpart,
                  cudaStream_t st) {
+  if (M.strip.on) {
+    if (M.strip.grid == 0) return;
+    auto go = [&](auto stream, auto pair) {
+      spmv_strip<Epi, decltype(stream)::value, decltype(pair)::value>
+          <<<M.strip.grid, kThreads, 0, st>>>(strip_mat(M), part, lpart, epi);
+    };
+    using Yes = std::true_type;
+    using No = std::false_type;
+    // FP32: in pairs or not ("FP32 sums" in strip.cuh)
+    if constexpr (sizeof(typename Epi::val_t) == 8) {
+      if (strip_streams(M)) go(Yes{}, No{});
+      else go(No{}, No{});
+    } else if (M.strip.pairs) {
+      if (strip_streams(M)) go(Yes{}, Yes{});
+      else go(No{}, Yes{});
+    } else {
+      if (strip_streams(M)) go(Yes{}, No{});
+      else go(No{}, No{});
+    }
+    PDLP_LAUNCH_CHECK();
+    return;
+  }
   if (use_pipe(M)) {
     set_pipe_smem<Epi>();
     spmv_pipe<Epi><<<M.pipe.grid, kPipeBlock, kPipeSmem, st>>>(M.ptr, M.col, M.val, M.pipe,

@@ -143,6 +143,7 @@ cupdlpx_result_t *solve_refined(const DevProblem &P, const pdhg_parameters_t &pa
   for (const DevCsr *W : {&P.A, &P.AT}) {
     need((size_t)W->plan.nlong * 4); need((size_t)W->plan.nblk * 8);
     need((size_t)W->pipe.nlong * 4); need((size_t)W->pipe.ntile * 8); need(4);
+    need((size_t)W->strip.nlong * 4); need((size_t)W->strip.nitem * 8);
   }
   char *mem = (char *)dev_alloc(bytes, st);
   struct Free {
@@ -179,6 +180,10 @@ cupdlpx_result_t *solve_refined(const DevProblem &P, const pdhg_parameters_t &pa
     if (W->pipe.nlong)
       PDLP_CUDA(cudaMemsetAsync(W->pipe.lcnt, 0, (size_t)W->pipe.nlong * 4, st));
     PDLP_CUDA(cudaMemsetAsync(W->pipe.err, 0, sizeof(int), st));
+    W->strip.lcnt = (unsigned *)take((size_t)W->strip.nlong * 4);
+    W->strip.lsum = (double *)take((size_t)W->strip.nitem * 8);
+    if (W->strip.nlong)
+      PDLP_CUDA(cudaMemsetAsync(W->strip.lcnt, 0, (size_t)W->strip.nlong * 4, st));
   }
   if (n) {
     PDLP_CUDA(cudaMemsetAsync(xbar, 0, vn * 8, st));
@@ -203,7 +208,10 @@ cupdlpx_result_t *solve_refined(const DevProblem &P, const pdhg_parameters_t &pa
   Q.tile = P.tile;
   Q.A = P.A;
   Q.AT = P.AT;
-  Q.shape_key = P.shape_key;  // same structure: the rounds run round 0's kernels
+  Q.strips = P.strips;
+  Q.nsm = P.nsm;
+  Q.perm_m = P.perm_m;
+  Q.perm_n = P.perm_n;
   Q.c = c2;
   Q.lv = lv2;
   Q.uv = uv2;
@@ -320,9 +328,8 @@ cupdlpx_result_t *solve_refined(const DevProblem &P, const pdhg_parameters_t &pa
       s.enable_snapshot();
       s.run();
       if (round == 0) {
-        rep.kernel_A = s.pipe_A() ? 1 : 0;
-        rep.kernel_AT = s.pipe_AT() ? 1 : 0;
-        for (int q = 0; q < 4; ++q) rep.tune_ms[q] = s.tune_ms(q);
+        rep.kernel_A = s.kernel_A();
+        rep.kernel_AT = s.kernel_AT();
         omega0 = s.primal_weight();
         cb0 = s.cb();
         ob0 = s.ob();
@@ -406,7 +413,10 @@ cupdlpx_result_t *solve_refined(const DevProblem &P, const pdhg_parameters_t &pa
     W.tile = P.tile;
     W.A = P.A;
     W.AT = P.AT;
-    W.shape_key = P.shape_key;
+    W.strips = P.strips;
+    W.nsm = P.nsm;
+    W.perm_m = P.perm_m;
+    W.perm_n = P.perm_n;
     W.c = P.c;
     W.lv = P.lv;
     W.uv = P.uv;
@@ -480,6 +490,17 @@ cupdlpx_result_t *solve_refined(const DevProblem &P, const pdhg_parameters_t &pa
     free(res->reduced_cost);
     free(res);
     throw std::bad_alloc();
+  }
+  // back to the caller's order
+  if (n && P.perm_n) {
+    launch_scatter(n, xbar, P.perm_n, z, st);
+    launch_scatter(n, rc, P.perm_n, lz, st);
+    xbar = z;
+    rc = lz;
+  }
+  if (m && P.perm_m) {
+    launch_scatter(m, ybar, P.perm_m, w, st);
+    ybar = w;
   }
   if (n) {
     PDLP_CUDA(cudaMemcpyAsync(res->primal_solution, xbar, vn * 8, cudaMemcpyDeviceToHost, st));

@@ -172,6 +172,8 @@ long long pdlp_estimate_device_bytes(int m, int n, long long nnz, int precision)
   const long long vm = m, vn = n;
   // resident problem: A and A^T in CSR, plans, objective and bounds
   long long b = 24 * nnz + 4 * (vm + vn + 2) + 40 * vn + 16 * vm + (nnz / 512 + 64) * 56;
+  // row words and tiles of the resident team
+  b += 2 * nnz + ((vm + vn) / 256 + nnz / 512 + 64) * 64;
   // FP64 solve: scaled values, iterates and work vectors, partial sums
   b += 16 * nnz + 8 * (24 * vn + 18 * vm) + (nnz / 512 + 64) * 160 + (1 << 20);
   if (precision != PDLP_PRECISION_FP64) {

@@ -9,6 +9,8 @@
 #include <algorithm>
 #include <atomic>
 #include <exception>
+#include <mutex>
+#include <future>
 #include <thread>
 
 #include "solver_impl.cuh"
@@ -47,28 +49,33 @@ __global__ void __launch_bounds__(kThreads) k_pm_dot_fin(PowDev d) {
   Ctl *c = d.ctl;
   if (c->pm_done) return;
   __shared__ double sm[32];
-  double dotqv = fold_site<false>(d.p_pa, d.nblkA, d.lp_pa, d.nlongA, 0, sm);
-  double vv = fold_site<false>(d.p_pa, d.nblkA, d.lp_pa, d.nlongA, 1, sm);
+  double v[2];  // q.v', |v'|^2
+  fold_site<2, 0u>(d.p_pa, d.nblkA, d.lp_pa, d.nlongA, sm, v);
   if (threadIdx.x == 0) {
-    c->pm_sigma_sq = dotqv;
-    c->pm_res = vv;  // |v'|^2, turned into 1/|v'| after the residual
+    c->pm_sigma_sq = v[0];
+    c->pm_res = v[1];  // |v'|^2, turned into 1/|v'| after the residual
   }
 }
 
-__global__ void __launch_bounds__(kThreads)
-    k_pm_resid(PowDev d, const double *v, const double *vnext) {
-  if (d.ctl->pm_done) return;
-  __shared__ double red[16];
-  double inv = d.ctl->pm_inv_norm, ns = -d.ctl->pm_sigma_sq;
+// block `b` of d.ew_grid: its partial of |v' - sigma^2 q|^2
+__device__ __forceinline__ void resid_block(const PowDev &d, const double *v, const double *vnext,
+                                            double inv, double ns, int b, double *red) {
   double a[1] = {0.0};
-  long stride = (long)gridDim.x * kThreads;
-  for (long i = blockIdx.x * (long)kThreads + threadIdx.x; i < d.m; i += stride) {
+  const long stride = (long)d.ew_grid * kThreads;
+#pragma unroll 2
+  for (long i = b * (long)kThreads + threadIdx.x; i < d.m; i += stride) {
     double q = inv * v[i];
     double r = 1.0 * vnext[i] + ns * q;
     a[0] += r * r;
   }
   block_reduce_fields<1, 0u>(a, red);
-  if (threadIdx.x == 0) d.p_pr[blockIdx.x] = a[0];
+  if (threadIdx.x == 0) d.p_pr[b] = a[0];
+}
+__global__ void __launch_bounds__(kThreads)
+    k_pm_resid(PowDev d, const double *v, const double *vnext) {
+  if (d.ctl->pm_done) return;
+  __shared__ double red[16];
+  resid_block(d, v, vnext, d.ctl->pm_inv_norm, -d.ctl->pm_sigma_sq, blockIdx.x, red);
 }
 
 __global__ void __launch_bounds__(kThreads) k_pm_resid_fin(PowDev d) {
@@ -88,6 +95,176 @@ __global__ void __launch_bounds__(kThreads) k_pm_resid_fin(PowDev d) {
     }
   }
 }
+
+// ---- strip format
+__global__ void k_invert(int n, const int *__restrict__ perm, int *__restrict__ inv) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    inv[perm[i]] = (int)i;
+}
+__global__ void k_gather(int n, const double *__restrict__ src, const int *__restrict__ perm,
+                         double *__restrict__ dst) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    dst[i] = src[perm[i]];
+}
+__global__ void k_scatter_back(int n, const double *__restrict__ src, const int *__restrict__ perm,
+                               double *__restrict__ dst) {
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
+    dst[perm[i]] = src[i];
+}
+void launch_gather(int n, const double *src, const int *perm, double *dst, cudaStream_t st) {
+  if (n <= 0) return;
+  k_gather<<<grid_for(n), kThreads, 0, st>>>(n, src, perm, dst);
+  PDLP_LAUNCH_CHECK();
+}
+void launch_scatter(int n, const double *src, const int *perm, double *dst, cudaStream_t st) {
+  if (n <= 0) return;
+  k_scatter_back<<<grid_for(n), kThreads, 0, st>>>(n, src, perm, dst);
+  PDLP_LAUNCH_CHECK();
+}
+
+// The stored elements of a strip-format matrix from CSR rows sptr / scol /
+// sval: row i is the source's row perm[i] with its entries in their order,
+// column j becomes icol[j] (null permutations: the identity).  A warp per
+// front row, then a warp per strip.
+__global__ void __launch_bounds__(kThreads)
+    k_strip_fill(StripMat<double> A, const int *__restrict__ sptr, const int *__restrict__ scol,
+                 const double *__restrict__ sval, const int *__restrict__ perm,
+                 const int *__restrict__ icol, int *__restrict__ col, double *__restrict__ val) {
+  const int lane = threadIdx.x & 31;
+  const int W = gridDim.x * (kThreads / 32);
+  for (int w = (blockIdx.x * kThreads + threadIdx.x) >> 5; w < A.p.nfront + A.p.nstrip; w += W) {
+    if (w < A.p.nfront) {
+      const int a = sptr[perm ? perm[w] : w], to = A.ptr[w], len = A.ptr[w + 1] - to;
+      for (int k = lane; k < len; k += 32) {
+        const int c = scol[a + k];
+        col[to + k] = icol ? icol[c] : c;
+        val[to + k] = sval[a + k];
+      }
+      continue;
+    }
+    const int s = w - A.p.nfront, lg = A.p.lg;
+    const int row = A.p.nfront + s * (32 >> lg) + (lane >> lg), sub = lane & ((1 << lg) - 1);
+    int a = 0, len = 0;
+    if (row < A.rows) {
+      const int r = perm ? perm[row] : row;
+      a = sptr[r];
+      len = sptr[r + 1] - a;
+    }
+    const size_t o0 = (size_t)A.p.off[s] * 32 + lane;
+    const int width = A.p.off[s + 1] - A.p.off[s];
+    for (int k = 0; k < width; ++k) {
+      int c = -1;
+      double v = 0.0;
+      const int e = (k << lg) + sub;
+      if (e < len) {
+        c = scol[a + e];
+        if (icol) c = icol[c];
+        v = sval[a + e];
+      }
+      col[o0 + (size_t)k * 32] = c;
+      val[o0 + (size_t)k * 32] = v;
+    }
+  }
+}
+
+struct TeamPower {
+  PowDev d;
+  StripMat<double> A, AT;
+};
+
+// The power method (reference src/utils.cu:66-171): iterations until the
+// residual is below sv_tol or `maxit` are done, two barriers each.  Every CTA
+// folds the sums itself; the residual of an iteration is checked after the
+// next one's A^T product, which writes nothing the result depends on.
+__global__ void __launch_bounds__(kTeamThreads, kTeamCtasPerSm)
+    team_power(const __grid_constant__ TeamPower data, const __grid_constant__ TeamBar bar,
+               int maxit) {
+  __shared__ TeamSmem sm;
+  __shared__ TeamPower sd;
+  Ctl *c = data.d.ctl;
+  if (ld_flag(&c->pm_done)) return;
+  team_copy(data, sd, sm);
+  const PowDev &d = sd.d;
+  int it = 0;
+  double inv = c->pm_inv_norm, sigma_sq = 0.0, res = 0.0;
+  bool check = false;  // the last iteration left partial sums of its residual
+  StripHead<double> xT;
+  strip_head<false>(sd.AT, team_strip(), xT);
+  for (;;) {
+    if (it < maxit)
+      team_phase<0, 0u>(
+          sd, [](const TeamPower &x) -> const auto & { return x.AT; },
+          [=](const TeamPower &x) {
+            return PowAtEpi<const PowDev &>{x.d, (it & 1) ? x.d.v[1] : x.d.v[0], inv};
+          },
+          nullptr, xT);
+    StripHead<double> xA;
+    strip_head<false>(sd.A, team_strip(), xA);
+    if (!team_sync(bar, sm)) return;
+    if (check) {  // residual of iteration it - 1
+      double v[1];
+      block_fold_fields<1, 0u>(d.p_pr, d.ew_grid, sm.red, v);
+      res = sqrt(v[0]);
+    }
+    if (it == maxit || (check && res < d.sv_tol)) break;
+    team_phase<2, 0u>(
+        sd, [](const TeamPower &x) -> const auto & { return x.A; },
+        [=](const TeamPower &x) {
+          return PowAEpi<const PowDev &>{x.d, (it & 1) ? x.d.v[1] : x.d.v[0],
+                                         (it & 1) ? x.d.v[0] : x.d.v[1], inv};
+        },
+        d.p_pa, xA);
+    strip_head<false>(sd.AT, team_strip(), xT);
+    if (!team_sync(bar, sm)) return;
+    double v[2];  // q.v', |v'|^2
+    fold_site<2, 0u>(d.p_pa, d.nblkA, d.lp_pa, d.nlongA, sm.red, v);
+    sigma_sq = v[0];
+    // |v' - sigma^2 q|^2 = |v'|^2 - sigma^4, up to rounding of about 1e-15
+    // |v'|^2: the residual itself is only summed where that does not already
+    // show that it is far above the tolerance
+    const double about = v[1] - sigma_sq * sigma_sq;
+    check = !(about - 1e-12 * v[1] > 4.0 * d.sv_tol * d.sv_tol) || it + 1 == maxit;
+    if (check)
+      for (int b = blockIdx.x; b < d.ew_grid; b += gridDim.x) {
+        resid_block(d, (it & 1) ? d.v[1] : d.v[0], (it & 1) ? d.v[0] : d.v[1], inv, -sigma_sq, b,
+                    sm.red);
+        __syncthreads();
+      }
+    inv = 1.0 / sqrt(v[1]);
+    ++it;
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    c->pm_iters = it;
+    c->pm_sigma_sq = sigma_sq;
+    c->pm_inv_norm = inv;
+    c->pm_res = res;
+    c->pm_done = check && res < d.sv_tol ? 1 : 0;
+    if (c->pm_done) {
+      __threadfence_system();
+      d.hflag->pm_done = 1;
+    }
+  }
+}
+
+void launch_team_power(int ctas, cudaStream_t st, const PowDev &d, const StripMat<double> &A,
+                       const StripMat<double> &AT, const TeamBar &bar, int maxit) {
+  team_launch(ctas, team_power, st, TeamPower{d, A, AT}, bar, maxit);
+}
+
+namespace {
+std::atomic<int> g_solves{0};
+std::mutex g_team_mu;
+}  // namespace
+
+SolveInFlight::SolveInFlight() { g_solves.fetch_add(1); }
+SolveInFlight::~SolveInFlight() { g_solves.fetch_sub(1); }
+TeamTurn::TeamTurn(bool wanted) {
+  held_ = wanted && alone() && g_team_mu.try_lock();
+}
+TeamTurn::~TeamTurn() {
+  if (held_) g_team_mu.unlock();
+}
+bool TeamTurn::alone() { return g_solves.load() <= 1; }
 
 // A^T in CSR, entries of each column in row order (a stable counting sort).
 // Matrices of 4M+ non-zeros are transposed by up to 8 threads, each owning a
@@ -175,16 +352,6 @@ int kernel_override() {
 }
 
 namespace {
-std::mutex g_choice_mu;
-std::map<uint64_t, std::array<int, 2>> g_choice[3];
-
-// FNV-1a over 32-bit words (the fingerprint only has to separate structures
-// within one process)
-uint64_t fnv1a(uint64_t h, const int *v, size_t count) {
-  for (size_t i = 0; i < count; ++i) h = (h ^ (uint32_t)v[i]) * 1099511628211ull;
-  return h;
-}
-
 // Host threads for the upload's passes over the non-zeros (LPs of 2M+
 // non-zeros; smaller ones stay on the calling thread).
 int upload_threads(long nnz) {
@@ -205,22 +372,6 @@ void parallel_slices(int T, long count, F &&f) {
   for (auto &x : th) x.join();
 }
 }  // namespace
-
-bool lookup_kernel_choice(uint64_t key, int prec, int c[2]) {
-  std::lock_guard<std::mutex> lk(g_choice_mu);
-  auto it = g_choice[prec].find(key);
-  if (it == g_choice[prec].end()) return false;
-  c[0] = it->second[0];
-  c[1] = it->second[1];
-  return true;
-}
-
-void settle_kernel_choice(uint64_t key, int prec, int c[2]) {
-  std::lock_guard<std::mutex> lk(g_choice_mu);
-  auto it = g_choice[prec].emplace(key, std::array<int, 2>{c[0], c[1]}).first;
-  c[0] = it->second[0];
-  c[1] = it->second[1];
-}
 
 DevProblem::~DevProblem() {
   if (arena) dev_free(arena, owner);
@@ -276,12 +427,12 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st) {
     }
     for (int c = 0; c < n; ++c) tp[c + 1] += tp[c];
   }
-  {
-    const int dims[3] = {m, n, nnz};
-    uint64_t h = fnv1a(1469598103934665603ull, dims, 3);
-    h = fnv1a(h, prob->constraint_matrix_row_pointers, (size_t)m + 1);
-    P->shape_key = fnv1a(h, tp.data(), (size_t)n + 1);
-  }
+  const bool strips = kernel_override() < 0;  // else the forced kernel's CSR
+  P->strips = strips;
+  int dev = 0, nsm = kNumSms;
+  PDLP_CUDA(cudaGetDevice(&dev));
+  PDLP_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  P->nsm = nsm;
   std::vector<int4> blkA, blkT;
   std::vector<int2> lrA, lrT;
   const int chunk = pick_chunk(P->tile);
@@ -290,7 +441,41 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st) {
   // LPs, beside A^T's.
   std::vector<int4> pblkA, pblkT;
   std::vector<int2> plrA, plrT;
+  StripHost shA, shT;
+  auto strips_of = [&](int rows, const int *ptr, int nv, StripHost &h) {
+    std::vector<unsigned char> sums;
+    bool pairs = false;
+    auto fp32_sums = [&] {
+      bool front = false;
+      for (int r = 0; r < rows && !front; ++r) front = ptr[r + 1] - ptr[r] > kStripRow;
+      pairs = nnz >= kTeamMaxNnz && !front;
+      if (pairs) strip_sums_pipe(rows, ptr, nv, sums);
+      else strip_sums_fused(rows, ptr, P->tile, chunk, sums);
+    };
+    const int T = upload_threads(nnz);
+    if (T > 1) {
+      auto other = std::async(std::launch::async, fp32_sums);
+      build_strip_host(rows, ptr, nsm, chunk, h);
+      other.get();
+    } else {
+      build_strip_host(rows, ptr, nsm, chunk, h);
+      fp32_sums();
+    }
+    h.pairs = pairs;
+    if (h.identity) {
+      h.sums = std::move(sums);
+    } else {
+      h.sums.resize(rows);
+      parallel_slices(T, rows, [&](long a, long b) {
+        for (long i = a; i < b; ++i) h.sums[i] = sums[h.perm[i]];
+      });
+    }
+  };
   auto plans_A = [&] {
+    if (strips) {
+      strips_of(m, prob->constraint_matrix_row_pointers, 4, shA);
+      return;
+    }
     build_plan_host(m, prob->constraint_matrix_row_pointers, P->tile, blkA, lrA, chunk);
     build_pipe_plan_host(m, prob->constraint_matrix_row_pointers, 4, pblkA, plrA);
   };
@@ -307,17 +492,18 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st) {
   else
     plans_A();
   try {
-    build_plan_host(n, tp.data(), P->tile, blkT, lrT, chunk);
-    build_pipe_plan_host(n, tp.data(), 5, pblkT, plrT);
+    if (strips) {
+      strips_of(n, tp.data(), 5, shT);
+    } else {
+      build_plan_host(n, tp.data(), P->tile, blkT, lrT, chunk);
+      build_pipe_plan_host(n, tp.data(), 5, pblkT, plrT);
+    }
   } catch (...) {
     if (thread_A.joinable()) thread_A.join();
     throw;
   }
   if (thread_A.joinable()) thread_A.join();
   if (failed_A) std::rethrow_exception(failed_A);
-  int dev = 0, nsm = kNumSms;
-  PDLP_CUDA(cudaGetDevice(&dev));
-  PDLP_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   // norms of the unscaled objective and bounds (reference pdlp_core_op.cu:232-286)
   {
     double ss = 0, mx = 0;
@@ -346,8 +532,18 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st) {
   }
   const size_t vn = n, vm = m;
   Sizer z;
-  z.add<int>(vm + 1); z.add<int>(nnz); z.add<double>(nnz);
-  z.add<int>(vn + 1); z.add<int>(nnz); z.add<double>(nnz);
+  if (strips) {
+    for (const StripHost *h : {&shA, &shT}) {
+      z.add<int>(h->store); z.add<double>(h->store);
+      z.add<int>(h->fptr.size()); z.add<int>(h->off.size());
+      z.add<int4>(h->item.size()); z.add<int2>(h->lrow.size());
+      z.add<unsigned char>(h->sums.size());
+      if (!h->identity) z.add<int>(h->perm.size());
+    }
+  } else {
+    z.add<int>(vm + 1); z.add<int>(nnz); z.add<double>(nnz);
+    z.add<int>(vn + 1); z.add<int>(nnz); z.add<double>(nnz);
+  }
   z.add<int4>(blkA.size()); z.add<int2>(lrA.size());
   z.add<int4>(blkT.size()); z.add<int2>(lrT.size());
   z.add<int4>(pblkA.size()); z.add<int2>(plrA.size());
@@ -392,8 +588,45 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st) {
     if (!plr.empty())
       PDLP_CUDA(cudaMemcpyAsync(M.pipe.lrow, plr.data(), plr.size() * 8, cudaMemcpyHostToDevice, st));
   };
-  mat(P->A, m, n, blkA, lrA, pblkA, plrA);
-  mat(P->AT, n, m, blkT, lrT, pblkT, plrT);
+  auto up = [&](auto *&dst, const auto &src) {
+    using E = typename std::remove_reference_t<decltype(src)>::value_type;
+    E *p = ar.take<E>(src.size());
+    dst = p;
+    if (!src.empty())
+      PDLP_CUDA(cudaMemcpyAsync(p, src.data(), src.size() * sizeof(E), cudaMemcpyHostToDevice, st));
+  };
+  auto strip = [&](DevCsr &M, int rows, int cols, const StripHost &h, const int *&perm) {
+    M.rows = rows;
+    M.cols = cols;
+    M.nnz = nnz;
+    M.col = ar.take<int>(h.store);
+    M.val = ar.take<double>(h.store);
+    StripPlan &p = M.strip;
+    p.on = 1;
+    p.nfront = (int)h.fptr.size() - 1;
+    p.nitem = (int)h.item.size();
+    p.nlong = (int)h.lrow.size();
+    p.nstrip = (int)h.off.size() - 1;
+    p.lg = h.lg;
+    p.store = h.store;
+    const long warps = (long)p.nitem + p.nstrip, per = kThreads / 32;
+    p.grid = (int)((warps + per - 1) / per);
+    p.unit_parts = nnz < kTeamMaxNnz;
+    p.pairs = h.pairs;
+    up(M.ptr, h.fptr);
+    up(p.off, h.off);
+    up(p.item, h.item);
+    up(p.lrow, h.lrow);
+    up(p.sums, h.sums);
+    if (!h.identity) up(perm, h.perm);
+  };
+  if (strips) {
+    strip(P->A, m, n, shA, P->perm_m);
+    strip(P->AT, n, m, shT, P->perm_n);
+  } else {
+    mat(P->A, m, n, blkA, lrA, pblkA, plrA);
+    mat(P->AT, n, m, blkT, lrT, pblkT, plrT);
+  }
   P->c = ar.take<double>(vn);
   P->lv = ar.take<double>(vn);
   P->uv = ar.take<double>(vn);
@@ -402,29 +635,75 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st) {
   auto h2d = [&](void *dst, const void *src, size_t b) {
     if (b) PDLP_CUDA(cudaMemcpyAsync(dst, src, b, cudaMemcpyHostToDevice, st));
   };
-  h2d(P->A.ptr, prob->constraint_matrix_row_pointers, (vm + 1) * 4);
-  h2d(P->A.col, prob->constraint_matrix_col_indices, (size_t)nnz * 4);
-  h2d(P->A.val, prob->constraint_matrix_values, (size_t)nnz * 8);
+  // device scratch of the upload, released on its stream
+  struct Scratch {
+    void *p = nullptr;
+    cudaStream_t st;
+    ~Scratch() { dev_free(p, st); }
+  };
   {
-    // stable transpose on the device (reference: cusparseCsr2cscEx2,
-    // src/pdlp_core_op.cu:109-130), scratch released on this stream
-    void *scratch = dev_alloc(device_transpose_scratch_bytes(n, nnz), st);
-    device_transpose(m, n, nnz, P->A.ptr, P->A.col, P->A.val, P->AT.ptr, P->AT.col, P->AT.val,
-                     scratch, st);
-    dev_free(scratch, st);
+    // A as given, then its stable transpose on the device (reference:
+    // cusparseCsr2cscEx2, src/pdlp_core_op.cu:109-130); in the strip format
+    // both are then laid out in the order of their rows' lengths
+    Sizer zs;
+    if (strips) {
+      zs.add<int>(vm + 1); zs.add<int>(nnz); zs.add<double>(nnz);
+      zs.add<int>(vn + 1); zs.add<int>(nnz); zs.add<double>(nnz);
+      zs.add<int>(vm); zs.add<int>(vn);
+    }
+    zs.add<char>(device_transpose_scratch_bytes(n, nnz));
+    Scratch sc{dev_alloc(zs.bytes, st), st};
+    Arena sa{(char *)sc.p, 0};
+    int *ptr = P->A.ptr, *col = P->A.col, *tptr = P->AT.ptr, *tcol = P->AT.col;
+    double *val = P->A.val, *tval = P->AT.val;
+    int *inv_m = nullptr, *inv_n = nullptr;
+    if (strips) {
+      ptr = sa.take<int>(vm + 1); col = sa.take<int>(nnz); val = sa.take<double>(nnz);
+      tptr = sa.take<int>(vn + 1); tcol = sa.take<int>(nnz); tval = sa.take<double>(nnz);
+      inv_m = sa.take<int>(vm); inv_n = sa.take<int>(vn);
+    }
+    h2d(ptr, prob->constraint_matrix_row_pointers, (vm + 1) * 4);
+    h2d(col, prob->constraint_matrix_col_indices, (size_t)nnz * 4);
+    h2d(val, prob->constraint_matrix_values, (size_t)nnz * 8);
+    device_transpose(m, n, nnz, ptr, col, val, tptr, tcol, tval,
+                     sa.take<char>(device_transpose_scratch_bytes(n, nnz)), st);
+    if (strips) {
+      if (P->perm_m) k_invert<<<grid_for(m), kThreads, 0, st>>>(m, P->perm_m, inv_m);
+      if (P->perm_n) k_invert<<<grid_for(n), kThreads, 0, st>>>(n, P->perm_n, inv_n);
+      auto fill = [&](DevCsr &M, const int *sp, const int *sc, const double *sv, const int *perm,
+                      const int *icol) {
+        const long warps = (long)M.strip.nfront + M.strip.nstrip;
+        if (warps == 0) return;
+        k_strip_fill<<<grid_for(warps * 32), kThreads, 0, st>>>(strip_mat(M), sp, sc, sv, perm,
+                                                               icol, M.col, M.val);
+        PDLP_LAUNCH_CHECK();
+      };
+      fill(P->A, ptr, col, val, P->perm_m, P->perm_n ? inv_n : nullptr);
+      fill(P->AT, tptr, tcol, tval, P->perm_n, P->perm_m ? inv_m : nullptr);
+    }
   }
-  h2d(P->c, prob->objective_vector, vn * 8);
-  h2d(P->lv, prob->variable_lower_bound, vn * 8);
-  h2d(P->uv, prob->variable_upper_bound, vn * 8);
-  h2d(P->lc, prob->constraint_lower_bound, vm * 8);
-  h2d(P->uc, prob->constraint_upper_bound, vm * 8);
-  if (prob->primal_start) {
-    P->xs = ar.take<double>(vn);
-    h2d(P->xs, prob->primal_start, vn * 8);
-  }
-  if (prob->dual_start) {
-    P->ys = ar.take<double>(vm);
-    h2d(P->ys, prob->dual_start, vm * 8);
+  {
+    // the vectors, in the order of the format
+    const size_t most = std::max(vn, vm);
+    Scratch sc{P->perm_m || P->perm_n ? dev_alloc(most * 8, st) : nullptr, st};
+    auto vec = [&](double *dst, const double *src, int count, const int *perm) {
+      if (count == 0) return;
+      h2d(perm ? sc.p : dst, src, (size_t)count * 8);
+      if (perm) launch_gather(count, (const double *)sc.p, perm, dst, st);
+    };
+    vec(P->c, prob->objective_vector, n, P->perm_n);
+    vec(P->lv, prob->variable_lower_bound, n, P->perm_n);
+    vec(P->uv, prob->variable_upper_bound, n, P->perm_n);
+    vec(P->lc, prob->constraint_lower_bound, m, P->perm_m);
+    vec(P->uc, prob->constraint_upper_bound, m, P->perm_m);
+    if (prob->primal_start) {
+      P->xs = ar.take<double>(vn);
+      vec(P->xs, prob->primal_start, n, P->perm_n);
+    }
+    if (prob->dual_start) {
+      P->ys = ar.take<double>(vm);
+      vec(P->ys, prob->dual_start, m, P->perm_m);
+    }
   }
   PDLP_CUDA(cudaStreamSynchronize(st));  // host staging (plans) must outlive the copies
   return P.release();

@@ -9,7 +9,6 @@
 
 #include <array>
 #include <map>
-#include <mutex>
 #include <memory>
 #include <new>
 #include <string>
@@ -20,6 +19,8 @@
 #include "cupdlpx_types.h"
 #include "spmv.cuh"
 #include "spmv_pipe.cuh"
+#include "strip.cuh"
+#include "team.cuh"
 
 namespace pdlp {
 
@@ -32,9 +33,19 @@ struct DevCsrT {
   T *val = nullptr;
   SpmvPlan plan;
   PipePlan pipe;
+  // the strip format: then ptr holds the front's row offsets and col / val
+  // strip.store elements; otherwise plain CSR with the two plans above
+  StripPlan strip;
   bool pipe_on = false;  // this matrix's SpMVs run on the pipelined kernel
+  // elements of col / val
+  size_t store() const { return strip.on ? (size_t)strip.store : (size_t)nnz; }
 };
 using DevCsr = DevCsrT<double>;
+
+template <class T>
+StripMat<T> strip_mat(const DevCsrT<T> &A) {
+  return StripMat<T>{A.ptr, A.col, A.val, A.rows, A.strip};
+}
 
 // Everything a kernel of the iteration needs, passed by value (kernel
 // parameter space), so concurrent solves never share a global.
@@ -96,6 +107,7 @@ struct Dev {
   // so the iteration kernels load them instead of dividing per block
   const double *hw;
   int hw_len;
+  int fp32_sums;  // Fp32Sums: how an FP32 matrix is summed (see strip.cuh)
 };
 
 // The power method always runs in FP64 on the FP64 scaled matrix.
@@ -109,6 +121,9 @@ struct PowDev {
   double sv_tol;
 };
 
+// LPs below this many non-zeros run their loop and power method as a resident
+// team (team.cuh).
+constexpr long kTeamMaxNnz = 1L << 22;
 constexpr int kMiscPart = 4096;
 constexpr int kHalpernTable = 1 << 16;
 
@@ -122,7 +137,7 @@ struct IterFlags {
   bool eval, infeas, restart_check, maybe_restart, major_kernel, fpe, fpe_restart_only;
 };
 
-inline IterFlags iteration_flags(int t, int F) {
+__host__ __device__ inline IterFlags iteration_flags(int t, int F) {
   IterFlags f;
   bool top_major = t > 0 && t % F == 0;  // is_this_major_iteration at loop top
   f.eval = top_major || t == 0 || t % print_frequency(t) == 0;
@@ -137,8 +152,11 @@ inline IterFlags iteration_flags(int t, int F) {
 }
 
 // An LP resident in HBM, as the caller gave it (unscaled): A and its
-// transpose in CSR with their SpMV plans, bounds, objective, warm start.
-// Read-only once built; any number of solves can run from it.  A derived
+// transpose in the strip format (in CSR with the fused and pipelined kernels'
+// plans when PDLP_STEP_KERNEL forces one of those), bounds, objective, warm
+// start.  In the strip format constraints and variables stand in the order
+// of their rows' lengths (strip.cuh): everything of a solve is in that order
+// but its inputs and results.  Read-only once built; any number of solves can run from it.  A derived
 // problem (refinement) shares the matrices of its parent and owns only its
 // vectors.
 struct DevProblem {
@@ -146,6 +164,8 @@ struct DevProblem {
   DevCsr A, AT;  // original values; plan scratch (lcnt/lsum) is per solve
   double *c = nullptr, *lv = nullptr, *uv = nullptr, *lc = nullptr, *uc = nullptr;
   double *xs = nullptr, *ys = nullptr;  // warm start (unscaled) or null
+  // position -> original index of constraints and variables (null: the same)
+  const int *perm_m = nullptr, *perm_n = nullptr;
   double cnorm_l2 = 0, cnorm_linf = 0, bnorm_l2 = 0, bnorm_linf = 0, c0 = 0;
   // correction LP of a refinement round: centre and original objective data
   const double *shift_x = nullptr, *shift_y = nullptr, *orig_c = nullptr;
@@ -160,27 +180,13 @@ struct DevProblem {
   // (pdlp_device_problem_t) switches to the per-thread stream: its solves
   // return only after their work on the problem has finished.
   cudaStream_t owner = cudaStreamPerThread;
-  // SpMV kernel per matrix and precision (index: 0 FP64, 1 FP32, 2 FP32
-  // matrix), chosen by the first solve of each precision: -1 not yet
-  // chosen, 0 fused, 1 pipelined; {A, A^T}
-  mutable int kernel_choice[3][2] = {{-1, -1}, {-1, -1}, {-1, -1}};
-  // fingerprint of the structure the kernel choice depends on: m, n, nnz
-  // and the row lengths of A and A^T (FNV-1a over both row-pointer arrays)
-  uint64_t shape_key = 0;
-  mutable std::mutex tune_mu;
+  bool strips = false;  // strip format (else plain CSR)
+  int nsm = kNumSms;  // SMs of the device it was uploaded to
   ~DevProblem();
 };
 
 // Validate, transpose (host), plan and upload.  Throws on a malformed CSR.
 DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st);
-
-// Kernel choices of this process by structure fingerprint and precision
-// index: every problem of one structure runs the kernels the first timed
-// solve of that structure chose.  lookup fills c and returns true when a
-// choice is recorded; settle records c unless one is already recorded, and
-// returns the recorded choice in c.
-bool lookup_kernel_choice(uint64_t key, int prec, int c[2]);
-void settle_kernel_choice(uint64_t key, int prec, int c[2]);
 
 // KKT measures of a point, in the reference's definitions.
 struct Kkt {
@@ -228,8 +234,10 @@ class Solve {
   void run();
   // Reduced cost, unscale, copy to a malloc'ed result.
   cupdlpx_result_t *result();
-  // Unscaled FP64 primal, dual and dual slack into device buffers.
-  void result_device(double *x, double *y, double *lam);
+  // Unscaled FP64 primal, dual and dual slack into device buffers, in the
+  // solve's order or at the places pn / pm give.
+  void result_device(double *x, double *y, double *lam, const int *pn = nullptr,
+                     const int *pm = nullptr);
   // KKT of the given unscaled point (device buffers) on this solve's problem;
   // meaningful for a solve prepared without rescaling.
   Kkt evaluate(const double *x, const double *y, const double *lam);
@@ -299,25 +307,19 @@ class Solve {
   int timed_iteration(int t0, int t1) const;
   void read_timing(int slot);
   void power_method();
+  void power_method_team();
+  void run_team(int t, int t1);
+  void run_graphs(int t, int L);
+  void check_team_error() const;
   void check_pipe_errors() const;
-  // kernel choice per matrix: apply (pipe_A, pipe_T) to the matrices and the
-  // fold counts; tune_kernels times both kernels on the step epilogues
-  void apply_kernels(bool pipe_A, bool pipe_T);
-  void tune_kernels();
-  int precision_index() const { return sizeof(T) == 4 ? 1 : sizeof(M) == 4 ? 2 : 0; }
-  bool tuned_ = false;
+  void apply_kernels(bool pipe);
 
  public:
-  // kernels per matrix after tuning (pipelined or not) and the tuning's
-  // measured ms per launch: {A fused, A pipelined, A^T fused, A^T pipelined}
-  // (zeros when the choice came from the problem's cache or an override)
-  bool pipe_A() const { return A64_.pipe_on; }
-  bool pipe_AT() const { return AT64_.pipe_on; }
-  double tune_ms(int i) const { return tune_ms_[i]; }
+  // kernels of the products: 0 fused, 1 pipelined, 2 strip
+  int kernel_A() const { return A64_.strip.on ? 2 : A64_.pipe_on ? 1 : 0; }
+  int kernel_AT() const { return AT64_.strip.on ? 2 : AT64_.pipe_on ? 1 : 0; }
 
  private:
-  double tune_ms_[4] = {0, 0, 0, 0};
-
   pdhg_parameters_t p_;
   cudaStream_t st_;
   const DevProblem &P_;
@@ -349,6 +351,12 @@ class Solve {
   double rescale_sec_ = 0.0, loop_sec_ = 0.0;
   long launches_ = 0;
   bool snapshot_ = false;
+  // resident team: its CTAs (0: one kernel per product) and buffers
+  int team_ = 0;
+  unsigned *team_count_ = nullptr;
+  int *team_err_ = nullptr;
+  int team_n_ = 0;  // iterations timed in a team and their summed step times
+  double team_primal_ms_ = 0.0, team_dual_ms_ = 0.0;
   void *snap_mem_ = nullptr;
   double fixed_cb_ = 0.0, fixed_ob_ = 0.0;
 };
@@ -359,10 +367,11 @@ extern template class Solve<double, float>;
 
 // GPU rescaling (precond.cu): Ruiz, Pock-Chambolle, bound/objective scaling
 // on the device copies of A, A^T, c, bounds.  Fills Dr, Dc, cb, ob.
+// tmp_n, tmp_m: two work vectors each.
 void gpu_rescale(const pdhg_parameters_t &p, DevCsr &A, DevCsr &AT, double *c,
                  double *lv, double *uv, double *lc, double *uc, double *Dr,
-                 double *Dc, double *cb, double *ob, double *tmp_n, double *tmp_m,
-                 double *part, cudaStream_t st, double fixed_cb = 0.0,
+                 double *Dc, double *cb, double *ob, double *const (&tmp_n)[2],
+                 double *const (&tmp_m)[2], double *part, cudaStream_t st, double fixed_cb = 0.0,
                  double fixed_ob = 0.0);
 
 // Host buffer whose elements are left uninitialised on resize (filled
@@ -394,6 +403,10 @@ void device_transpose(int m, int n, int nnz, const int *ptr, const int *col, con
 void host_transpose(int m, int n, const int *ap, const int *aj, const double *ax,
                     std::vector<int> &tp, host_buf<int> &tj, host_buf<double> &tx);
 
+// dst[i] = src[perm[i]] and dst[perm[i]] = src[i]
+void launch_gather(int n, const double *src, const int *perm, double *dst, cudaStream_t st);
+void launch_scatter(int n, const double *src, const int *perm, double *dst, cudaStream_t st);
+
 // Options of the mixed-precision solve (refine.cu).
 struct RefineOptions {
   int max_rounds = 8;       // outer refinement rounds
@@ -403,7 +416,6 @@ struct RefineOptions {
 
 struct RefineReport {
   int kernel_A = 0, kernel_AT = 0;  // SpMV kernels of the FP32 rounds (1: pipelined)
-  double tune_ms[4] = {0, 0, 0, 0};
   int rounds = 0;
   int power_iterations = 0;
   double sigma_max = 0.0;

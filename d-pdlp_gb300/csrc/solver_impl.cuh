@@ -49,27 +49,33 @@ enum EvalMode { kEvalCheck = 0, kEvalIterLimit = 1, kEvalOnly = 2 };
 
 // ======================================================= element kernels
 
-// Ray projection + infinity norms (utils.cu:533-559, :744-748)
+// Ray projection + infinity norms (utils.cu:533-559, :744-748) of entries
+// first, first + stride, ...; a: largest |dx|, |dy|
 template <class T>
-__global__ void __launch_bounds__(kThreads) k_ray_project(Dev<T> d) {
-  if (d.ctl->done) return;
-  __shared__ double red[24];
-  double a[2] = {0.0, 0.0};
-  long stride = (long)gridDim.x * kThreads;
-  for (long j = blockIdx.x * (long)kThreads + threadIdx.x; j < d.n; j += stride) {
+__device__ __forceinline__ void ray_project(const Dev<T> &d, long first, long stride,
+                                            double (&a)[2]) {
+  for (long j = first; j < d.n; j += stride) {
     T v = d.dx[j];
     if (isfinite(d.lv[j])) v = fmax(v, T(0));
     if (isfinite(d.uv[j])) v = fmin(v, T(0));
     d.dx[j] = v;
     a[0] = fmax(a[0], fabs((double)v));
   }
-  for (long i = blockIdx.x * (long)kThreads + threadIdx.x; i < d.m; i += stride) {
+  for (long i = first; i < d.m; i += stride) {
     T v = d.dy[i];
     if (!isfinite(d.lc[i])) v = fmin(v, T(0));
     if (!isfinite(d.uc[i])) v = fmax(v, T(0));
     d.dy[i] = v;
     a[1] = fmax(a[1], fabs((double)v));
   }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_ray_project(Dev<T> d) {
+  if (d.ctl->done) return;
+  __shared__ double red[24];
+  double a[2] = {0.0, 0.0};
+  ray_project(d, blockIdx.x * (long)kThreads + threadIdx.x, (long)gridDim.x * kThreads, a);
   block_reduce_fields<2, 3u>(a, red);
   if (threadIdx.x == 0) {
     d.p_i0[blockIdx.x] = a[0];
@@ -89,16 +95,14 @@ __global__ void __launch_bounds__(kThreads) k_ray_project_fin(Dev<T> d) {
   }
 }
 
-// Restart copy + distances (pdlp_core_op.cu:577-591, :621-632)
+// Restart copy + squared distances (pdlp_core_op.cu:577-591, :621-632) of
+// entries first, first + stride, ...
 template <class T>
-__global__ void __launch_bounds__(kThreads) k_restart(Dev<T> d, T *xcur, T *ycur) {
-  if (d.ctl->done || !d.ctl->do_restart) return;
-  __shared__ double red[24];
-  double a[2] = {0.0, 0.0};
-  long stride = (long)gridDim.x * kThreads;
+__device__ __forceinline__ void restart_copy(const Dev<T> &d, T *xcur, T *ycur, long first,
+                                             long stride, double (&a)[2]) {
   // polishing restarts one side (reference perform_primal / dual_restart)
   if (d.polish != 2)
-    for (long j = blockIdx.x * (long)kThreads + threadIdx.x; j < d.n; j += stride) {
+    for (long j = first; j < d.n; j += stride) {
       T xh = d.xhat[j];
       double dd = (double)xh - (double)d.x0[j];
       a[0] += dd * dd;
@@ -106,13 +110,22 @@ __global__ void __launch_bounds__(kThreads) k_restart(Dev<T> d, T *xcur, T *ycur
       xcur[j] = xh;
     }
   if (d.polish != 1)
-    for (long i = blockIdx.x * (long)kThreads + threadIdx.x; i < d.m; i += stride) {
+    for (long i = first; i < d.m; i += stride) {
       T yh = d.yhat[i];
       double dd = (double)yh - (double)d.y0[i];
       a[1] += dd * dd;
       d.y0[i] = yh;
       ycur[i] = yh;
     }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_restart(Dev<T> d, T *xcur, T *ycur) {
+  if (d.ctl->done || !d.ctl->do_restart) return;
+  __shared__ double red[24];
+  double a[2] = {0.0, 0.0};
+  restart_copy(d, xcur, ycur, blockIdx.x * (long)kThreads + threadIdx.x,
+               (long)gridDim.x * kThreads, a);
   block_reduce_fields<2, 0u>(a, red);
   if (threadIdx.x == 0) {
     d.p_rs[blockIdx.x] = a[0];
@@ -120,17 +133,13 @@ __global__ void __launch_bounds__(kThreads) k_restart(Dev<T> d, T *xcur, T *ycur
   }
 }
 
-// PID primal-weight update (pdlp_core_op.cu:593-619)
+// PID primal-weight update (pdlp_core_op.cu:593-619) of the restart at
+// iteration t; ps, ds: squared distances moved.  One thread.
 template <class T>
-__global__ void __launch_bounds__(kThreads) k_restart_fin(Dev<T> d, int off) {
+__device__ void restart_scalars(const Dev<T> &d, int t, double ps, double ds) {
   Ctl *c = d.ctl;
-  if (c->done || !c->do_restart) return;
-  __shared__ double sm[32];
-  double ps = block_fold<false>(d.p_rs, d.ew_grid, sm);
-  double ds = block_fold<false>(d.p_rs + d.ew_grid, d.ew_grid, sm);
-  if (threadIdx.x != 0) return;
   if (d.polish) {  // polishing keeps the primal weight
-    c->restart_t = c->t_base + off;
+    c->restart_t = t;
     c->last_trial_fixed_point_error = INFINITY;
     return;
   }
@@ -154,22 +163,25 @@ __global__ void __launch_bounds__(kThreads) k_restart_fin(Dev<T> d, int off) {
     c->best_primal_weight = c->primal_weight;
   }
   set_steps(c);
-  c->restart_t = c->t_base + off;
+  c->restart_t = t;
   c->last_trial_fixed_point_error = INFINITY;
 }
 
-// Fixed-point error (pdlp_core_op.cu:677-695) + restart bookkeeping
-// (solver.cu:89-95)
 template <class T>
-__global__ void __launch_bounds__(kThreads) k_fpe_fin(Dev<T> d, int restart_only) {
+__global__ void __launch_bounds__(kThreads) k_restart_fin(Dev<T> d, int off) {
   Ctl *c = d.ctl;
-  if (c->done) return;
-  if (restart_only && !c->do_restart) return;
+  if (c->done || !c->do_restart) return;
   __shared__ double sm[32];
-  double pn2 = fold_site<false>(d.p_pstep, d.nblkT, d.lp_pstep, d.nlongT, 0, sm);
-  double dn2 = fold_site<false>(d.p_dstep, d.nblkA, d.lp_dstep, d.nlongA, 0, sm);
-  double cross = fold_site<false>(d.p_fpe, d.nblkT, d.lp_fpe, d.nlongT, 0, sm);
-  if (threadIdx.x != 0) return;
+  double ps = block_fold<false>(d.p_rs, d.ew_grid, sm);
+  double ds = block_fold<false>(d.p_rs + d.ew_grid, d.ew_grid, sm);
+  if (threadIdx.x == 0) restart_scalars(d, c->t_base + off, ps, ds);
+}
+
+// Fixed-point error (pdlp_core_op.cu:677-695) + restart bookkeeping
+// (solver.cu:89-95) from |dx|^2, |dy|^2 and <A^T dy, dx>.  One thread.
+template <class T>
+__device__ void fpe_scalars(const Dev<T> &d, double pn2, double dn2, double cross) {
+  Ctl *c = d.ctl;
   double pn = sqrt(pn2), dn = sqrt(dn2);
   double w = c->primal_weight;
   if (d.polish == 1) {  // reference compute_primal_fixed_point_error
@@ -187,32 +199,45 @@ __global__ void __launch_bounds__(kThreads) k_fpe_fin(Dev<T> d, int restart_only
   }
 }
 
-// Evaluation: KKT scalars, optional ray statistics, termination test,
-// restart decision, trace record (utils.cu:639-813, :239-293; solver.cu:59-83)
+// |dx|^2, |dy|^2 and the cross term from their partials, by one block.
 template <class T>
-__global__ void __launch_bounds__(kThreads)
-    k_eval_fin(Dev<T> d, int off, int infeas, int restart_check, int mode) {
+__device__ __forceinline__ void fold_fpe(const Dev<T> &d, double *sm, double &pn2, double &dn2,
+                                         double &cross) {
+  double v[1];
+  fold_site<1, 0u>(d.p_pstep, d.nblkT, d.lp_pstep, d.nlongT, sm, v);
+  pn2 = v[0];
+  fold_site<1, 0u>(d.p_dstep, d.nblkA, d.lp_dstep, d.nlongA, sm, v);
+  dn2 = v[0];
+  fold_site<1, 0u>(d.p_fpe, d.nblkT, d.lp_fpe, d.nlongT, sm, v);
+  cross = v[0];
+}
+
+template <class T>
+__global__ void __launch_bounds__(kThreads) k_fpe_fin(Dev<T> d, int restart_only) {
   Ctl *c = d.ctl;
   if (c->done) return;
+  if (restart_only && !c->do_restart) return;
   __shared__ double sm[32];
+  double pn2, dn2, cross;
+  fold_fpe(d, sm, pn2, dn2, cross);
+  if (threadIdx.x == 0) fpe_scalars(d, pn2, dn2, cross);
+}
+
+// Evaluation: KKT scalars, optional ray statistics, termination test,
+// restart decision, trace record (utils.cu:639-813, :239-293; solver.cu:59-83)
+// of iteration t from the sums over the products.  One thread.
+struct EvalSums {
+  double pr, qsum;      // over A: squared (or largest) primal residual, dual objective terms
+  double dr, cx, lx;    // over A^T: dual residual, c.x, lambda.x
+  double i1max, i1sum;  // ray over A
+  double i2sum, i2max, i2c;  // ray over A^T
+};
+template <class T>
+__device__ void eval_scalars(const Dev<T> &d, Ctl *c, int t, bool infeas, bool restart_check,
+                             int mode, const EvalSums &s) {
   const bool L = d.linf != 0;
-  double pr = L ? fold_site<true>(d.p_e1, d.nblkA, d.lp_e1, d.nlongA, 0, sm)
-                : fold_site<false>(d.p_e1, d.nblkA, d.lp_e1, d.nlongA, 0, sm);
-  double qsum = fold_site<false>(d.p_e1, d.nblkA, d.lp_e1, d.nlongA, 1, sm);
-  double dr = L ? fold_site<true>(d.p_e2, d.nblkT, d.lp_e2, d.nlongT, 0, sm)
-                : fold_site<false>(d.p_e2, d.nblkT, d.lp_e2, d.nlongT, 0, sm);
-  double cx = fold_site<false>(d.p_e2, d.nblkT, d.lp_e2, d.nlongT, 1, sm);
-  double lx = fold_site<false>(d.p_e2, d.nblkT, d.lp_e2, d.nlongT, 2, sm);
-  double i1max = 0, i1sum = 0, i2sum = 0, i2max = 0, i2c = 0;
-  if (infeas) {
-    i1max = fold_site<true>(d.p_i1, d.nblkA, d.lp_i1, d.nlongA, 0, sm);
-    i1sum = fold_site<false>(d.p_i1, d.nblkA, d.lp_i1, d.nlongA, 1, sm);
-    i2sum = fold_site<false>(d.p_i2, d.nblkT, d.lp_i2, d.nlongT, 0, sm);
-    i2max = fold_site<true>(d.p_i2, d.nblkT, d.lp_i2, d.nlongT, 1, sm);
-    i2c = fold_site<false>(d.p_i2, d.nblkT, d.lp_i2, d.nlongT, 2, sm);
-  }
-  if (threadIdx.x != 0) return;
-  const int t = c->t_base + off;
+  const double pr = s.pr, qsum = s.qsum, dr = s.dr, cx = s.cx, lx = s.lx;
+  const double i1max = s.i1max, i1sum = s.i1sum, i2sum = s.i2sum, i2max = s.i2max, i2c = s.i2c;
   const double cbo = d.cb * d.ob;
   c->abs_primal_res = (L ? pr : sqrt(pr)) / d.cb;
   c->abs_dual_res = (L ? dr : sqrt(dr)) / d.ob;
@@ -329,30 +354,80 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+// The sums of an evaluation from their partials, by one block.
+template <class T>
+__device__ __forceinline__ EvalSums fold_eval(const Dev<T> &d, bool infeas, double *sm) {
+  EvalSums s{};
+  double a[2], b[3];
+  if (d.linf) {
+    fold_site<2, 1u>(d.p_e1, d.nblkA, d.lp_e1, d.nlongA, sm, a);
+    fold_site<3, 1u>(d.p_e2, d.nblkT, d.lp_e2, d.nlongT, sm, b);
+  } else {
+    fold_site<2, 0u>(d.p_e1, d.nblkA, d.lp_e1, d.nlongA, sm, a);
+    fold_site<3, 0u>(d.p_e2, d.nblkT, d.lp_e2, d.nlongT, sm, b);
+  }
+  s.pr = a[0];
+  s.qsum = a[1];
+  s.dr = b[0];
+  s.cx = b[1];
+  s.lx = b[2];
+  if (infeas) {
+    fold_site<2, 1u>(d.p_i1, d.nblkA, d.lp_i1, d.nlongA, sm, a);
+    fold_site<3, 2u>(d.p_i2, d.nblkT, d.lp_i2, d.nlongT, sm, b);
+    s.i1max = a[0];
+    s.i1sum = a[1];
+    s.i2sum = b[0];
+    s.i2max = b[1];
+    s.i2c = b[2];
+  }
+  return s;
+}
+
+template <class T>
+__global__ void __launch_bounds__(kThreads)
+    k_eval_fin(Dev<T> d, int off, int infeas, int restart_check, int mode) {
+  Ctl *c = d.ctl;
+  if (c->done) return;
+  __shared__ double sm[32];
+  const EvalSums s = fold_eval(d, infeas, sm);
+  if (threadIdx.x == 0) eval_scalars(d, c, c->t_base + off, infeas, restart_check, mode, s);
+}
+
 // Copy the evaluated iterate into the snapshot when it is the best so far.
 template <class T>
-__global__ void k_snapshot(Dev<T> d) {
-  if (!d.ctl->snap_now) return;
-  long stride = (long)gridDim.x * blockDim.x;
-  for (long j = blockIdx.x * (long)blockDim.x + threadIdx.x; j < d.n; j += stride) {
+__device__ __forceinline__ void snapshot_copy(const Dev<T> &d, long first, long stride) {
+  for (long j = first; j < d.n; j += stride) {
     d.bx[j] = d.xhat[j];
     d.bl[j] = d.lam[j];
   }
-  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < d.m; i += stride)
-    d.by[i] = d.yhat[i];
+  for (long i = first; i < d.m; i += stride) d.by[i] = d.yhat[i];
+}
+template <class T>
+__global__ void k_snapshot(Dev<T> d) {
+  if (!d.ctl->snap_now) return;
+  snapshot_copy(d, blockIdx.x * (long)blockDim.x + threadIdx.x, (long)gridDim.x * blockDim.x);
 }
 
+}  // namespace pdlp
+
+#include "team_loop.cuh"  // the same iterations by a resident team
+
+namespace pdlp {
+
 // Unscale (pdlp_core_op.cu:464-480) into FP64 outputs; the dual slack maps
-// back like the reduced cost (times Dc / ob).
+// back like the reduced cost (times Dc / ob).  pn, pm: where each entry goes
+// (null: its own place).
 template <class T>
-__global__ void k_unscale(Dev<T> d, double *x, double *y, double *lam) {
+__global__ void k_unscale(Dev<T> d, double *x, double *y, double *lam, const int *pn,
+                          const int *pm) {
   long stride = (long)gridDim.x * blockDim.x;
   for (long j = blockIdx.x * (long)blockDim.x + threadIdx.x; j < d.n; j += stride) {
-    x[j] = (double)d.xhat[j] / d.Dc[j] / d.cb;
-    if (lam) lam[j] = (double)d.lam[j] * d.Dc[j] / d.ob;
+    const long o = pn ? pn[j] : j;
+    x[o] = (double)d.xhat[j] / d.Dc[j] / d.cb;
+    if (lam) lam[o] = (double)d.lam[j] * d.Dc[j] / d.ob;
   }
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < d.m; i += stride)
-    y[i] = (double)d.yhat[i] / d.Dr[i] / d.ob;
+    y[pm ? pm[i] : i] = (double)d.yhat[i] / d.Dr[i] / d.ob;
 }
 
 // Scale an original-units point into this solve's scaled space.
@@ -459,7 +534,7 @@ template <class T, class M>
 void Solve<T, M>::alloc() {
   constexpr bool F64 = sizeof(T) == 8;   // iterates in FP64
   constexpr bool M64 = sizeof(M) == 8;   // matrix in FP64
-  const int n = P_.n, m = P_.m, nnz = P_.nnz;
+  const int n = P_.n, m = P_.m;
   const int ew = grid_for((long)n + m, 4);
   const size_t vn = n, vm = m;
   // reduction partials of an SpMV site: one per CTA of the pipelined kernel
@@ -467,12 +542,15 @@ void Solve<T, M>::alloc() {
   const size_t nbA = spmv_partials_max(P_.A), nbT = spmv_partials_max(P_.AT);
   const size_t nlA = spmv_long_rows_max(P_.A), nlT = spmv_long_rows_max(P_.AT);
   Sizer z;
-  z.add<double>(nnz); z.add<double>(nnz);                      // FP64 scaled values
-  if (!M64) { z.add<M>(nnz); z.add<M>(nnz); }                  // iteration values
+  const size_t sA = P_.A.store(), sT = P_.AT.store();
+  z.add<double>(sA); z.add<double>(sT);                        // FP64 scaled values
+  if (!M64) { z.add<M>(sA); z.add<M>(sT); }                    // iteration values
   for (const DevCsr *W : {&P_.A, &P_.AT}) {                    // SpMV scratch of both kernels
     z.add<unsigned>(W->plan.nlong); z.add<double>(W->plan.nblk);
     z.add<unsigned>(W->pipe.nlong); z.add<double>(W->pipe.ntile); z.add<int>(1);
+    z.add<unsigned>(W->strip.nlong); z.add<double>(W->strip.nitem);
   }
+  z.add<unsigned>(64);                                         // team counter, error flag
   for (int i = 0; i < 3; ++i) z.add<double>(vn);               // c lv uv (FP64 scaled)
   for (int i = 0; i < 2; ++i) z.add<double>(vm);               // lc uc
   z.add<double>(vn); z.add<double>(vm);                        // Dc Dr
@@ -501,7 +579,7 @@ void Solve<T, M>::alloc() {
 
   auto mat64 = [&](DevCsr &W, const DevCsr &S) {
     W = S;
-    W.val = ar.take<double>(nnz);
+    W.val = ar.take<double>(S.store());
     W.plan.lcnt = ar.take<unsigned>(S.plan.nlong);
     W.plan.lsum = ar.take<double>(S.plan.nblk);
     if (S.plan.nlong) PDLP_CUDA(cudaMemsetAsync(W.plan.lcnt, 0, (size_t)S.plan.nlong * 4, st_));
@@ -510,9 +588,15 @@ void Solve<T, M>::alloc() {
     W.pipe.err = ar.take<int>(1);
     if (S.pipe.nlong) PDLP_CUDA(cudaMemsetAsync(W.pipe.lcnt, 0, (size_t)S.pipe.nlong * 4, st_));
     PDLP_CUDA(cudaMemsetAsync(W.pipe.err, 0, sizeof(int), st_));
+    W.strip.lcnt = ar.take<unsigned>(S.strip.nlong);
+    W.strip.lsum = ar.take<double>(S.strip.nitem);
+    if (S.strip.nlong) PDLP_CUDA(cudaMemsetAsync(W.strip.lcnt, 0, (size_t)S.strip.nlong * 4, st_));
   };
   mat64(A64_, P_.A);
   mat64(AT64_, P_.AT);
+  team_count_ = ar.take<unsigned>(64);
+  team_err_ = (int *)team_count_ + 32;
+  PDLP_CUDA(cudaMemsetAsync(team_count_, 0, 64 * sizeof(unsigned), st_));
   auto matT = [&](DevCsrT<M> &W, const DevCsr &S64) {
     W.rows = S64.rows;
     W.cols = S64.cols;
@@ -521,8 +605,9 @@ void Solve<T, M>::alloc() {
     W.col = S64.col;
     W.plan = S64.plan;  // shares the per-solve scratch of the FP64 copy
     W.pipe = S64.pipe;
+    W.strip = S64.strip;
     if constexpr (M64) W.val = (M *)S64.val;
-    else W.val = ar.take<M>(nnz);
+    else W.val = ar.take<M>(S64.store());
   };
   matT(A_, A64_);
   matT(AT_, AT64_);
@@ -593,29 +678,21 @@ void Solve<T, M>::alloc() {
   pw_.ctl = d.ctl;
   pw_.hflag = dflag;
   pw_.ew_grid = ew;
-  // kernels: the problem's measured choice for this precision, a forced one,
-  // or the fused kernel until run() measures both
-  int cA = 0, cT = 0;
-  {
-    std::lock_guard<std::mutex> lk(P_.tune_mu);
-    const int *ch = P_.kernel_choice[precision_index()];
-    if (kernel_override() >= 0) {
-      cA = cT = kernel_override();
-      tuned_ = true;
-    } else if (ch[0] >= 0 && ch[1] >= 0) {
-      cA = ch[0];
-      cT = ch[1];
-      tuned_ = true;
-    }
-  }
-  apply_kernels(cA != 0, cT != 0);
+  apply_kernels(kernel_override() == 1);
+  if (P_.strips && P_.nnz > 0 && P_.nnz < kTeamMaxNnz)
+    team_ = team_ctas(P_.A.strip, P_.AT.strip, P_.nsm);
 }
 
+// The kernel of a CSR matrix's products (forced; the strip format has one) and
+// the counts its partials are folded with.
 template <class T, class M>
-void Solve<T, M>::apply_kernels(bool pipe_A, bool pipe_T) {
+void Solve<T, M>::apply_kernels(bool pipe) {
   Dev<T> &d = d_;
-  A64_.pipe_on = A_.pipe_on = pipe_A && P_.A.pipe.ntile > 0;
-  AT64_.pipe_on = AT_.pipe_on = pipe_T && P_.AT.pipe.ntile > 0;
+  A64_.pipe_on = A_.pipe_on = pipe && P_.A.pipe.ntile > 0;
+  AT64_.pipe_on = AT_.pipe_on = pipe && P_.AT.pipe.ntile > 0;
+  d.fp32_sums = (P_.strips ? P_.A.strip.pairs != 0 : pipe) ? kFp32Pairs
+                : P_.tile == 512                              ? kFp32Tiles512
+                                                              : kFp32Tiles;
   d.nblkA = (int)spmv_partials(A64_);
   d.nlongA = (int)spmv_long_rows(A64_);
   d.nblkT = (int)spmv_partials(AT64_);
@@ -624,69 +701,10 @@ void Solve<T, M>::apply_kernels(bool pipe_A, bool pipe_T) {
   pw_.nlongA = d.nlongA;
 }
 
-// The SpMV kernel of each matrix, chosen once per problem and precision.
-// Below kTuneMinNnz non-zeros both matrices take the fused kernel (launches
-// of a few microseconds, where it is never slower).  Above, the step kernel
-// of each matrix (primal step over A^T, dual step over A) is timed on both
-// kernels, 2 warm and 5 timed launches each, CUDA events on the solve's
-// stream, and the pipelined kernel is kept where it is at least 3% faster.
-// The choice is recorded for the structure (settle_kernel_choice), so every
-// later solve of a matrix of that structure in the process runs the same
-// kernels and returns the same bits.  Runs before the first iteration (the
-// step kernels only write the next iterates and x_ref, which the loop
-// writes before it reads them).
-constexpr long kTuneMinNnz = 1L << 22;
-
-template <class T, class M>
-void Solve<T, M>::tune_kernels() {
-  if (tuned_) return;
-  tuned_ = true;
-  std::lock_guard<std::mutex> lk(P_.tune_mu);
-  int *ch = P_.kernel_choice[precision_index()];
-  if (ch[0] < 0 || ch[1] < 0) {
-    if (P_.nnz < kTuneMinNnz) {
-      ch[0] = ch[1] = 0;
-    } else if (!lookup_kernel_choice(P_.shape_key, precision_index(), ch)) {
-      Dev<T> &d = d_;
-      cudaEvent_t e0, e1;
-      PDLP_CUDA(cudaEventCreate(&e0));
-      PDLP_CUDA(cudaEventCreate(&e1));
-      auto timed = [&](auto &&launch) {
-        for (int i = 0; i < 2; ++i) launch();
-        PDLP_CUDA(cudaEventRecord(e0, st_));
-        for (int i = 0; i < 5; ++i) launch();
-        PDLP_CUDA(cudaEventRecord(e1, st_));
-        PDLP_CUDA(cudaEventSynchronize(e1));
-        float ms = 0.f;
-        PDLP_CUDA(cudaEventElapsedTime(&ms, e0, e1));
-        return ms;
-      };
-      PrimalEpi<T, M, false, false, true> pe{d, 0, d.x[0], d.y[0], d.x[1], T(0), T(0), T(0)};
-      DualEpi<T, M, false, false, true> de{d, 0, d.y[0], d.y[1], T(0), T(0), T(0), T(0)};
-      float tf[2] = {0.f, 0.f}, tp[2] = {0.f, 0.f};
-      for (int k = 0; k < 2; ++k) {
-        apply_kernels(k != 0, k != 0);
-        float a = timed([&] { launch_spmv(A_, de, d.p_dstep, d.lp_dstep, st_); });
-        float t = timed([&] { launch_spmv(AT_, pe, d.p_pstep, d.lp_pstep, st_); });
-        (k ? tp : tf)[0] = a;
-        (k ? tp : tf)[1] = t;
-      }
-      cudaEventDestroy(e0);
-      cudaEventDestroy(e1);
-      ch[0] = P_.A.pipe.ntile > 0 && tp[0] < 0.97f * tf[0] ? 1 : 0;
-      ch[1] = P_.AT.pipe.ntile > 0 && tp[1] < 0.97f * tf[1] ? 1 : 0;
-      settle_kernel_choice(P_.shape_key, precision_index(), ch);
-      tune_ms_[0] = tf[0] / 5; tune_ms_[1] = tp[0] / 5;
-      tune_ms_[2] = tf[1] / 5; tune_ms_[3] = tp[1] / 5;
-    }
-  }
-  apply_kernels(ch[0] != 0, ch[1] != 0);
-}
-
 template <class T, class M>
 void Solve<T, M>::prepare() {
   Dev<T> &d = d_;
-  const int n = d.n, m = d.m, nnz = P_.nnz;
+  const int n = d.n, m = d.m;
   auto t0 = std::chrono::steady_clock::now();
   d.c0 = P_.c0;
   d.shifted = P_.shift_x != nullptr;
@@ -725,20 +743,20 @@ void Solve<T, M>::prepare() {
   auto d2d = [&](const void *dst, const void *src, size_t b) {
     if (b) PDLP_CUDA(cudaMemcpyAsync((void *)dst, src, b, cudaMemcpyDeviceToDevice, st_));
   };
-  d2d(A64_.val, P_.A.val, (size_t)nnz * 8);
-  d2d(AT64_.val, P_.AT.val, (size_t)nnz * 8);
+  d2d(A64_.val, P_.A.val, P_.A.store() * 8);
+  d2d(AT64_.val, P_.AT.val, P_.AT.store() * 8);
   d2d(c64_, P_.c, (size_t)n * 8);
   d2d(lv64_, P_.lv, (size_t)n * 8);
   d2d(uv64_, P_.uv, (size_t)n * 8);
   d2d(lc64_, P_.lc, (size_t)m * 8);
   d2d(uc64_, P_.uc, (size_t)m * 8);
   gpu_rescale(p_, A64_, AT64_, c64_, lv64_, uv64_, lc64_, uc64_, (double *)d.Dr,
-              (double *)d.Dc, &d.cb, &d.ob, outx_, outy_, d.p_misc, st_, fixed_cb_, fixed_ob_);
+              (double *)d.Dc, &d.cb, &d.ob, {outx_, outl_}, {outy_, pw_.v[0]}, d.p_misc, st_, fixed_cb_, fixed_ob_);
   int g = grid_for((long)n + m);
   if constexpr (sizeof(M) != 8) {
-    int gz = grid_for(nnz);
-    k_convert<M><<<gz, kThreads, 0, st_>>>(nnz, A64_.val, A_.val);
-    k_convert<M><<<gz, kThreads, 0, st_>>>(nnz, AT64_.val, AT_.val);
+    for (auto [src, dst] : {std::pair{&A64_, &A_}, std::pair{&AT64_, &AT_}})
+      k_convert<M><<<grid_for((long)src->store()), kThreads, 0, st_>>>((long)src->store(), src->val,
+                                                                       dst->val);
     PDLP_LAUNCH_CHECK();
   }
   if constexpr (sizeof(T) != 8) {
@@ -792,18 +810,25 @@ void Solve<T, M>::power_method() {
     std::normal_distribution<double> dist(0.0, 1.0);
     for (int i = 0; i < m; ++i) v0[i] = dist(gen);
   }
-  PDLP_CUDA(cudaMemcpyAsync(w.v[0], v0.data(), (size_t)m * 8, cudaMemcpyHostToDevice, st_));
+  // draw i belongs to the caller's constraint i
+  double *const to = P_.perm_m ? outy_ : w.v[0];
+  PDLP_CUDA(cudaMemcpyAsync(to, v0.data(), (size_t)m * 8, cudaMemcpyHostToDevice, st_));
+  if (P_.perm_m) launch_gather(m, outy_, P_.perm_m, w.v[0], st_);
   k_pm_norm<<<w.ew_grid, kThreads, 0, st_>>>(w, w.v[0]);
   k_pm_norm_fin<<<1, kThreads, 0, st_>>>(w);
   PDLP_LAUNCH_CHECK();
   launches_ += 2;
+  if (TeamTurn turn(team_ > 0); turn) {
+    power_method_team();
+    return;
+  }
   // chunks of power iterations, captured once and replayed until converged
   const int CH = 16;
   auto enqueue = [&](int it) {
     const double *v = w.v[it & 1];
     double *vn = w.v[(it + 1) & 1];
-    launch_spmv(AT64_, PowAtEpi{w, v, 0.0}, nullptr, nullptr, st_);
-    launch_spmv(A64_, PowAEpi{w, v, vn, 0.0}, w.p_pa, w.lp_pa, st_);
+    launch_spmv(AT64_, PowAtEpi<>{w, v, 0.0}, nullptr, nullptr, st_);
+    launch_spmv(A64_, PowAEpi<>{w, v, vn, 0.0}, w.p_pa, w.lp_pa, st_);
     k_pm_dot_fin<<<1, kThreads, 0, st_>>>(w);
     k_pm_resid<<<w.ew_grid, kThreads, 0, st_>>>(w, v, vn);
     k_pm_resid_fin<<<1, kThreads, 0, st_>>>(w);
@@ -836,6 +861,38 @@ void Solve<T, M>::power_method() {
   PDLP_CUDA(cudaStreamSynchronize(st_));
   pm_iters_ = c.pm_iters;
   sigma_max_ = sqrt(c.pm_sigma_sq);
+}
+
+template <class T, class M>
+void Solve<T, M>::power_method_team() {
+  PDLP_CUDA(cudaMemsetAsync(team_count_, 0, sizeof(unsigned), st_));
+  launch_team_power(team_, st_, pw_, strip_mat(A64_), strip_mat(AT64_), {team_count_, team_err_},
+                    p_.sv_max_iter);
+  launches_ += 1;
+  Ctl c;
+  read_ctl(c);
+  check_team_error();
+  pm_iters_ = c.pm_iters;
+  sigma_max_ = sqrt(c.pm_sigma_sq);
+}
+
+template <class T, class M>
+void Solve<T, M>::check_team_error() const {
+  int e = 0;
+  PDLP_CUDA(cudaMemcpyAsync(&e, team_err_, sizeof(int), cudaMemcpyDeviceToHost, st_));
+  PDLP_CUDA(cudaStreamSynchronize(st_));
+  if (e) throw std::runtime_error("resident team: a barrier did not complete within its wait limit");
+}
+
+// Iterations [t, t1) as one launch of a team (t1 - t <= kTeamChunk).
+template <class T, class M>
+void Solve<T, M>::run_team(int t, int t1) {
+  const TeamRun r{{team_count_, team_err_}, snapshot_ ? 1 : 0};
+  const TeamData<T, M> data{d_, strip_mat(A_), strip_mat(AT_), strip_mat(A64_), strip_mat(AT64_)};
+  PDLP_CUDA(cudaMemsetAsync(team_count_, 0, sizeof(unsigned), st_));
+  team_launch(team_, team_loop<T, M>, st_, data, r, t, t1);
+  launches_ += 1;
+  check_team_error();
 }
 
 template <class T, class M>
@@ -1043,8 +1100,8 @@ void Solve<T, M>::read_timing(int slot) {
 
 template <class T, class M>
 double Solve<T, M>::live_primal_ms() const {
-  double s = 0;
-  int k = 0;
+  double s = team_primal_ms_;
+  int k = team_n_;
   for (const auto &x : tsamples_)
     if (x.t + 10 < final_count_) s += x.primal_ms, ++k;
   return k ? s / k : 0.0;
@@ -1052,8 +1109,8 @@ double Solve<T, M>::live_primal_ms() const {
 
 template <class T, class M>
 double Solve<T, M>::live_dual_ms() const {
-  double s = 0;
-  int k = 0;
+  double s = team_dual_ms_;
+  int k = team_n_;
   for (const auto &x : tsamples_)
     if (x.t + 10 < final_count_) s += x.dual_ms, ++k;
   return k ? s / k : 0.0;
@@ -1061,7 +1118,7 @@ double Solve<T, M>::live_dual_ms() const {
 
 template <class T, class M>
 int Solve<T, M>::live_samples() const {
-  int k = 0;
+  int k = team_n_;
   for (const auto &x : tsamples_) k += x.t + 10 < final_count_;
   return k;
 }
@@ -1070,16 +1127,44 @@ template <class T, class M>
 void Solve<T, M>::run() {
   Dev<T> &d = d_;
   const int L = p_.termination_criteria.iteration_limit;
-  const int CH = 100;
-  tune_kernels();
   auto t0 = std::chrono::steady_clock::now();
   k_loop_start<<<1, 1, 0, st_>>>(d.ctl);
   PDLP_LAUNCH_CHECK();
   launches_ += 1;
+  for (int t = 0; t < L && !hflag_->done;) {
+    int t1 = L;
+    if (team_ > 0) t1 = (int)std::min<long>((long)L, (long)t + kTeamChunk);
+    if (TeamTurn turn(team_ > 0); turn) run_team(t, t1);
+    else run_graphs(t, t1);
+    t = t1;
+  }
+  Ctl c;
+  read_ctl(c);
+  team_n_ = c.live_n;
+  team_primal_ms_ = c.live_primal_ns * 1e-6;
+  team_dual_ms_ = c.live_dual_ns * 1e-6;
+  if (!hflag_->done) {
+    // iteration limit: one more evaluation at total_count = L (solver.cu:105-109)
+    k_set_tbase<<<1, 1, 0, st_>>>(d.ctl, L);
+    enqueue_eval(0, false, false, kEvalIterLimit);
+    launches_ += 4;
+    PDLP_CUDA(cudaStreamSynchronize(st_));
+  }
+  loop_sec_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
+  final_count_ = total_count();
+  check_pipe_errors();
+}
+
+// Iterations [t, L) as replayed graphs of 100 iterations, one kernel per
+// product.
+template <class T, class M>
+void Solve<T, M>::run_graphs(int t, const int L) {
+  Dev<T> &d = d_;
+  const int CH = 100;
   cudaEvent_t ev[2];
   PDLP_CUDA(cudaEventCreateWithFlags(&ev[0], cudaEventDisableTiming));
   PDLP_CUDA(cudaEventCreateWithFlags(&ev[1], cudaEventDisableTiming));
-  int t = 0, k = 0;
+  int k = 0;
   while (t < L) {
     if (hflag_->done) break;
     int t1 = (int)std::min<long>((long)L, ((long)t / CH + 1) * CH);
@@ -1110,16 +1195,6 @@ void Solve<T, M>::run() {
   read_timing(1);
   cudaEventDestroy(ev[0]);
   cudaEventDestroy(ev[1]);
-  if (!hflag_->done) {
-    // iteration limit: one more evaluation at total_count = L (solver.cu:105-109)
-    k_set_tbase<<<1, 1, 0, st_>>>(d.ctl, L);
-    enqueue_eval(0, false, false, kEvalIterLimit);
-    launches_ += 4;
-    PDLP_CUDA(cudaStreamSynchronize(st_));
-  }
-  loop_sec_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
-  final_count_ = total_count();
-  check_pipe_errors();
 }
 
 // A stage wait of the pipelined kernel that timed out leaves a flag (the
@@ -1298,7 +1373,8 @@ std::vector<double> Solve<T, M>::trace() const {
 }
 
 template <class T, class M>
-void Solve<T, M>::result_device(double *x, double *y, double *lam) {
+void Solve<T, M>::result_device(double *x, double *y, double *lam, const int *pn,
+                                const int *pm) {
   Dev<T> d = d_;
   if (snapshot_) {  // the best evaluated iterate of the run
     Ctl c;
@@ -1310,7 +1386,7 @@ void Solve<T, M>::result_device(double *x, double *y, double *lam) {
       d.lam = d.bl;
     }
   }
-  k_unscale<T><<<grid_for((long)d.n + d.m), kThreads, 0, st_>>>(d, x, y, lam);
+  k_unscale<T><<<grid_for((long)d.n + d.m), kThreads, 0, st_>>>(d, x, y, lam, pn, pm);
   PDLP_LAUNCH_CHECK();
 }
 
@@ -1332,8 +1408,8 @@ template <class T, class M>
 cupdlpx_result_t *Solve<T, M>::result() {
   Dev<T> &d = d_;
   const int n = d.n, m = d.m;
-  launch_spmv(AT_, ReducedCostEpi<T, M>{d, outl_}, nullptr, nullptr, st_);
-  result_device(outx_, outy_, nullptr);
+  launch_spmv(AT_, ReducedCostEpi<T, M>{d, outl_, P_.perm_n}, nullptr, nullptr, st_);
+  result_device(outx_, outy_, nullptr, P_.perm_n, P_.perm_m);
   launches_ += 2;
   auto *r = (cupdlpx_result_t *)calloc(1, sizeof(cupdlpx_result_t));
   if (!r) throw std::bad_alloc();

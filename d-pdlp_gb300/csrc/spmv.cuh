@@ -99,6 +99,51 @@ inline bool plan_direct(const std::vector<int4> &blk, long nnz) {
   return nnz > 0 && 2 * in >= nnz;
 }
 
+// Per-lane accumulation of a run of products.  FP64 matrices: one FMA per
+// non-zero.  FP32 matrices: a compensated (double-float) sum -- each product
+// split exactly with an FMA, each addition with its rounding error (2Sum,
+// Knuth) -- so rows of tens of thousands of cancelling terms keep close to
+// FP64 accuracy at about 9 FP32 instructions per non-zero, which GB300's
+// FP32 pipe (64x its FP64 rate) absorbs.  The _rn intrinsics keep the
+// compiler from contracting the error terms into FMAs.
+template <class M>
+struct LaneAcc;
+template <>
+struct LaneAcc<double> {
+  double s = 0.0;
+  __device__ __forceinline__ void add(double a, double x) { s = fma(a, x, s); }
+  __device__ __forceinline__ void add_pair(double h, double) { s += h; }
+  __device__ __forceinline__ double hi() const { return s; }
+  __device__ __forceinline__ double lo() const { return 0.0; }
+  __device__ __forceinline__ double total() const { return s; }
+  __device__ __forceinline__ double rounded() const { return s; }
+};
+template <>
+struct LaneAcc<float> {
+  float h = 0.f, l = 0.f;
+  __device__ __forceinline__ void two_sum(float b) {
+    const float s = __fadd_rn(h, b);
+    const float bb = __fsub_rn(s, h);
+    const float e = __fadd_rn(__fsub_rn(h, __fsub_rn(s, bb)), __fsub_rn(b, bb));
+    h = s;
+    l = __fadd_rn(l, e);
+  }
+  __device__ __forceinline__ void add(float a, float x) {
+    const float p = __fmul_rn(a, x);
+    const float pe = fmaf(a, x, -p);  // exact: a x = p + pe
+    two_sum(p);
+    l = __fadd_rn(l, pe);
+  }
+  __device__ __forceinline__ void add_pair(float hb, float lb) {
+    two_sum(hb);
+    l = __fadd_rn(l, lb);
+  }
+  __device__ __forceinline__ float hi() const { return h; }
+  __device__ __forceinline__ float lo() const { return l; }
+  __device__ __forceinline__ double total() const { return (double)h + (double)l; }
+  __device__ __forceinline__ float rounded() const { return __fadd_rn(h, l); }
+};
+
 template <class T>
 __device__ __forceinline__ T ld_stream(const T *p) {
   return __ldcs(p);  // matrix data is read once per sweep: evict first
@@ -523,13 +568,17 @@ __global__ void __launch_bounds__(kThreads,
   }
 }
 
-// Fold per-block and long-row partials of field f of one SpMV site.
-template <bool IS_MAX>
-__device__ double fold_site(const double *part, int nblk, const double *lpart,
-                            int nlong, int f, double *smem) {
-  double a = block_fold<IS_MAX>(part + (long)f * nblk, nblk, smem);
-  double b = block_fold<IS_MAX>(lpart + (long)f * nlong, nlong, smem);
-  return IS_MAX ? fmax(a, b) : a + b;
+// Fold the partials and long-row partials of one SpMV site's NF fields.
+template <int NF, unsigned MAXMASK>
+__device__ __forceinline__ void fold_site(const double *part, int nblk, const double *lpart,
+                                          int nlong, double *smem, double (&out)[NF]) {
+  block_fold_fields<NF, MAXMASK>(part, nblk, smem, out);
+  if (nlong == 0) return;  // the same for every thread
+  double l[NF];
+  block_fold_fields<NF, MAXMASK>(lpart, nlong, smem, l);
+#pragma unroll
+  for (int f = 0; f < NF; ++f)
+    out[f] = ((MAXMASK >> f) & 1u) ? fmax(out[f], l[f]) : out[f] + l[f];
 }
 
 }  // namespace pdlp

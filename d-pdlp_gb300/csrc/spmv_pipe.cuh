@@ -173,51 +173,6 @@ __device__ __forceinline__ unsigned ticket_release(unsigned *p) {
   return prev;
 }
 
-// Per-lane accumulation of a run of products.  FP64 matrices: one FMA per
-// non-zero.  FP32 matrices: a compensated (double-float) sum -- each product
-// split exactly with an FMA, each addition with its rounding error (2Sum,
-// Knuth) -- so rows of tens of thousands of cancelling terms keep close to
-// FP64 accuracy at about 9 FP32 instructions per non-zero, which GB300's
-// FP32 pipe (64x its FP64 rate) absorbs.  The _rn intrinsics keep the
-// compiler from contracting the error terms into FMAs.
-template <class M>
-struct LaneAcc;
-template <>
-struct LaneAcc<double> {
-  double s = 0.0;
-  __device__ __forceinline__ void add(double a, double x) { s = fma(a, x, s); }
-  __device__ __forceinline__ void add_pair(double h, double) { s += h; }
-  __device__ __forceinline__ double hi() const { return s; }
-  __device__ __forceinline__ double lo() const { return 0.0; }
-  __device__ __forceinline__ double total() const { return s; }
-  __device__ __forceinline__ double rounded() const { return s; }
-};
-template <>
-struct LaneAcc<float> {
-  float h = 0.f, l = 0.f;
-  __device__ __forceinline__ void two_sum(float b) {
-    const float s = __fadd_rn(h, b);
-    const float bb = __fsub_rn(s, h);
-    const float e = __fadd_rn(__fsub_rn(h, __fsub_rn(s, bb)), __fsub_rn(b, bb));
-    h = s;
-    l = __fadd_rn(l, e);
-  }
-  __device__ __forceinline__ void add(float a, float x) {
-    const float p = __fmul_rn(a, x);
-    const float pe = fmaf(a, x, -p);  // exact: a x = p + pe
-    two_sum(p);
-    l = __fadd_rn(l, pe);
-  }
-  __device__ __forceinline__ void add_pair(float hb, float lb) {
-    two_sum(hb);
-    l = __fadd_rn(l, lb);
-  }
-  __device__ __forceinline__ float hi() const { return h; }
-  __device__ __forceinline__ float lo() const { return l; }
-  __device__ __forceinline__ double total() const { return (double)h + (double)l; }
-  __device__ __forceinline__ float rounded() const { return __fadd_rn(h, l); }
-};
-
 // The pipelined step kernel's plan (per matrix): tiles, long rows, grid.
 struct PipePlan {
   int ntile = 0, nlong = 0, grid = 0;

@@ -1,0 +1,589 @@
+// strip.cuh -- the sparse matrix format of the solver and its product kernel.
+//
+// Replaces the reference's cusparseSpMV(CSR_ALG2) calls
+// (src/pdlp_core_op.cu:501-504, :534-537, :671-674, :801-804;
+// src/utils.cu:134-140, :645-653, :750-758) and the element kernels after
+// them, as spmv.cuh does on plain CSR.
+//
+// The upload orders the rows of A and of A^T (the constraints and the
+// variables) by decreasing length, stably, and the solve works in that order
+// throughout; only its inputs and results are permuted.  Then
+//   * rows of at most kStripRow non-zeros form strips of 32 consecutive rows
+//     of (nearly) one length, stored element-major: element k of the strip's
+//     rows is 32 consecutive columns and values.  A warp takes a strip, a
+//     lane a row: every load of the matrix and of the per-row vectors is
+//     coalesced, a row's sum stays in its lane's registers (no shared memory,
+//     no barrier, no cross-lane sum), and the epilogue runs with all lanes.
+//     GB300 issues one FP64 warp instruction per 16 cycles and SM whatever
+//     lanes are active, so the one FMA per non-zero and the full epilogues
+//     are what an FP64 product can cost least.  A matrix with too few rows
+//     to give the chip's warps a strip each has 2, 4 or 8 lanes to a row (and
+//     16, 8 or 4 rows to a strip): there the time is the chain of a strip's
+//     loads (about 1,300 cycles for four elements), not the issue slots;
+//   * longer rows come first (the front), in CSR order: a warp takes items of
+//     consecutive rows of together up to kStripItem non-zeros (lanes stride a
+//     row, its lane sums are added across lanes in FP64, and the item's rows
+//     run their epilogues together), or an eighth of a chunk of a longer row
+//     (32 of every 256 elements), whose sums are added in order by the last
+//     one to finish (atomic ticket).
+// Shorter rows of a strip are padded with column -1, which is skipped.
+// Items and strips are dealt to the warps of a fixed grid in a fixed order,
+// so every sum has a fixed order and results are bitwise reproducible.
+//
+// FP32 sums.  An FP32 solve's path depends on the rounding of its sums (the
+// 20M-non-zero power-law LP takes 55,200 or 69,400 iterations to 1e-4 with two
+// orders of the same products), so FP32 matrices keep the order that the fused
+// kernel gives them, or the FP32 pairs of the pipelined one (kTeamMaxNnz
+// non-zeros or more, and no front: the rows that kernel is the faster one
+// for): a row's elements are folded in segments that end at
+// fixed distances from the start of the row's tile of that kernel's plan, and
+// the segments are added in order.  StripHost::sums holds, per row, the
+// segment length and the row's phase in it, or the number of lanes that the
+// kernel strides a long row with.
+#pragma once
+
+#include <algorithm>
+#include <vector>
+
+#include "common.cuh"
+#include "spmv.cuh"
+#include "spmv_pipe.cuh"
+
+namespace pdlp {
+
+constexpr int kStripRow = 64;     // longest row of a strip
+constexpr int kStripItem = 1024;  // non-zeros of a front item
+
+struct StripPlan {
+  int on = 0;                  // the matrix is stored in this format
+  int nfront = 0;              // rows longer than kStripRow (they come first)
+  int nitem = 0, nlong = 0, nstrip = 0;
+  int lg = 0;                  // a strip's rows have 1 << lg lanes each
+  // reduction partials: one per item and strip (in that order), whatever warp
+  // took it, or, for matrices too large for a team, one per block
+  int unit_parts = 0;
+  int pairs = 0;               // FP32 sums in pairs (see above)
+  int grid = 0;                // blocks of the product kernel (8 items or strips each)
+  long store = 0;              // stored elements, padding included
+  int *off = nullptr;          // strip s: 32-element columns off[s] .. off[s + 1]
+  // {first row, rows, first element, end}, or for 32 of every 256 elements of
+  // a chunk of a long row {row, -(long id + 1), first element, chunk end}
+  int4 *item = nullptr;
+  int2 *lrow = nullptr;        // per long row {first item, items}
+  const unsigned char *sums = nullptr;  // per row, for FP32 matrices (StripHost::sums)
+  unsigned *lcnt = nullptr;    // per long row arrival counter (per solve, kept at 0)
+  double *lsum = nullptr;      // per item: its sum (per solve)
+};
+
+struct StripHost {
+  std::vector<int> perm;       // position -> original row
+  bool identity = true;        // perm is 0, 1, 2, ...
+  std::vector<int> fptr;       // element offsets of the front's rows
+  std::vector<int4> item;
+  std::vector<int2> lrow;
+  std::vector<int> off;
+  std::vector<unsigned char> sums;  // how each row is summed in FP32
+  bool pairs = false;
+  int lg = 0;
+  long store = 0;
+};
+
+// Lanes of a row (as their logarithm): as many as keep the strips within 8
+// warps of each of `sms` SMs.
+inline int strip_lanes(long rows, int sms) {
+  int lg = 0;
+  while (lg < 3 && (rows << (lg + 1)) <= 32L * 8 * sms) ++lg;
+  return lg;
+}
+
+// FP32 sum of a row: low 4 bits the phase, high 4 the segment length; or
+// kSumStrided + log2(lanes).
+constexpr int kSumStrided = 0xF0;
+
+// Per row of a CSR matrix, from the tiles of the fused kernel (tile and chunk
+// as its plan) ...
+inline void strip_sums_fused(int rows, const int *ptr, int tile, int chunk,
+                             std::vector<unsigned char> &sums) {
+  std::vector<int4> blk;
+  std::vector<int2> lrow;
+  build_plan_host(rows, ptr, tile, blk, lrow, chunk);
+  const bool direct = tile == 1024 && rows > 0 && plan_direct(blk, ptr[rows]);
+  sums.assign(rows, 0);
+  for (const int4 &b : blk) {
+    const int R = b.y - b.x, len = b.w - b.z;
+    if (b.y < 0) {
+      sums[b.x] = kSumStrided + 8;
+    } else if (R > 1 && len <= 64 * R) {
+      const int seg = direct && len >= kDirectMinAvg * R ? 4 : 8;
+      const int from = seg == 4 ? b.z & ~3 : b.z;
+      for (int r = b.x; r < b.y; ++r)
+        sums[r] = (unsigned char)((ptr[r] - from) % seg | seg << 4);
+    } else {
+      int g = 8;  // one row: all 256 threads
+      if (R > 1)
+        for (g = 0; (2 << g) <= kThreads / R && g < 5;) ++g;
+      for (int r = b.x; r < b.y; ++r) sums[r] = (unsigned char)(kSumStrided + g);
+    }
+  }
+}
+
+// ... or of the pipelined kernel (nv row vectors staged; its one-row tiles are
+// summed in pairs too, where the order hardly matters).
+inline void strip_sums_pipe(int rows, const int *ptr, int nv, std::vector<unsigned char> &sums) {
+  std::vector<int4> blk;
+  std::vector<int2> lrow;
+  build_pipe_plan_host(rows, ptr, nv, blk, lrow);
+  sums.assign(rows, 15 << 4);
+  for (const int4 &b : blk) {
+    if (b.y - b.x < 2) continue;
+    const int seg = ((b.w - b.z + kThreads - 1) / kThreads) | 1;
+    for (int r = b.x; r < b.y; ++r) sums[r] = (unsigned char)((ptr[r] - b.z) % seg | seg << 4);
+  }
+}
+
+// Host: order and cut the rows of a CSR matrix; chunk: elements of a long
+// row's chunk (a multiple of 256).
+inline void build_strip_host(int rows, const int *ptr, int sms, int chunk, StripHost &h) {
+  h = StripHost();
+  h.lg = strip_lanes(rows, sms);
+  h.perm.resize(rows);
+  // stable order by decreasing length: the front by sorting, the rest by
+  // counting
+  std::vector<int> front;
+  std::vector<int> count(kStripRow + 2, 0);
+  for (int r = 0; r < rows; ++r) {
+    const int len = ptr[r + 1] - ptr[r];
+    if (len > kStripRow) front.push_back(r);
+    else ++count[kStripRow - len + 1];
+  }
+  std::stable_sort(front.begin(), front.end(), [&](int a, int b) {
+    return ptr[a + 1] - ptr[a] > ptr[b + 1] - ptr[b];
+  });
+  const int nfront = (int)front.size();
+  std::copy(front.begin(), front.end(), h.perm.begin());
+  count[0] = nfront;
+  for (int l = 1; l <= kStripRow + 1; ++l) count[l] += count[l - 1];
+  for (int r = 0; r < rows; ++r) {
+    const int len = ptr[r + 1] - ptr[r];
+    if (len <= kStripRow) h.perm[count[kStripRow - len]++] = r;
+  }
+  for (int i = 0; i < rows && h.identity; ++i) h.identity = h.perm[i] == i;
+  // front: items and chunks.  Items of a small front are smaller, down to a
+  // row each: as many as keep them within 8 warps of each SM (a transport LP
+  // of 854 x 94, 800 FP64 iterations and the set-up: 22.0 -> 17.4 ms)
+  h.fptr.assign(1, 0);
+  for (int i = 0; i < nfront; ++i)
+    h.fptr.push_back(h.fptr.back() + ptr[front[i] + 1] - ptr[front[i]]);
+  const int most = std::min(kStripItem, h.fptr.back() / (8 * sms));
+  for (int i = 0; i < nfront;) {
+    const int a = h.fptr[i], e = h.fptr[i + 1];
+    if (e - a > kStripItem) {
+      h.lrow.push_back(make_int2((int)h.item.size(), 0));
+      for (int k = a; k < e; k += chunk) {
+        const int end = std::min(k + chunk, e);
+        for (int j = k; j < std::min(k + 256, end); j += 32) {
+          h.item.push_back(make_int4(i, -(int)h.lrow.size(), j, end));
+          ++h.lrow.back().y;
+        }
+      }
+      ++i;
+    } else {
+      const int i0 = i;
+      do ++i;
+      while (i < nfront && i - i0 < 32 && h.fptr[i + 1] - a <= most);
+      h.item.push_back(make_int4(i0, i - i0, a, h.fptr[i]));
+    }
+  }
+  // strips
+  long at = ((long)h.fptr.back() + 31) / 32;
+  const int lanes = 1 << h.lg;
+  for (int r = nfront; r < rows; r += 32 / lanes) {
+    h.off.push_back((int)at);
+    // its first row is its longest
+    at += (ptr[h.perm[r] + 1] - ptr[h.perm[r]] + lanes - 1) / lanes;
+  }
+  h.off.push_back((int)at);
+  h.store = at * 32;
+}
+
+// One matrix as the kernels read it (arrays of `store` elements; ptr: the
+// front's rows).
+template <class M>
+struct StripMat {
+  const int *ptr, *col;
+  const M *val;
+  int rows;
+  StripPlan p;
+};
+
+// Matrix data: read once a sweep from HBM (evict first), or kept in L2 by LPs
+// that fit there.
+template <bool STREAM, class T>
+__device__ __forceinline__ T ld_matrix(const T *p) {
+  if constexpr (STREAM) return __ldcs(p);
+  else return __ldg(p);
+}
+
+// A strip row's running sum in its lane.  FP64: two independent chains, so that
+// a lane waits for half of its row's additions; one for rows of two, where the
+// chains' addition would take as long and an issue slot more.
+template <class M, bool PAIR>
+struct StripSum {
+  double s[2] = {0.0, 0.0};
+  __device__ __forceinline__ explicit StripSum(int) {}
+  __device__ __forceinline__ void add(bool second, double a, double x) {
+    if (second) s[1] = fma(a, x, s[1]);
+    else s[0] = fma(a, x, s[0]);
+  }
+  __device__ __forceinline__ double total(bool both) const { return both ? s[0] + s[1] : s[0]; }
+};
+// FP32: segment by segment (see above); PAIR: each in an FP32 pair.
+template <bool PAIR>
+struct StripSum<float, PAIR> {
+  using Acc = typename std::conditional<PAIR, LaneAcc<float>, float>::type;
+  Acc seg{}, all{};
+  int left, len;  // elements until the segment ends, its length
+  __device__ __forceinline__ explicit StripSum(int how) {
+    len = how >> 4;
+    if (len == 15 && !PAIR) len = 8;
+    left = len - (how & 15);
+    if (left <= 0) left = len;
+    if constexpr (!PAIR) all = -0.f;  // -0 + s is s
+  }
+  __device__ __forceinline__ void end() {
+    if constexpr (PAIR) {
+      all.add_pair(seg.hi(), seg.lo());
+      seg = LaneAcc<float>();
+    } else {
+      all += seg;
+      seg = 0.f;
+    }
+  }
+  __device__ __forceinline__ void add(bool, float a, float x) {
+    if (left == 0) {
+      end();
+      left = len;
+    }
+    --left;
+    if constexpr (PAIR) seg.add(a, x);
+    else seg = fmaf(a, x, seg);
+  }
+  __device__ __forceinline__ float total(bool) {
+    end();
+    if constexpr (PAIR) return isfinite(all.lo()) ? all.rounded() : all.hi();
+    else return all;
+  }
+};
+
+template <class Epi, class M>
+__device__ __forceinline__ void strip_epilogue(const Epi &epi, int row, M sum,
+                                               const typename pre_of<Epi>::type &pre,
+                                               double *acc) {
+  if constexpr (has_preload<Epi>::value) epi.row_pre(row, sum, pre, acc);
+  else epi.row(row, sum, acc);
+}
+
+// Four elements of a strip's lanes.
+template <class M>
+struct StripQuad {
+  int c[4];
+  M v[4];
+};
+template <bool STREAM, class M>
+__device__ __forceinline__ void strip_load(const int *col, const M *val, int left,
+                                           StripQuad<M> &q) {
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    q.c[u] = -1;
+    q.v[u] = M(0);
+    if (u < left) {
+      q.c[u] = ld_matrix<STREAM>(col + u * 32);
+      q.v[u] = ld_matrix<STREAM>(val + u * 32);
+    }
+  }
+}
+
+// The start of a strip (a team loads its next one before it waits).
+template <class M>
+struct StripHead {
+  int o0, n;
+  StripQuad<M> q;
+};
+template <bool STREAM, class M>
+__device__ __forceinline__ void strip_head(const StripMat<M> &A, int s, StripHead<M> &x) {
+  x.o0 = x.n = 0;
+  if (s < A.p.nstrip) {
+    x.o0 = __ldg(A.p.off + s);
+    x.n = __ldg(A.p.off + s + 1) - x.o0;
+  }
+  const size_t at = (size_t)x.o0 * 32 + (threadIdx.x & 31);
+  strip_load<STREAM>(A.col + at, A.val + at, x.n, x.q);
+}
+
+// Row of this lane in strip s, and whether it is the lane that ends the row.
+template <class M>
+__device__ __forceinline__ int strip_row(const StripMat<M> &A, int s, bool &ends) {
+  const int lane = threadIdx.x & 31, lg = A.p.lg;
+  const int row = A.p.nfront + s * (32 >> lg) + (lane >> lg);
+  ends = row < A.rows && (lane & ((1 << lg) - 1)) == 0;
+  return row;
+}
+
+// Strip s, by a warp; `head` as strip_head loaded it.
+template <bool STREAM, bool PAIR, class Epi, class M>
+__device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi, double *acc,
+                                           int s, const StripHead<M> &head) {
+  const int lane = threadIdx.x & 31, o0 = head.o0, n = head.n;
+  StripQuad<M> q = head.q;
+  bool ends;
+  const int row = strip_row(A, s, ends);
+  const int *col = A.col + (size_t)o0 * 32 + lane;
+  const M *val = A.val + (size_t)o0 * 32 + lane;
+  typename pre_of<Epi>::type pre;
+  if constexpr (has_preload<Epi>::value)
+    if (ends) epi.preload(row, pre);
+  const int lg = A.p.lg;
+  int how = 0;
+  if constexpr (sizeof(M) == 4) how = row < A.rows ? __ldg(A.p.sums + row) : 8 << 4;
+  StripSum<M, PAIR> sum(how);
+  // four elements ahead, but not in FP32 kernels that stream: at their 40
+  // registers it spills (power-law dual step 0.088 ms ahead, 0.053 without;
+  // FP64 0.083 ahead, 0.087 without)
+  constexpr bool kAhead = sizeof(M) == 8 || !STREAM;
+#pragma unroll 1
+  for (int k = 0; k < n; k += 4) {
+    M x[4];
+    // padding: no load, and 0 times the padding's 0
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      x[u] = M(0);
+      if (q.c[u] >= 0) x[u] = epi.gather(q.c[u]);
+    }
+    StripQuad<M> next;
+    if constexpr (kAhead)
+      strip_load<STREAM>(col + (k + 4) * 32, val + (k + 4) * 32, n - k - 4, next);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (k + u >= n) break;  // the same for every lane
+      if (sizeof(M) == 8 || lg == 0) {
+        if (sizeof(M) == 8 || q.c[u] >= 0) sum.add(u % 2 && n > 2, q.v[u], x[u]);
+      } else {
+        // a row's elements in their order, by every lane of the row
+        const int base = lane & ~((1 << lg) - 1);
+        for (int g = 0; g < (1 << lg); ++g) {
+          const M v = __shfl_sync(0xffffffffu, q.v[u], base + g);
+          const M y = __shfl_sync(0xffffffffu, x[u], base + g);
+          if (__shfl_sync(0xffffffffu, q.c[u], base + g) >= 0) sum.add(false, v, y);
+        }
+      }
+    }
+    if constexpr (kAhead)
+      q = next;
+    else
+      strip_load<STREAM>(col + (k + 4) * 32, val + (k + 4) * 32, n - k - 4, q);
+  }
+  M total = sum.total(n > 2);
+  if constexpr (sizeof(M) == 8)
+    for (int o = 1; o < (1 << lg); o <<= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+  if (ends) strip_epilogue(epi, row, total, pre, acc);
+}
+
+// Sum, by a warp, of elements a + lane, a + lane + step, ... below e of a front
+// row (every lane returns it): lane chains, across lanes in FP64.  The chains
+// of an FP32 matrix are single ones in FP32, or pairs.
+template <bool STREAM, bool PAIR, class Epi, class M>
+__device__ __forceinline__ double strip_warp_sum(const StripMat<M> &A, const Epi &epi, int a,
+                                                 int e, int step) {
+  constexpr int U = 4;
+  const int lane = threadIdx.x & 31;
+  LaneAcc<M> pair[2];
+  M one = M(0);
+#pragma unroll 1
+  for (int k = a + lane; k < e; k += step * U) {
+    int c[U];
+    M v[U], x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k + step * u < e) {
+        c[u] = ld_matrix<STREAM>(A.col + k + step * u);
+        v[u] = ld_matrix<STREAM>(A.val + k + step * u);
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k + step * u < e) x[u] = epi.gather(c[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k + step * u < e) {
+        if constexpr (sizeof(M) == 4 && !PAIR) one = fmaf(v[u], x[u], one);
+        else pair[u % 2].add(v[u], x[u]);
+      }
+  }
+  if constexpr (sizeof(M) == 4 && !PAIR) {
+    return warp_sum((double)one);
+  } else {
+    pair[0].add_pair(pair[1].hi(), pair[1].lo());
+    return warp_sum(pair[0].total());
+  }
+}
+
+// Sum of the whole front row [a, e) as `how` says (FP32, see above).
+template <bool STREAM, class Epi>
+__device__ __forceinline__ float strip_row_sum(const StripMat<float> &A, const Epi &epi, int a,
+                                               int e, int how) {
+  const int lane = threadIdx.x & 31;
+  if (how >= kSumStrided) {
+    const int lanes = 1 << (how - kSumStrided);
+    double t = 0.0;
+    for (int j = lane; j < lanes; j += 32) {
+      float s = 0.f;
+      for (int k = a + j; k < e; k += lanes)
+        s = fmaf(ld_matrix<STREAM>(A.val + k), epi.gather(ld_matrix<STREAM>(A.col + k)), s);
+      t += (double)s;
+    }
+    return (float)warp_sum(t);
+  }
+  // segments: a lane each, added in order
+  const int len = how >> 4, phase = how & 15;
+  const int count = (e - a + phase + len - 1) / len;
+  float all = -0.f;
+  for (int j = 0; j < count; j += 32) {
+    const int k0 = max(a, a - phase + (j + lane) * len), k1 = min(e, a - phase + (j + lane + 1) * len);
+    float s = 0.f;
+    for (int k = k0; k < k1; ++k)
+      s = fmaf(ld_matrix<STREAM>(A.val + k), epi.gather(ld_matrix<STREAM>(A.col + k)), s);
+    const int n = min(32, count - j);
+    for (int g = 0; g < n; ++g) all += __shfl_sync(0xffffffffu, s, g);
+  }
+  return all;
+}
+
+// Front item i, by a warp; `chunk(i, b, sum)` takes the sum of a chunk of a
+// long row (called by every lane).
+template <bool STREAM, bool PAIR, class Epi, class M, class Chunk>
+__device__ __forceinline__ void strip_front(const StripMat<M> &A, const Epi &epi, double *acc,
+                                            int i, Chunk &&chunk) {
+  const int lane = threadIdx.x & 31;
+  const int4 b = __ldg(A.p.item + i);
+  if (b.y < 0) {
+    chunk(i, b, strip_warp_sum<STREAM, PAIR>(A, epi, b.z, b.w, 256));
+    return;
+  }
+  typename pre_of<Epi>::type pre;
+  int a = 0, e = 0;
+  if (lane < b.y) {
+    a = __ldg(A.ptr + b.x + lane);
+    e = __ldg(A.ptr + b.x + lane + 1);
+    if constexpr (has_preload<Epi>::value) epi.preload(b.x + lane, pre);
+  }
+  M mine = M(0);
+#pragma unroll 1
+  for (int r = 0; r < b.y; ++r) {
+    const int ra = __shfl_sync(0xffffffffu, a, r), re = __shfl_sync(0xffffffffu, e, r);
+    M t;
+    if constexpr (sizeof(M) == 4 && !PAIR)
+      t = strip_row_sum<STREAM>(A, epi, ra, re, __ldg(A.p.sums + b.x + r));
+    else
+      t = (M)strip_warp_sum<STREAM, PAIR>(A, epi, ra, re, 32);
+    if (lane == r) mine = t;
+  }
+  if (lane < b.y) strip_epilogue(epi, b.x + lane, mine, pre, acc);
+}
+
+// Partials of one unit's reductions, by its warp.
+template <int NF, unsigned MAXMASK, int NA>
+__device__ __forceinline__ void strip_partials(double (&acc)[NA], double *part, int unit,
+                                               int units) {
+#pragma unroll
+  for (int f = 0; f < NF; ++f)
+    acc[f] = ((MAXMASK >> f) & 1u) ? warp_max(acc[f]) : warp_sum(acc[f]);
+  if ((threadIdx.x & 31) == 0) {
+#pragma unroll
+    for (int f = 0; f < NF; ++f) part[(long)f * units + unit] = acc[f];
+  }
+}
+
+// Partials of a block's: through shared memory, a warp for each reduction.  A
+// shuffle tree in every warp costs 5 FP64 issue slots of 16 cycles per warp and
+// reduction, more than the strips' own arithmetic in the three sums of a
+// transport LP's evaluation; this takes 12 per block and reduction.
+template <int NF, unsigned MAXMASK, int NA>
+__device__ __forceinline__ void strip_block_partials(const double (&acc)[NA], double *part) {
+  __shared__ double all[NF][kThreads];
+  const int lane = threadIdx.x & 31, f = threadIdx.x >> 5;
+#pragma unroll
+  for (int g = 0; g < NF; ++g) all[g][threadIdx.x] = acc[g];
+  __syncthreads();
+  if (f >= NF) return;
+  const bool most = (MAXMASK >> f) & 1u;
+  double v = all[f][lane];
+#pragma unroll
+  for (int k = 32; k < kThreads; k += 32) {
+    const double o = all[f][lane + k];
+    v = most ? fmax(v, o) : v + o;
+  }
+  v = most ? warp_max(v) : warp_sum(v);
+  if (lane == 0) part[(long)f * gridDim.x + blockIdx.x] = v;
+}
+
+// Epi as for spmv_fused (spmv.cuh).  A warp takes one item or strip, so that
+// nothing but the kernel's parameters outlives a strip: in a loop over strips
+// the compiler keeps a dozen vector pointers in registers (spills at 48), at
+// the price of the gathers in flight.
+template <class Epi, bool STREAM, bool PAIR>
+__global__ void __launch_bounds__(kThreads, sizeof(typename Epi::val_t) == 8 ? 5 : 6)
+    spmv_strip(const __grid_constant__ StripMat<typename Epi::val_t> A,
+               double *__restrict__ part, double *__restrict__ lpart, Epi epi) {
+  using M = typename Epi::val_t;
+  constexpr int NF = Epi::NF;
+  __shared__ double sc[4];
+  // the warps of a block are far apart in the (longest first) list
+  const int w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  const int units = A.p.nitem + A.p.nstrip;
+  if (!epi.init()) return;
+  if (threadIdx.x == 0) epi.prologue(sc);
+  __syncthreads();
+  epi.bind(sc);
+  double acc[NF > 0 ? NF : 1];
+#pragma unroll
+  for (int f = 0; f < (NF > 0 ? NF : 1); ++f) acc[f] = 0.0;
+  const int lane = threadIdx.x & 31;
+  auto unit = [&](int i) {
+    if (i >= A.p.nitem) {
+      StripHead<M> head;
+      strip_head<STREAM>(A, i - A.p.nitem, head);
+      strip_rows<STREAM, PAIR>(A, epi, acc, i - A.p.nitem, head);
+      return;
+    }
+    strip_front<STREAM, PAIR>(A, epi, acc, i, [&](int at, const int4 &b, double sum) {
+      if (lane != 0) return;
+      const int lid = -b.y - 1;
+      A.p.lsum[at] = sum;
+      __threadfence();
+      const int2 L = A.p.lrow[lid];
+      if (atomicAdd(A.p.lcnt + lid, 1u) != (unsigned)L.y - 1u) return;
+      __threadfence();
+      double tot = 0.0;
+#pragma unroll 4
+      for (int c = 0; c < L.y; ++c) tot += __ldcg(A.p.lsum + L.x + c);
+      double lacc[NF > 0 ? NF : 1];
+#pragma unroll
+      for (int f = 0; f < (NF > 0 ? NF : 1); ++f) lacc[f] = 0.0;
+      epi.row(b.x, (M)tot, lacc);
+      if constexpr (NF > 0) {
+#pragma unroll
+        for (int f = 0; f < NF; ++f) lpart[f * A.p.nlong + lid] = lacc[f];
+      }
+      A.p.lcnt[lid] = 0u;  // ready for the next launch
+    });
+  };
+  if (w < units) unit(w);
+  if constexpr (NF > 0) {
+    if (A.p.unit_parts) {
+      if (w < units) strip_partials<NF, Epi::MAXMASK>(acc, part, w, units);
+      return;
+    }
+    strip_block_partials<NF, Epi::MAXMASK>(acc, part);
+  }
+}
+
+}  // namespace pdlp

@@ -43,12 +43,10 @@ typedef struct {
   int fp64_finish;            /* 1 when a mixed-precision solve ended with FP64
                                  PDHG warm-started from its best FP64 point */
   int spmv_kernel_A;          /* SpMV kernel of A (dual step and its other
-                                 products): 0 fused, 1 pipelined */
+                                 products): 0 fused, 1 pipelined (the two that
+                                 PDLP_STEP_KERNEL can force), 2 strip */
   int spmv_kernel_AT;         /* the same for A^T (primal step) */
-  double tune_ms[4];          /* the measurement that chose them, ms per
-                                 launch: A fused, A pipelined, A^T fused, A^T
-                                 pipelined (zeros when the choice was reused
-                                 from an earlier solve of the problem) */
+  double tune_ms[4];          /* unused, zeros (kept for the layout) */
 } pdlp_solve_info_t;
 
 /* Arithmetic of the PDHG iteration.

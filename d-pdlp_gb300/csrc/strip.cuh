@@ -529,6 +529,13 @@ __device__ __forceinline__ void strip_block_partials(const double (&acc)[NA], do
 // nothing but the kernel's parameters outlives a strip: in a loop over strips
 // the compiler keeps a dozen vector pointers in registers (spills at 48), at
 // the price of the gathers in flight.
+// Bound by FP64 issue (16 cycles per warp instruction and SM) and by the
+// gathers' L2 requests.  20M non-zeros, ms per launch, before (the faster of
+// the CSR kernels) and now: power-law dual step 0.121 -> 0.083 (FP32 0.101 ->
+// 0.053), primal step 0.152 -> 0.146 (FP32 0.103 -> 0.141: the segments of its
+// sums); transport evaluation over A^T 0.375 -> 0.305, primal step, whose rows
+// have two entries, 0.185 -> 0.203.  5 blocks per SM: 6 spill more, 4 (no
+// spills) take the transport primal step to 0.258.
 template <class Epi, bool STREAM, bool PAIR>
 __global__ void __launch_bounds__(kThreads, sizeof(typename Epi::val_t) == 8 ? 5 : 6)
     spmv_strip(const __grid_constant__ StripMat<typename Epi::val_t> A,

@@ -23,8 +23,8 @@
 // Bound by HBM for short rows and by the gathers of x for long ones.  Before,
 // a thread added each row from global memory, which a warp's longest row held
 // up, and a block's first row came from a 25-step serial search.  Measured,
-// through the entry point: 20M non-zeros with power-law columns 358 -> 166 us,
-// a transport matrix (5,000 entries a row) 1,287 -> 162 us (1.6 TB/s of
+// through the entry point: 20M non-zeros with power-law columns 358 -> 161 us,
+// a transport matrix (5,000 entries a row) 1,280 -> 146 us (1.7 TB/s of
 // matrix and vectors), 20k non-zeros 35 -> 34 us, which is launches and the
 // read of the error flag.
 #include <cuda_runtime.h>
@@ -54,7 +54,11 @@ struct Scratch {
 
 static __device__ __align__(256) Scratch g_scratch;
 
-constexpr int kShort = 32;  // products of a row that one thread adds
+// Products of a row that one thread adds.  A warp's sum costs 5 FP64 issue slots
+// (16 cycles each) for its tree besides its products, so a warp of threads is
+// the cheaper one while a tile has a warp's worth of rows; beyond, it is a
+// serial chain.  9.7M non-zeros in rows of about 34: 200 us with 32, 111 with 64.
+constexpr int kShort = 64;
 
 // First r in [0, rows) with ptr[r] >= key, else rows, by a warp: each step
 // keeps the one of 33 parts that the answer is in.

@@ -1,7 +1,7 @@
 """pdlp_spmv_noalloc at the edges of its tiles and of its two row paths.
 
 The kernel cuts tiles at every 2,048 non-zeros; a thread adds a row of at most
-32 products of a tile, a warp a longer one; a row that crosses tiles is added
+64 products of a tile, a warp a longer one; a row that crosses tiles is added
 from its tiles' partial sums, by a warp when there are more than 32 of them.
 """
 import ctypes as C
@@ -22,7 +22,9 @@ LENGTHS = {
     "rows_end_at_tiles": [2048, 0, 2048, 0, 0],
     "rows_straddle_tiles": [2047, 2, 2046, 3, 1],
     "thread_or_warp_rows": [31, 32, 33, 0, 34] * 40,
+    "thread_or_warp_rows_64": [63, 64, 65, 0, 66] * 40,
     "piece_of_32_or_33": [2016, 64, 1999, 50],
+    "piece_of_64_or_65": [1984, 128, 1919, 130],
     "32_partials_or_33": [7, 2048 * 33, 5, 2048 * 34, 9],
     "empty_rows_at_ends": [0] * 300 + [1] * 2100 + [0] * 300,
     "no_non_zeros": [0, 0, 0],

@@ -20,11 +20,11 @@
 // per tile in the scratch array, and a second kernel adds them in a fixed
 // order, so the result is bitwise reproducible.
 //
-// Bound by HBM for short rows and by the gathers of x for long ones.  Before,
-// a thread added each row from global memory, which a warp's longest row held
-// up, and a block's first row came from a 25-step serial search.  Measured,
-// through the entry point: 20M non-zeros with power-law columns 358 -> 161 us,
-// a transport matrix (5,000 entries a row) 1,280 -> 146 us (1.7 TB/s of
+// Bound by the gathers of x and by each tile's round trips.  Before, a thread
+// added every row of a tile, however long, and a block's first row came from
+// two serial binary searches before its first barrier.  Measured, through the
+// entry point: 20M non-zeros with power-law columns 358 -> 161 us,
+// a transport matrix (5,000 entries a row) 1,280 -> 146 us (1.6 TB/s of
 // matrix and vectors), 20k non-zeros 35 -> 34 us, which is launches and the
 // read of the error flag.
 #include <cuda_runtime.h>

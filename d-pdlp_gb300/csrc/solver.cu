@@ -206,7 +206,8 @@ __global__ void __launch_bounds__(kTeamThreads, kTeamCtasPerSm)
       block_fold_fields<1, 0u>(d.p_pr, d.ew_grid, sm.red, v);
       res = sqrt(v[0]);
     }
-    if (it == maxit || (check && res < d.sv_tol)) break;
+    // `>=`: a limit below zero ends it here too (a launch must always end)
+    if (it >= maxit || (check && res < d.sv_tol)) break;
     team_phase<2, 0u>(
         sd, [](const TeamPower &x) -> const auto & { return x.A; },
         [=](const TeamPower &x) {

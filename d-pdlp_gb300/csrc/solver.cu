@@ -247,9 +247,15 @@ __global__ void __launch_bounds__(kTeamThreads, kTeamCtasPerSm)
   }
 }
 
-void launch_team_power(int ctas, cudaStream_t st, const PowDev &d, const StripMat<double> &A,
+bool launch_team_power(int ctas, cudaStream_t st, const PowDev &d, const StripMat<double> &A,
                        const StripMat<double> &AT, const TeamBar &bar, int maxit) {
-  team_launch(ctas, team_power, st, TeamPower{d, A, AT}, bar, maxit);
+  return team_launch(ctas, team_power, st, TeamPower{d, A, AT}, bar, maxit);
+}
+
+long long team_wait_cycles() {
+  const char *e = getenv("PDLP_TEAM_WAIT_CYCLES");
+  const long long v = e ? atoll(e) : 0;
+  return v > 0 ? v : kBulkWaitCycles;
 }
 
 namespace {

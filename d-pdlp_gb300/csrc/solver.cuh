@@ -307,10 +307,10 @@ class Solve {
   int timed_iteration(int t0, int t1) const;
   void read_timing(int slot);
   void power_method();
-  void power_method_team();
-  void run_team(int t, int t1);
+  bool power_method_team();
+  bool run_team(int t, int t1);
   void run_graphs(int t, int L);
-  void check_team_error() const;
+  bool team_finished(bool launched);
   void check_pipe_errors() const;
   void apply_kernels(bool pipe);
 
@@ -351,8 +351,12 @@ class Solve {
   double rescale_sec_ = 0.0, loop_sec_ = 0.0;
   long launches_ = 0;
   bool snapshot_ = false;
-  // resident team: its CTAs (0: one kernel per product) and buffers
+  // resident team: its CTAs (0: one kernel per product), its buffers, and the
+  // iterates and control block as they were before its launch (state_bytes_
+  // from d_.x[0] on)
   int team_ = 0;
+  void *team_save_ = nullptr;
+  size_t state_bytes_ = 0, snap_bytes_ = 0;
   unsigned *team_count_ = nullptr;
   int *team_err_ = nullptr;
   int team_n_ = 0;  // iterations timed in a team and their summed step times

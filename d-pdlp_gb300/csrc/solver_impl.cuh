@@ -537,6 +537,8 @@ void Solve<T, M>::alloc() {
   const int n = P_.n, m = P_.m;
   const int ew = grid_for((long)n + m, 4);
   const size_t vn = n, vm = m;
+  if (P_.strips && P_.nnz > 0 && P_.nnz < kTeamMaxNnz)
+    team_ = team_ctas(P_.A.strip, P_.AT.strip, P_.nsm);
   // reduction partials of an SpMV site: one per CTA of the pipelined kernel
   // (or per block of the fused kernel) plus one per long row
   const size_t nbA = spmv_partials_max(P_.A), nbT = spmv_partials_max(P_.AT);
@@ -560,8 +562,12 @@ void Solve<T, M>::alloc() {
   }
   for (int i = 0; i < 2; ++i) z.add<T>(vn);                    // lvf uvf
   for (int i = 0; i < 2; ++i) z.add<T>(vm);                    // lcf ucf
+  const size_t state0 = z.bytes;
   for (int i = 0; i < 8; ++i) z.add<T>(vn);                    // x[2] x0 xref xhat lam dx auxn
   for (int i = 0; i < 6; ++i) z.add<T>(vm);                    // y[2] y0 yhat dy auxm
+  z.add<Ctl>(1);
+  state_bytes_ = z.bytes - state0;
+  if (team_) z.add<char>(state_bytes_);
   z.add<double>(vm); z.add<double>(vm); z.add<double>(vn);     // power v[2], g
   z.add<double>(vn); z.add<double>(vm); z.add<double>(vn);     // FP64 outputs x, y, rc/lam
   size_t pa = nbA + nlA + 2, pt = nbT + nlT + 2;
@@ -573,7 +579,7 @@ void Solve<T, M>::alloc() {
   z.add<double>(pa * 2); z.add<double>((size_t)ew);           // power partials
   z.add<double>((size_t)kMiscPart);
   z.add<double>((size_t)kHalpernTable);
-  z.add<Ctl>(1); z.add<double>((size_t)trace_cap_ * 10 + 1);
+  z.add<double>((size_t)trace_cap_ * 10 + 1);
   arena_ = dev_alloc(z.bytes, st_);
   Arena ar{(char *)arena_, 0};
 
@@ -633,6 +639,8 @@ void Solve<T, M>::alloc() {
   d.dx = ar.take<T>(vn); d.auxn = ar.take<T>(vn);
   d.y[0] = ar.take<T>(vm); d.y[1] = ar.take<T>(vm); d.y0 = ar.take<T>(vm);
   d.yhat = ar.take<T>(vm); d.dy = ar.take<T>(vm); d.auxm = ar.take<T>(vm);
+  d.ctl = ar.take<Ctl>(1);  // last of the state that a team's launch changes
+  if (team_) team_save_ = ar.take<char>(state_bytes_);
   pw_.v[0] = ar.take<double>(vm); pw_.v[1] = ar.take<double>(vm); pw_.g = ar.take<double>(vn);
   outx_ = ar.take<double>(vn); outy_ = ar.take<double>(vm); outl_ = ar.take<double>(vn);
   d.nblkA = (int)nbA; d.nlongA = (int)nlA; d.nblkT = (int)nbT; d.nlongT = (int)nlT;
@@ -662,7 +670,6 @@ void Solve<T, M>::alloc() {
     d.hw = hw;
     d.hw_len = kHalpernTable;
   }
-  d.ctl = ar.take<Ctl>(1);
   d.trace = trace_cap_ > 0 ? ar.take<double>((size_t)trace_cap_ * 10) : nullptr;
   d.trace_cap = trace_cap_;
 
@@ -679,8 +686,6 @@ void Solve<T, M>::alloc() {
   pw_.hflag = dflag;
   pw_.ew_grid = ew;
   apply_kernels(kernel_override() == 1);
-  if (P_.strips && P_.nnz > 0 && P_.nnz < kTeamMaxNnz)
-    team_ = team_ctas(P_.A.strip, P_.AT.strip, P_.nsm);
 }
 
 // The kernel of a CSR matrix's products (forced; the strip format has one) and
@@ -810,17 +815,24 @@ void Solve<T, M>::power_method() {
     std::normal_distribution<double> dist(0.0, 1.0);
     for (int i = 0; i < m; ++i) v0[i] = dist(gen);
   }
-  // draw i belongs to the caller's constraint i
-  double *const to = P_.perm_m ? outy_ : w.v[0];
-  PDLP_CUDA(cudaMemcpyAsync(to, v0.data(), (size_t)m * 8, cudaMemcpyHostToDevice, st_));
-  if (P_.perm_m) launch_gather(m, outy_, P_.perm_m, w.v[0], st_);
-  k_pm_norm<<<w.ew_grid, kThreads, 0, st_>>>(w, w.v[0]);
-  k_pm_norm_fin<<<1, kThreads, 0, st_>>>(w);
-  PDLP_LAUNCH_CHECK();
-  launches_ += 2;
+  auto start = [&] {
+    // draw i belongs to the caller's constraint i
+    double *const to = P_.perm_m ? outy_ : w.v[0];
+    PDLP_CUDA(cudaMemcpyAsync(to, v0.data(), (size_t)m * 8, cudaMemcpyHostToDevice, st_));
+    if (P_.perm_m) launch_gather(m, outy_, P_.perm_m, w.v[0], st_);
+    k_pm_norm<<<w.ew_grid, kThreads, 0, st_>>>(w, w.v[0]);
+    k_pm_norm_fin<<<1, kThreads, 0, st_>>>(w);
+    PDLP_LAUNCH_CHECK();
+    launches_ += 2;
+  };
+  start();
   if (TeamTurn turn(team_ > 0); turn) {
-    power_method_team();
-    return;
+    if (power_method_team()) return;
+    // from the start vector again, with a kernel per product
+    static_assert(offsetof(Ctl, pm_iters) == offsetof(Ctl, pm_done) + sizeof(int), "cleared at once");
+    PDLP_CUDA(cudaMemsetAsync(&w.ctl->pm_done, 0, 2 * sizeof(int), st_));
+    hflag_->pm_done = 0;
+    start();
   }
   // chunks of power iterations, captured once and replayed until converged
   const int CH = 16;
@@ -864,35 +876,55 @@ void Solve<T, M>::power_method() {
 }
 
 template <class T, class M>
-void Solve<T, M>::power_method_team() {
+bool Solve<T, M>::power_method_team() {
   PDLP_CUDA(cudaMemsetAsync(team_count_, 0, sizeof(unsigned), st_));
-  launch_team_power(team_, st_, pw_, strip_mat(A64_), strip_mat(AT64_), {team_count_, team_err_},
-                    p_.sv_max_iter);
-  launches_ += 1;
+  const bool launched =
+      launch_team_power(team_, st_, pw_, strip_mat(A64_), strip_mat(AT64_),
+                        {team_count_, team_err_, team_wait_cycles()}, p_.sv_max_iter);
+  launches_ += launched;
+  if (!team_finished(launched)) return false;
   Ctl c;
   read_ctl(c);
-  check_team_error();
   pm_iters_ = c.pm_iters;
   sigma_max_ = sqrt(c.pm_sigma_sq);
+  return true;
 }
 
+// Waits for a team's launch.  False when it did not do its work: the solve
+// then goes on with a kernel per product.
 template <class T, class M>
-void Solve<T, M>::check_team_error() const {
-  int e = 0;
-  PDLP_CUDA(cudaMemcpyAsync(&e, team_err_, sizeof(int), cudaMemcpyDeviceToHost, st_));
-  PDLP_CUDA(cudaStreamSynchronize(st_));
-  if (e) throw std::runtime_error("resident team: a barrier did not complete within its wait limit");
+bool Solve<T, M>::team_finished(bool launched) {
+  int e = 1;
+  if (launched) {
+    PDLP_CUDA(cudaMemcpyAsync(&e, team_err_, sizeof(int), cudaMemcpyDeviceToHost, st_));
+    PDLP_CUDA(cudaStreamSynchronize(st_));
+  }
+  if (e) team_ = 0;
+  return e == 0;
 }
 
-// Iterations [t, t1) as one launch of a team (t1 - t <= kTeamChunk).
+// Iterations [t, t1) as one launch of a team (t1 - t <= kTeamChunk); false
+// when a barrier's wait ran out: the state is then again that of iteration t.
 template <class T, class M>
-void Solve<T, M>::run_team(int t, int t1) {
-  const TeamRun r{{team_count_, team_err_}, snapshot_ ? 1 : 0};
+bool Solve<T, M>::run_team(int t, int t1) {
+  const TeamRun r{{team_count_, team_err_, team_wait_cycles()}, snapshot_ ? 1 : 0};
   const TeamData<T, M> data{d_, strip_mat(A_), strip_mat(AT_), strip_mat(A64_), strip_mat(AT64_)};
+  auto copy = [&](void *dst, const void *src, size_t bytes) {
+    if (bytes) PDLP_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, st_));
+  };
+  // a launch is at least a few ms of iterations, the copies a few us
+  const size_t snap = snapshot_ ? snap_bytes_ : 0;
+  char *const snap_save = (char *)snap_mem_ + snap_bytes_;
+  copy(team_save_, d_.x[0], state_bytes_);
+  copy(snap_save, snap_mem_, snap);
   PDLP_CUDA(cudaMemsetAsync(team_count_, 0, sizeof(unsigned), st_));
-  team_launch(team_, team_loop<T, M>, st_, data, r, t, t1);
-  launches_ += 1;
-  check_team_error();
+  const bool launched = team_launch(team_, team_loop<T, M>, st_, data, r, t, t1);
+  launches_ += launched;
+  if (team_finished(launched)) return true;
+  copy(d_.x[0], team_save_, state_bytes_);
+  copy(snap_mem_, snap_save, snap);
+  hflag_->done = 0;
+  return false;
 }
 
 template <class T, class M>
@@ -949,8 +981,9 @@ template <class T, class M>
 void Solve<T, M>::enable_snapshot() {
   if (snapshot_) return;
   Dev<T> &d = d_;
-  size_t bytes = ((size_t)d.n * 2 + d.m) * sizeof(T) + 1024;
-  void *mem = dev_alloc(bytes, st_);
+  // twice where a team may have to take its changes back
+  snap_bytes_ = align256(((size_t)d.n * 2 + d.m) * sizeof(T) + 1024);
+  void *mem = dev_alloc(team_ ? 2 * snap_bytes_ : snap_bytes_, st_);
   snap_mem_ = mem;
   d.bx = (T *)mem;
   d.bl = d.bx + d.n;
@@ -1134,8 +1167,9 @@ void Solve<T, M>::run() {
   for (int t = 0; t < L && !hflag_->done;) {
     int t1 = L;
     if (team_ > 0) t1 = (int)std::min<long>((long)L, (long)t + kTeamChunk);
-    if (TeamTurn turn(team_ > 0); turn) run_team(t, t1);
-    else run_graphs(t, t1);
+    bool ran = false;
+    if (TeamTurn turn(team_ > 0); turn) ran = run_team(t, t1);
+    if (!ran) run_graphs(t, t1);
     t = t1;
   }
   Ctl c;

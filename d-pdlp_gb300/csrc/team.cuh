@@ -34,6 +34,7 @@ constexpr int kTeamCtasPerSm = 2;
 struct TeamBar {
   unsigned *count;  // arrivals so far (0 at launch)
   int *err;         // set when a wait ran out
+  long long wait;   // its limit in cycles
 };
 
 struct TeamSmem {
@@ -43,8 +44,9 @@ struct TeamSmem {
 };
 
 // Barrier over the team: writes before it are visible after it.  False, in
-// every thread of the CTA, when the wait ran out (kBulkWaitCycles): the caller
-// returns, and the other CTAs' waits run out too.
+// every thread of the CTA, when the wait ran out (TeamBar::wait): the caller
+// returns, and the other CTAs' waits run out too.  The host then takes the
+// launch's work back and repeats it with a kernel per product.
 __device__ __forceinline__ bool team_sync(const TeamBar &b, TeamSmem &sm) {
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -58,7 +60,7 @@ __device__ __forceinline__ bool team_sync(const TeamBar &b, TeamSmem &sm) {
       unsigned seen;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(b.count) : "memory");
       if ((int)(seen - target) >= 0) break;
-      if (clock64() - t0 > kBulkWaitCycles) {
+      if (clock64() - t0 > b.wait) {
         atomicOr(b.err, 1);
         ok = 0;
         break;
@@ -160,8 +162,15 @@ inline int team_ctas(const StripPlan &A, const StripPlan &AT, int nsm) {
   return work <= nsm * kTeamWarps ? std::max(1, std::min(work, nsm)) : nsm * kTeamCtasPerSm;
 }
 
+// Limit of a barrier's wait: that of the mbarrier waits, or
+// PDLP_TEAM_WAIT_CYCLES.  It runs out when the CTAs stop running at the same
+// time, as on a GPU whose time slices are longer.
+long long team_wait_cycles();
+
+// False when the device cannot hold the team's CTAs at once (an SM limit on
+// the process, say): nothing was launched.
 template <class... Params, class... Args>
-void team_launch(int ctas, void (*kernel)(Params...), cudaStream_t st, Args &&...args) {
+bool team_launch(int ctas, void (*kernel)(Params...), cudaStream_t st, Args &&...args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(ctas);
   cfg.blockDim = dim3(kTeamThreads);
@@ -171,7 +180,13 @@ void team_launch(int ctas, void (*kernel)(Params...), cudaStream_t st, Args &&..
   at[0].val.cooperative = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  PDLP_CUDA(cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...));
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, std::forward<Args>(args)...);
+  if (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported) {
+    cudaGetLastError();
+    return false;
+  }
+  PDLP_CUDA(e);
+  return true;
 }
 
 }  // namespace pdlp

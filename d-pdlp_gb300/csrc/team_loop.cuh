@@ -352,8 +352,8 @@ __global__ void __launch_bounds__(kTeamThreads, kTeamCtasPerSm)
   }
 }
 
-// The power method by a team (solver.cu).
-void launch_team_power(int ctas, cudaStream_t st, const PowDev &d, const StripMat<double> &A,
+// The power method by a team (solver.cu); false when it was not launched.
+bool launch_team_power(int ctas, cudaStream_t st, const PowDev &d, const StripMat<double> &A,
                        const StripMat<double> &AT, const TeamBar &bar, int maxit);
 
 }  // namespace pdlp

@@ -12,21 +12,23 @@
 // loads this library holds until the process exits.
 //
 // Tiles are cut at fixed non-zero offsets, so no row plan has to be built or
-// stored: a block loads its tile's columns and values with coalesced loads,
-// gathers x and leaves the products in shared memory; two of its warps look up
-// the rows that start in the tile meanwhile (32 row pointers a step); then a
-// thread adds each short row, and a warp each row (or piece of one) of more
-// than kShort products.  A row that continues past its tile leaves one partial
-// per tile in the scratch array, and a second kernel adds them in a fixed
-// order, so the result is bitwise reproducible.
+// stored.  A thread of a block loads the columns and values of kRun consecutive
+// non-zeros (16 bytes a load where the caller's arrays are aligned), gathers x
+// and keeps the products' factors in registers; two of the block's warps look up
+// the rows that start in the tile meanwhile (32 row pointers a step).  The rows
+// then mark where they start, and each thread folds its non-zeros run by run --
+// a run is one row's share of them -- with one FMA a product, so that none is
+// rounded by itself; the runs meet in shared memory, where a thread adds those
+// of each row, or a warp where there are more than kShort.  A row that continues
+// past its tile leaves one partial per tile in the scratch array, and a second
+// kernel adds them in a fixed order, so the result is bitwise reproducible.
 //
-// Bound by the gathers of x and by each tile's round trips.  Before, a thread
-// added every row of a tile, however long, and a block's first row came from
-// two serial binary searches before its first barrier.  Measured, through the
-// entry point: 20M non-zeros with power-law columns 358 -> 161 us,
-// a transport matrix (5,000 entries a row) 1,280 -> 146 us (1.6 TB/s of
-// matrix and vectors), 20k non-zeros 35 -> 34 us, which is launches and the
-// read of the error flag.
+// Bound by the gathers of x and by each tile's round trips.  Through the entry
+// point, against a thread adding each row from both factors in shared memory:
+// 20M non-zeros with power-law columns 358 -> 145 us, a transport matrix (rows
+// of 2,000 and 5,000) 1,280 -> 141 us (2.3 TB/s of matrix and vectors), 10M in
+// rows of 34 185 -> 94 us, of 65 184 -> 95 us; 20k non-zeros 35 -> 33 us, which
+// is launches and the read of the error flag.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include <stdio.h>
@@ -40,6 +42,8 @@
 namespace {
 
 constexpr int kTile = 2048;  // non-zeros per thread block
+constexpr int kRun = kTile / pdlp::kThreads;  // consecutive non-zeros of a thread
+static_assert(kRun == 8, "a thread's row marks are one 8-byte word");
 constexpr int kMaxTiles = PDLP_NOALLOC_MAX_TILES;
 
 // Scratch of every call: own[t] (partial of the row that starts in tile t and
@@ -54,10 +58,9 @@ struct Scratch {
 
 static __device__ __align__(256) Scratch g_scratch;
 
-// Products of a row that one thread adds.  A warp's sum costs 5 FP64 issue slots
-// (16 cycles each) for its tree besides its products, so a warp of threads is
-// the cheaper one while a tile has a warp's worth of rows; beyond, it is a
-// serial chain.  9.7M non-zeros in rows of about 34: 200 us with 32, 111 with 64.
+// Runs of a row that one thread adds (up to 512 products); beyond, its adds in
+// turn take longer than a warp's, whose tree of shuffles costs 5 FP64 issue slots
+// of 16 cycles.  10M non-zeros in rows of 65: 94 us with 64 or 16, 181 with 8.
 constexpr int kShort = 64;
 
 // First r in [0, rows) with ptr[r] >= key, else rows, by a warp: each step
@@ -79,37 +82,56 @@ __device__ __forceinline__ int lower_bound_rows(const int *ptr, int rows, int ke
   return lo;
 }
 
-// Sum of sp[lo, hi) by a warp, in a fixed order; every lane returns it.
-__device__ __forceinline__ double warp_products(const double *sp, int lo, int hi) {
-  double s0 = 0.0, s1 = 0.0;
-  int i = lo + (int)(threadIdx.x & 31);
-  for (; i + 32 < hi; i += 64) {
-    s0 += sp[i];
-    s1 += sp[i + 32];
-  }
-  if (i < hi) s0 += sp[i];
-  return pdlp::warp_sum(s0 + s1);
+// Sum of the runs of [lo, hi) by a warp, in a fixed order: sp[lo] and sp at the
+// multiples of kRun above it, below hi.  Every lane returns it.
+__device__ __forceinline__ double warp_runs(const double *sp, int lo, int hi) {
+  const int first = lo / kRun;  // run of lo
+  double s = 0.0;
+#pragma unroll 4
+  for (int g = first + (int)(threadIdx.x & 31); g * kRun < hi; g += 32)
+    s += sp[g == first ? lo : g * kRun];
+  return pdlp::warp_sum(s);
 }
 
-__global__ void __launch_bounds__(pdlp::kThreads)
+// 5 blocks per SM: 6 spill (powerlaw 155 us), 4 leave too few loads in flight
+// (156 us).  Row marks are bytes: as bits, set by atomics, rows of one entry took
+// 107 us instead of 94 (5M of them).
+__global__ void __launch_bounds__(pdlp::kThreads, 5)
     k_spmv_tiles(int rows, int cols, int nnz, int ntiles, const int *__restrict__ ptr,
                  const int *__restrict__ col, const double *__restrict__ val,
                  const double *__restrict__ x, double *__restrict__ y, Scratch *s, int slot) {
-  constexpr int kPer = kTile / pdlp::kThreads;
-  __shared__ double sp[kTile];
+  __shared__ double sp[kTile];  // sums of runs, each where its run starts
+  __shared__ __align__(8) unsigned char starts[kTile];  // 1: a row starts here
   __shared__ int s_rows[2];
   const int t = blockIdx.x, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int k0 = t * kTile;
   const int k1 = min(nnz, k0 + kTile);
   const int len = k1 > k0 ? k1 - k0 : 0;
-  int c[kPer];
-  double v[kPer];
+  const int mine = tid * kRun, n = min(kRun, len - mine);  // this thread's elements
+  int c[kRun];
+  double v[kRun];
+  const bool aligned =
+      ((reinterpret_cast<uintptr_t>(col) | reinterpret_cast<uintptr_t>(val)) & 15) == 0;
+  if (aligned && n == kRun) {
 #pragma unroll
-  for (int u = 0; u < kPer; ++u) {
-    const int i = tid + u * pdlp::kThreads;
-    if (i < len) {
-      c[u] = __ldcs(col + k0 + i);
-      v[u] = __ldcs(val + k0 + i);
+    for (int u = 0; u < kRun; u += 4) {
+      const int4 q = __ldcs(reinterpret_cast<const int4 *>(col + k0 + mine + u));
+      c[u] = q.x; c[u + 1] = q.y; c[u + 2] = q.z; c[u + 3] = q.w;
+    }
+#pragma unroll
+    for (int u = 0; u < kRun; u += 2) {
+      const double2 q = __ldcs(reinterpret_cast<const double2 *>(val + k0 + mine + u));
+      v[u] = q.x; v[u + 1] = q.y;
+    }
+  } else {
+#pragma unroll
+    for (int u = 0; u < kRun; ++u) {
+      c[u] = 0;
+      v[u] = 0.0;
+      if (u < n) {
+        c[u] = __ldcs(col + k0 + mine + u);
+        v[u] = __ldcs(val + k0 + mine + u);
+      }
     }
   }
   if (warp < 2) {
@@ -118,6 +140,7 @@ __global__ void __launch_bounds__(pdlp::kThreads)
     if (first ? t > 0 : t < ntiles - 1) r = lower_bound_rows(ptr, rows, first ? k0 : k1);
     if (lane == 0) s_rows[warp] = r;
   }
+  reinterpret_cast<unsigned long long *>(starts)[tid] = 0ull;
   if (tid == 0) {
     if (t == 0 && (ptr[0] != 0 || ptr[rows] != nnz)) atomicOr(&s->error[slot], 1);
     if (t == 0) s->error[slot ^ 1] = 0;
@@ -128,18 +151,41 @@ __global__ void __launch_bounds__(pdlp::kThreads)
   for (long r = (long)t * pdlp::kThreads + tid; r < rows; r += (long)ntiles * pdlp::kThreads)
     if (ptr[r] > ptr[r + 1]) atomicOr(&s->error[slot], 1);
   bool bad = false;
+  double g[kRun];
 #pragma unroll
-  for (int u = 0; u < kPer; ++u) {
-    const int i = tid + u * pdlp::kThreads;
-    if (i < len) {
-      const bool in = c[u] >= 0 && c[u] < cols;
-      bad |= !in;  // flagged, never dereferenced
-      sp[i] = v[u] * (in ? __ldg(x + c[u]) : 0.0);
-    }
+  for (int u = 0; u < kRun; ++u) {
+    const bool in = c[u] >= 0 && c[u] < cols;
+    if (u < n) bad |= !in;  // flagged, never dereferenced
+    g[u] = u < n && in ? __ldg(x + c[u]) : 0.0;
   }
   if (bad) atomicOr(&s->error[slot], 2);
   __syncthreads();
   const int rA = s_rows[0], rB = s_rows[1];
+#pragma unroll 1
+  for (int r = rA + tid; r < rB; r += pdlp::kThreads) {
+    const int a = ptr[r] - k0;
+    if (a >= 0 && a < len) starts[a] = 1;
+  }
+  __syncthreads();
+  {
+    // the runs among this thread's elements, each left where it starts; bit u of
+    // `here`: a row starts at element u (the lowest bits of the eight bytes)
+    const unsigned long long bytes = reinterpret_cast<const unsigned long long *>(starts)[tid];
+    const unsigned here = (unsigned)((bytes * 0x0102040810204080ull) >> 56);
+    double sum = 0.0;
+    int from = mine;
+#pragma unroll
+    for (int u = 0; u < kRun; ++u) {
+      if (u > 0 && ((here >> u) & 1u)) {
+        sp[from] = sum;
+        sum = 0.0;
+        from = mine + u;
+      }
+      if (u < n) sum = fma(v[u], g[u], sum);
+    }
+    sp[from] = sum;
+  }
+  __syncthreads();
   // rows starting in this tile; the one running past k1 leaves its partial
   for (int base = rA + 32 * warp; base < rB; base += pdlp::kThreads) {
     const int r = base + lane;
@@ -148,19 +194,22 @@ __global__ void __launch_bounds__(pdlp::kThreads)
     if (live) {
       a = ptr[r];
       e = ptr[r + 1];
-      live = a <= e && a >= 0 && e <= nnz;  // else flagged by the validation loop
+      live = a <= e && a >= k0 && e <= nnz;  // else flagged by the validation loop
     }
-    const int lo = max(a, k0) - k0, hi = min(e, k1) - k0;
+    const int lo = a - k0, hi = live ? min(e, k1) - k0 : lo;
     double sum = 0.0;
-    const bool wide = live && hi - lo > kShort;
-    if (live && !wide)
-      for (int i = lo; i < hi; ++i) sum += sp[i];
-    unsigned todo = __ballot_sync(0xffffffffu, wide);
+    const int runs = hi > lo ? (hi - 1) / kRun - lo / kRun + 1 : 0;
+    if (runs > 0 && runs <= kShort) {
+      sum = sp[lo];
+#pragma unroll 4
+      for (int q = (lo / kRun + 1) * kRun; q < hi; q += kRun) sum += sp[q];
+    }
+    unsigned todo = __ballot_sync(0xffffffffu, runs > kShort);
     while (todo) {
       const int src = __ffs(todo) - 1;
       todo &= todo - 1;
-      const double w = warp_products(sp, __shfl_sync(0xffffffffu, lo, src),
-                                     __shfl_sync(0xffffffffu, hi, src));
+      const double w = warp_runs(sp, __shfl_sync(0xffffffffu, lo, src),
+                                 __shfl_sync(0xffffffffu, hi, src));
       if (lane == src) sum = w;
     }
     if (live) {
@@ -175,7 +224,7 @@ __global__ void __launch_bounds__(pdlp::kThreads)
   // partial of the row (started in an earlier tile) that runs into this one
   if (warp == pdlp::kThreads / 32 - 1) {
     double in = 0.0;
-    if (t > 0 && rA > 0) in = warp_products(sp, 0, min(ptr[rA], k1) - k0);  // it ends where rA starts
+    if (t > 0 && rA > 0) in = warp_runs(sp, 0, min(ptr[rA], k1) - k0);  // it ends where rA starts
     if (lane == 0) s->in[t] = in;
   }
 }

@@ -3,28 +3,33 @@
 #include <stdio.h>
 #include <string.h>
 
+#include <memory>
 #include <string>
 #include <vector>
 
+#include "cupdlpx.h"
+#include "iter_kernels.cuh"
 #include "pdlp_gb300.h"
 #include "solver.cuh"
 
 namespace pdlp {
 
 // y[r] = sum_k a_rk x_k
-struct PlainEpi {
-  using val_t = double;
-  using acc_t = double;
+template <class T>
+struct RowSumEpi {
+  using val_t = T;
+  using acc_t = T;
   static constexpr int NF = 0;
   static constexpr unsigned MAXMASK = 0;
-  const double *x;
-  double *y;
+  const T *x;
+  T *y;
   __device__ bool init() { return true; }
   __device__ void prologue(double *) const {}
   __device__ void bind(const double *) {}
-  __device__ double gather(int j) const { return x[j]; }
-  __device__ void row(int r, double s, double *) const { y[r] = s; }
+  __device__ T gather(int j) const { return x[j]; }
+  __device__ void row(int r, T s, double *) const { y[r] = s; }
 };
+using PlainEpi = RowSumEpi<double>;
 
 }  // namespace pdlp
 
@@ -112,6 +117,59 @@ extern "C" int pdlp_gpu_spmv(int rows, int cols, const int *row_ptr, const int *
                              const double *vals, const double *x, double *y, int tile) {
   if (tile != 512 && tile != 2048) return -1;
   return pdlp_gpu_spmv_variant(rows, cols, row_ptr, col_ind, vals, x, y, tile, 0);
+}
+
+extern "C" int pdlp_gpu_products_fp32(const lp_problem_t *prob, int kernel, const float *x,
+                                      const float *y, float *ax, float *aty) {
+  using namespace pdlp;
+  if (!prob || !x || !y || !ax || !aty || kernel < -1 || kernel > 1) return -1;
+  const cudaStream_t st = cudaStreamPerThread;
+  try {
+    std::unique_ptr<DevProblem> P(upload_problem(prob, st, kernel));
+    pdhg_parameters_t p;
+    set_default_parameters(&p);
+    p.l_inf_ruiz_iterations = 0;  // the matrix as given
+    p.has_pock_chambolle_alpha = false;
+    p.bound_objective_rescaling = false;
+    Solve<float> s(p, st, *P, 0);
+    s.prepare();
+    const size_t vn = P->n, vm = P->m;
+    struct Mem {
+      float *p = nullptr;
+      cudaStream_t st;
+      ~Mem() { dev_free(p, st); }
+    } mem{(float *)dev_alloc((vn + vm) * 8 + 8, st), st};
+    auto order = [&](const int *perm, size_t count) {
+      std::vector<int> o(count);
+      for (size_t i = 0; i < count; ++i) o[i] = (int)i;
+      if (perm && count)
+        PDLP_CUDA(cudaMemcpyAsync(o.data(), perm, count * 4, cudaMemcpyDeviceToHost, st));
+      PDLP_CUDA(cudaStreamSynchronize(st));
+      return o;
+    };
+    const std::vector<int> om = order(P->perm_m, vm), on = order(P->perm_n, vn);
+    // out = M in, both in the caller's order
+    auto product = [&](const DevCsrT<float> &M, const float *in, const std::vector<int> &oin,
+                       float *out, const std::vector<int> &oout) {
+      std::vector<float> a(oin.size()), b(oout.size());
+      for (size_t i = 0; i < a.size(); ++i) a[i] = in[oin[i]];
+      float *da = mem.p, *db = mem.p + a.size();
+      if (!a.empty())
+        PDLP_CUDA(cudaMemcpyAsync(da, a.data(), a.size() * 4, cudaMemcpyHostToDevice, st));
+      launch_spmv(M, RowSumEpi<float>{da, db}, nullptr, nullptr, st);
+      if (!b.empty())
+        PDLP_CUDA(cudaMemcpyAsync(b.data(), db, b.size() * 4, cudaMemcpyDeviceToHost, st));
+      PDLP_CUDA(cudaStreamSynchronize(st));
+      for (size_t i = 0; i < b.size(); ++i) out[oout[i]] = b[i];
+    };
+    product(s.A(), x, on, ax, om);
+    product(s.AT(), y, om, aty, on);
+    return 0;
+  } catch (const std::exception &e) {
+    fprintf(stderr, "[cupdlpx-gb300] pdlp_gpu_products_fp32: %s\n", e.what());
+    cudaGetLastError();
+    return -2;
+  }
 }
 
 extern "C" int pdlp_host_transpose(int m, int n, const int *row_ptr, const int *col_ind,

@@ -415,9 +415,6 @@ __device__ __forceinline__ void set_steps(Ctl *c) {
 // on plain CSR the pipelined or the fused one when PDLP_STEP_KERNEL=pipe /
 // fused forces it.  Reduction partials are sized and folded with the counts
 // of the kernel in use.
-// 1: forced pipelined, 0: forced fused, -1: the strip kernel
-int kernel_override();
-
 template <class V>
 inline bool use_pipe(const DevCsrT<V> &M) {
   return M.pipe_on && M.pipe.ntile > 0;

@@ -208,6 +208,7 @@ cupdlpx_result_t *solve_refined(const DevProblem &P, const pdhg_parameters_t &pa
   Q.tile = P.tile;
   Q.A = P.A;
   Q.AT = P.AT;
+  Q.kernel = P.kernel;
   Q.strips = P.strips;
   Q.nsm = P.nsm;
   Q.perm_m = P.perm_m;
@@ -413,6 +414,7 @@ cupdlpx_result_t *solve_refined(const DevProblem &P, const pdhg_parameters_t &pa
     W.tile = P.tile;
     W.A = P.A;
     W.AT = P.AT;
+    W.kernel = P.kernel;
     W.strips = P.strips;
     W.nsm = P.nsm;
     W.perm_m = P.perm_m;

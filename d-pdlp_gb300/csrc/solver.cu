@@ -384,7 +384,7 @@ DevProblem::~DevProblem() {
   if (arena) dev_free(arena, owner);
 }
 
-DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st) {
+DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel) {
   const int n = prob->num_variables, m = prob->num_constraints;
   const int nnz = prob->constraint_matrix_num_nonzeros;
   // A malformed CSR must never reach the host transpose or a device gather.
@@ -434,7 +434,8 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st) {
     }
     for (int c = 0; c < n; ++c) tp[c + 1] += tp[c];
   }
-  const bool strips = kernel_override() < 0;  // else the forced kernel's CSR
+  const bool strips = kernel < 0;  // else that kernel's CSR
+  P->kernel = kernel;
   P->strips = strips;
   int dev = 0, nsm = kNumSms;
   PDLP_CUDA(cudaGetDevice(&dev));

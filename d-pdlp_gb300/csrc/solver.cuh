@@ -180,13 +180,20 @@ struct DevProblem {
   // (pdlp_device_problem_t) switches to the per-thread stream: its solves
   // return only after their work on the problem has finished.
   cudaStream_t owner = cudaStreamPerThread;
-  bool strips = false;  // strip format (else plain CSR)
+  // the kernel of its products: -1 strips, or on plain CSR 0 fused, 1 pipelined
+  int kernel = -1;
+  bool strips = true;  // strip format (kernel < 0)
   int nsm = kNumSms;  // SMs of the device it was uploaded to
   ~DevProblem();
 };
 
-// Validate, transpose (host), plan and upload.  Throws on a malformed CSR.
-DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st);
+// The kernel that PDLP_STEP_KERNEL forces (0 fused, 1 pipelined), else -1.
+int kernel_override();
+
+// Validate, transpose, plan and upload for the products' kernel (DevProblem::
+// kernel).  Throws on a malformed CSR.
+DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st,
+                           int kernel = kernel_override());
 
 // KKT measures of a point, in the reference's definitions.
 struct Kkt {
@@ -281,6 +288,7 @@ class Solve {
   int total_count() const;
   const Dev<T> &dev() const { return d_; }
   const DevCsrT<M> &A() const { return A_; }
+  const DevCsrT<M> &AT() const { return AT_; }
   const DevCsr &A64() const { return A64_; }
   // scaled FP64 vectors (valid after prepare)
   const double *c64() const { return c64_; }

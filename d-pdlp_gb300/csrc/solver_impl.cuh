@@ -685,7 +685,7 @@ void Solve<T, M>::alloc() {
   pw_.ctl = d.ctl;
   pw_.hflag = dflag;
   pw_.ew_grid = ew;
-  apply_kernels(kernel_override() == 1);
+  apply_kernels(P_.kernel == 1);
 }
 
 // The kernel of a CSR matrix's products (forced; the strip format has one) and

@@ -329,6 +329,39 @@ __device__ __forceinline__ int strip_row(const StripMat<M> &A, int s, bool &ends
   return row;
 }
 
+// Sums of the strip rows (FP32) that the fused kernel strides with several
+// lanes (see "FP32 sums"), by the whole warp, row by row: its lanes take those
+// lanes' parts of the row.  total: this lane's row's sum.  Such a row stands
+// beside long ones or alone at the end of that kernel's tile: 637 of the 2M
+// columns of the power-law LP, 513 of them with one entry (any order).
+template <bool STREAM, class Epi>
+__device__ __forceinline__ void strip_strided(const Epi &epi, const int *col, const float *val,
+                                              int n, int lg, bool mine, int how, float &total) {
+  const int lane = threadIdx.x & 31;
+  unsigned todo = __ballot_sync(0xffffffffu, mine && how >= kSumStrided);
+#pragma unroll 1
+  while (todo) {
+    const int src = __ffs(todo) - 1;
+    todo &= todo - 1;
+    const int lanes = 1 << (__shfl_sync(0xffffffffu, how, src) - kSumStrided);
+    double t = 0.0;
+#pragma unroll 1
+    for (int j = lane; j < lanes && j < n << lg; j += 32) {
+      float s = 0.f;
+#pragma unroll 1
+      for (int e = j; e < n << lg; e += lanes) {
+        // element e of the row whose first lane is src (col, val: lane 0's)
+        const int at = (e >> lg) * 32 + src + (e & ((1 << lg) - 1));
+        const int c = ld_matrix<STREAM>(col + at);
+        if (c >= 0) s = fmaf(ld_matrix<STREAM>(val + at), epi.gather(c), s);
+      }
+      t += (double)s;
+    }
+    t = warp_sum(t);
+    if (lane == src) total = (float)t;
+  }
+}
+
 // Strip s, by a warp; `head` as strip_head loaded it.
 template <bool STREAM, bool PAIR, class Epi, class M>
 __device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi, double *acc,
@@ -385,6 +418,8 @@ __device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi,
   M total = sum.total(n > 2);
   if constexpr (sizeof(M) == 8)
     for (int o = 1; o < (1 << lg); o <<= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+  if constexpr (sizeof(M) == 4 && !PAIR)
+    if (n > 1 || lg > 0) strip_strided<STREAM>(epi, col - lane, val - lane, n, lg, ends, how, total);
   if (ends) strip_epilogue(epi, row, total, pre, acc);
 }
 

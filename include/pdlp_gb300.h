@@ -310,6 +310,12 @@ int pdlp_host_transpose(int m, int n, const int *row_ptr, const int *col_ind,
                         const double *vals, int *t_row_ptr, int *t_col_ind,
                         double *t_vals);
 
+/* A x and A^T y as the FP32 rounds form them, on the matrix as given rounded to
+ * FP32, by the products' kernel: -1 the default one, 0 fused, 1 pipelined.
+ * Returns 0, -1 on bad arguments, -2 on a CUDA error. */
+int pdlp_gpu_products_fp32(const lp_problem_t *prob, int kernel, const float *x,
+                           const float *y, float *ax, float *aty);
+
 /* The device transpose of the upload path (the stable transpose above,
  * built on the GPU by a radix sort of the column indices), on host arrays
  * copied in and out.  Returns 0, -1 as pdlp_host_transpose, -2 on a CUDA

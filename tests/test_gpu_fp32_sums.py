@@ -1,0 +1,66 @@
+"""FP32 row sums of the default (strip) kernel against those of the fused one.
+
+Below 4,194,304 non-zeros the strip kernel adds a row's products in the fused
+kernel's order, whatever the row's place in that kernel's tiles: staged tiles
+(segments of 8), the register path (4), rows strided by 2 to 256 lanes and
+chunked ones.  Across lanes both add in FP64 and round once to FP32, so the
+results are the same bits."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+import cupdlpx as cp
+
+pytestmark = pytest.mark.gpu
+
+
+def products(lib, prob, kernel, x, y):
+    f = C.POINTER(C.c_float)
+    lib.pdlp_gpu_products_fp32.restype = C.c_int
+    lib.pdlp_gpu_products_fp32.argtypes = [C.POINTER(cp.LpProblem), C.c_int, f, f, f, f]
+    ax, aty = np.zeros(len(y), np.float32), np.zeros(len(x), np.float32)
+    assert lib.pdlp_gpu_products_fp32(prob.ptr, kernel, *(a.ctypes.data_as(f)
+                                                          for a in (x, y, ax, aty))) == 0
+    return ax, aty
+
+
+def matrix(lengths, n, seed):
+    """CSR of random columns; values that FP32 holds exactly."""
+    rng = np.random.default_rng(seed)
+    lengths = rng.permutation(np.asarray(lengths))
+    ptr = np.zeros(len(lengths) + 1, dtype=np.int32)
+    ptr[1:] = np.cumsum(lengths)
+    col = rng.integers(0, n, ptr[-1]).astype(np.int32)
+    val = rng.standard_normal(ptr[-1]).astype(np.float32)
+    x = rng.standard_normal(n).astype(np.float32)
+    y = rng.standard_normal(len(lengths)).astype(np.float32)
+    prob = cp.Problem.from_csr(ptr, col, val.astype(np.float64), n, c=np.zeros(n),
+                               lc=np.zeros(len(lengths)), uc=np.ones(len(lengths)),
+                               lv=np.zeros(n), uv=np.ones(n))
+    return prob, (ptr, col, val), x, y
+
+
+LENGTHS = {
+    # short rows between long ones: tiles whose rows are strided by several
+    # lanes, or that hold one short row
+    "short_between_long": ([3, 17, 64, 0, 2, 40] * 30 + [300, 450, 90, 65, 512] * 40, 900),
+    "short_alone": ([40, 500] * 60, 700),
+    "last_tile_one_row": ([16] * 32 + [7], 300),
+    "edges": ([63, 64, 65, 0, 1, 31, 32, 33] * 20 + [511, 512, 513, 1023, 1024, 1025, 5000], 6000),
+    "eight_lanes": ([9] * 3000, 5003),
+    "four_lanes": ([9] * 9000, 12000),
+    "one_lane": ([6] * 45001, 50021),
+    # 2M non-zeros or more: tiles of 1,024 and the register path
+    "register_path": ([21] * 100000, 300000),
+    "register_path_and_long": ([21] * 95000 + [3, 64, 900, 70] * 100, 300000),
+}
+
+
+@pytest.mark.parametrize("name", sorted(LENGTHS))
+def test_strip_sums_are_the_fused_kernels(lib, name):
+    lengths, n = LENGTHS[name]
+    prob, _, x, y = matrix(lengths, n, 29)
+    strip, fused = products(lib, prob, -1, x, y), products(lib, prob, 0, x, y)
+    assert np.array_equal(strip[0], fused[0])
+    assert np.array_equal(strip[1], fused[1])

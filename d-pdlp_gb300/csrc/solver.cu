@@ -454,9 +454,7 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel
     std::vector<unsigned char> sums;
     bool pairs = false;
     auto fp32_sums = [&] {
-      bool front = false;
-      for (int r = 0; r < rows && !front; ++r) front = ptr[r + 1] - ptr[r] > kStripRow;
-      pairs = nnz >= kTeamMaxNnz && !front;
+      pairs = strip_pairs(rows, ptr);
       if (pairs) strip_sums_pipe(rows, ptr, nv, sums);
       else strip_sums_fused(rows, ptr, P->tile, chunk, sums);
     };

@@ -33,9 +33,9 @@
 // FP32 sums.  An FP32 solve's path depends on the rounding of its sums (the
 // 20M-non-zero power-law LP takes 55,200 or 69,400 iterations to 1e-4 with two
 // orders of the same products), so FP32 matrices keep the order that the fused
-// kernel gives them, or the FP32 pairs of the pipelined one (kTeamMaxNnz
-// non-zeros or more, and no front: the rows that kernel is the faster one
-// for): a row's elements are folded in segments that end at
+// kernel gives them, or the FP32 pairs of the pipelined one (strip_pairs below:
+// by the lengths of all rows, so that one long row changes nothing for the
+// others): a row's elements are folded in segments that end at
 // fixed distances from the start of the row's tile of that kernel's plan, and
 // the segments are added in order.  StripHost::sums holds, per row, the
 // segment length and the row's phase in it, or the number of lanes that the
@@ -125,6 +125,28 @@ inline void strip_sums_fused(int rows, const int *ptr, int tile, int chunk,
       for (int r = b.x; r < b.y; ++r) sums[r] = (unsigned char)(kSumStrided + g);
     }
   }
+}
+
+// Whether an FP32 matrix is summed in pairs: one of kPairsMinNnz non-zeros or
+// more, unless more than a twentieth of them lie in rows that the pipelined
+// kernel takes at a loss -- alone in a tile they do not fill (more than
+// kPipeMedRows, up to kPipeFill entries) or in chunks.  Those two kernels' times
+// draw the line; above it a matrix keeps the pairs it has had there, below it
+// the fused kernel's sums.  Pipelined over fused, FP32 dual step: random rows of
+// 10 to 100 0.71-0.95, of 120 (a quarter of the non-zeros in rows above 128)
+// 1.9-2.0, of 160 1.8; uniform rows of 130 2.0, 300 1.06, 350 0.86, 500 0.88,
+// 800 0.65, 2,000 0.92, 2,100 2.0, 5,000 1.6; columns of power-law LPs 1.6-2.2.
+constexpr long kPairsMinNnz = 1L << 22;
+constexpr int kPipeFill = 340;
+inline bool strip_pairs(int rows, const int *ptr) {
+  const long nnz = rows > 0 ? ptr[rows] : 0;
+  if (nnz < kPairsMinNnz) return false;
+  long loss = 0;
+  for (int r = 0; r < rows; ++r) {
+    const int len = ptr[r + 1] - ptr[r];
+    if ((len > kPipeMedRows && len <= kPipeFill) || len > kPipeTile) loss += len;
+  }
+  return 20 * loss <= nnz;
 }
 
 // ... or of the pipelined kernel (nv row vectors staged; its one-row tiles are

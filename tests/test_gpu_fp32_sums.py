@@ -4,7 +4,10 @@ Below 4,194,304 non-zeros the strip kernel adds a row's products in the fused
 kernel's order, whatever the row's place in that kernel's tiles: staged tiles
 (segments of 8), the register path (4), rows strided by 2 to 256 lanes and
 chunked ones.  Across lanes both add in FP64 and round once to FP32, so the
-results are the same bits."""
+results are the same bits.
+
+From there on matrices are summed in FP32 pairs (rounded to FP32 once),
+but for those with many rows that the pipelined kernel takes at a loss."""
 import ctypes as C
 
 import numpy as np
@@ -64,3 +67,31 @@ def test_strip_sums_are_the_fused_kernels(lib, name):
     strip, fused = products(lib, prob, -1, x, y), products(lib, prob, 0, x, y)
     assert np.array_equal(strip[0], fused[0])
     assert np.array_equal(strip[1], fused[1])
+
+
+PAIRS = {
+    # one row of 65 entries or more leaves the other rows' sums as they are
+    "one_long_row": ([21] * 200000 + [70, 300], 400000),
+    "front_of_100": ([100] * 43000, 400000),
+    "rows_of_500": ([500] * 8500, 400000),
+}
+
+
+@pytest.mark.parametrize("name", sorted(PAIRS))
+def test_large_matrices_are_summed_in_pairs(lib, name):
+    lengths, n = PAIRS[name]
+    prob, (ptr, col, val), x, y = matrix(lengths, n, 31)
+    assert ptr[-1] >= 1 << 22
+    ax, aty = products(lib, prob, -1, x, y)
+    row = np.repeat(np.arange(len(lengths)), np.diff(ptr))
+    for got, to, of, vec in ((ax, row, col, x), (aty, col, row, y)):
+        term = val.astype(np.float64) * vec[of]
+        exact, size = np.zeros(len(got)), np.zeros(len(got))
+        np.add.at(exact, to, term)
+        np.add.at(size, to, np.abs(term))
+        count = np.bincount(to, minlength=len(got))
+        # one rounding to FP32 of the pair; its low part is at most k u size after
+        # k products (u = 2^-24) and each of up to four additions to it rounds by
+        # u of that
+        bar = 2.0 ** -24 * np.abs(exact) + 2.0 * count * (count + 1) * 2.0 ** -48 * size
+        assert np.all(np.abs(got - exact) <= bar * (1 + 1e-6))

@@ -483,6 +483,32 @@ __device__ __forceinline__ double strip_warp_sum(const StripMat<M> &A, const Epi
   }
 }
 
+// s plus the products of elements k, k + step, ... below e, in order.  Four
+// elements' loads at a time: one by one each gather waits for its own column.
+template <bool STREAM, class Epi>
+__device__ __forceinline__ float strip_chain(const StripMat<float> &A, const Epi &epi, int k,
+                                             int e, int step, float s) {
+  constexpr int U = 4;
+#pragma unroll 1
+  for (; k < e; k += U * step) {
+    int c[U];
+    float v[U], x[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k + u * step < e) {
+        c[u] = ld_matrix<STREAM>(A.col + k + u * step);
+        v[u] = ld_matrix<STREAM>(A.val + k + u * step);
+      }
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k + u * step < e) x[u] = epi.gather(c[u]);
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (k + u * step < e) s = fmaf(v[u], x[u], s);
+  }
+  return s;
+}
+
 // Sum of the whole front row [a, e) as `how` says (FP32, see above).
 template <bool STREAM, class Epi>
 __device__ __forceinline__ float strip_row_sum(const StripMat<float> &A, const Epi &epi, int a,
@@ -491,12 +517,8 @@ __device__ __forceinline__ float strip_row_sum(const StripMat<float> &A, const E
   if (how >= kSumStrided) {
     const int lanes = 1 << (how - kSumStrided);
     double t = 0.0;
-    for (int j = lane; j < lanes; j += 32) {
-      float s = 0.f;
-      for (int k = a + j; k < e; k += lanes)
-        s = fmaf(ld_matrix<STREAM>(A.val + k), epi.gather(ld_matrix<STREAM>(A.col + k)), s);
-      t += (double)s;
-    }
+    for (int j = lane; j < lanes; j += 32)
+      t += (double)strip_chain<STREAM>(A, epi, a + j, e, lanes, 0.f);
     return (float)warp_sum(t);
   }
   // segments: a lane each, added in order
@@ -505,9 +527,7 @@ __device__ __forceinline__ float strip_row_sum(const StripMat<float> &A, const E
   float all = -0.f;
   for (int j = 0; j < count; j += 32) {
     const int k0 = max(a, a - phase + (j + lane) * len), k1 = min(e, a - phase + (j + lane + 1) * len);
-    float s = 0.f;
-    for (int k = k0; k < k1; ++k)
-      s = fmaf(ld_matrix<STREAM>(A.val + k), epi.gather(ld_matrix<STREAM>(A.col + k)), s);
+    const float s = strip_chain<STREAM>(A, epi, k0, k1, 1, 0.f);
     const int n = min(32, count - j);
     for (int g = 0; g < n; ++g) all += __shfl_sync(0xffffffffu, s, g);
   }
@@ -589,12 +609,13 @@ __device__ __forceinline__ void strip_block_partials(const double (&acc)[NA], do
 // Bound by FP64 issue (16 cycles per warp instruction and SM) and by the
 // gathers' L2 requests.  20M non-zeros, ms per launch, before (the faster of
 // the CSR kernels) and now: power-law dual step 0.121 -> 0.083 (FP32 0.101 ->
-// 0.053), primal step 0.152 -> 0.146 (FP32 0.103 -> 0.141: the segments of its
+// 0.053), primal step 0.152 -> 0.146 (FP32 0.103 -> 0.132: the segments of its
 // sums); transport evaluation over A^T 0.375 -> 0.305, primal step, whose rows
-// have two entries, 0.185 -> 0.203.  5 blocks per SM: 6 spill more, 4 (no
-// spills) take the transport primal step to 0.258.
+// have two entries, 0.185 -> 0.203.  5 blocks per SM: 6 spill more (FP32 primal
+// step 0.139; FP32 pairs, which need fewer registers, run at 6), 4 (no spills)
+// take the transport primal step to 0.258.
 template <class Epi, bool STREAM, bool PAIR>
-__global__ void __launch_bounds__(kThreads, sizeof(typename Epi::val_t) == 8 ? 5 : 6)
+__global__ void __launch_bounds__(kThreads, sizeof(typename Epi::val_t) == 8 || !PAIR ? 5 : 6)
     spmv_strip(const __grid_constant__ StripMat<typename Epi::val_t> A,
                double *__restrict__ part, double *__restrict__ lpart, Epi epi) {
   using M = typename Epi::val_t;

@@ -617,7 +617,6 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel
     p.store = h.store;
     const long warps = (long)p.nitem + p.nstrip, per = kThreads / 32;
     p.grid = (int)((warps + per - 1) / per);
-    p.unit_parts = nnz < kTeamMaxNnz;
     p.pairs = h.pairs;
     up(M.ptr, h.fptr);
     up(p.off, h.off);
@@ -629,6 +628,8 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel
   if (strips) {
     strip(P->A, m, n, shA, P->perm_m);
     strip(P->AT, n, m, shT, P->perm_n);
+    P->A.strip.unit_parts = P->AT.strip.unit_parts =
+        team_ctas(nnz, P->A.strip, P->AT.strip, nsm) > 0;
   } else {
     mat(P->A, m, n, blkA, lrA, pblkA, plrA);
     mat(P->AT, n, m, blkT, lrT, pblkT, plrT);

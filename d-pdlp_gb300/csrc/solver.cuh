@@ -121,9 +121,6 @@ struct PowDev {
   double sv_tol;
 };
 
-// LPs below this many non-zeros run their loop and power method as a resident
-// team (team.cuh).
-constexpr long kTeamMaxNnz = 1L << 22;
 constexpr int kMiscPart = 4096;
 constexpr int kHalpernTable = 1 << 16;
 

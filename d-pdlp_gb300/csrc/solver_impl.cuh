@@ -537,8 +537,7 @@ void Solve<T, M>::alloc() {
   const int n = P_.n, m = P_.m;
   const int ew = grid_for((long)n + m, 4);
   const size_t vn = n, vm = m;
-  if (P_.strips && P_.nnz > 0 && P_.nnz < kTeamMaxNnz)
-    team_ = team_ctas(P_.A.strip, P_.AT.strip, P_.nsm);
+  if (P_.strips) team_ = team_ctas(P_.nnz, P_.A.strip, P_.AT.strip, P_.nsm);
   // reduction partials of an SpMV site: one per CTA of the pipelined kernel
   // (or per block of the fused kernel) plus one per long row
   const size_t nbA = spmv_partials_max(P_.A), nbT = spmv_partials_max(P_.AT);

@@ -59,8 +59,8 @@ struct StripPlan {
   int nfront = 0;              // rows longer than kStripRow (they come first)
   int nitem = 0, nlong = 0, nstrip = 0;
   int lg = 0;                  // a strip's rows have 1 << lg lanes each
-  // reduction partials: one per item and strip (in that order), whatever warp
-  // took it, or, for matrices too large for a team, one per block
+  // reduction partials: one per strip, whatever warp took it, for LPs that a
+  // team may run (team.cuh); else one per block
   int unit_parts = 0;
   int pairs = 0;               // FP32 sums in pairs (see above)
   int grid = 0;                // blocks of the product kernel (8 items or strips each)

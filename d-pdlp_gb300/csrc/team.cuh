@@ -27,6 +27,9 @@
 
 namespace pdlp {
 
+// LPs below this many non-zeros run their loop and power method as a resident
+// team, where team_ctas finds one.
+constexpr long kTeamMaxNnz = 1L << 22;
 constexpr int kTeamThreads = kThreads;
 constexpr int kTeamWarps = kTeamThreads / 32;
 constexpr int kTeamCtasPerSm = 2;
@@ -151,13 +154,20 @@ class TeamTurn {
   bool held_ = false;
 };
 
-// CTAs of the team for two matrices; 0: no team.  A matrix with a front (rows
+// CTAs of the team for an LP's matrices; 0: no team.  A matrix with a front (rows
 // of more than 64 entries) has none: its items and their sums need a barrier
 // more per product and leave most warps of a team idle (an LP with such rows:
-// 25 ms against 17 ms with a kernel per product).
-inline int team_ctas(const StripPlan &A, const StripPlan &AT, int nsm) {
-  if (A.nitem > 0 || AT.nitem > 0) return 0;
+// 25 ms against 17 ms with a kernel per product).  Nor has one with more than
+// two strips for a warp: the barriers no longer show beside the strips, but every
+// CTA folds every strip's partial sums itself.  FP64, 600 iterations with set-up,
+// team and single launches: 65k x 22k with 2 entries a row 15.1 and 17.2 ms, 131k
+// x 44k 25.9 and 27.2, 262k x 87k 40.3 and 38.2, 524k x 175k 64 and 54, 4M x 1.3M
+// 402 and 268; with 4M non-zeros throughout, 66k 75.4 and 73.8, 131k 134 and 131,
+// 262k 150 and 138.
+inline int team_ctas(long nnz, const StripPlan &A, const StripPlan &AT, int nsm) {
+  if (nnz <= 0 || nnz >= kTeamMaxNnz || A.nitem > 0 || AT.nitem > 0) return 0;
   const int work = std::max(A.nstrip, AT.nstrip);
+  if (work > 2 * nsm * kTeamCtasPerSm * kTeamWarps) return 0;
   // one CTA per SM until its warps have a strip each, then two
   return work <= nsm * kTeamWarps ? std::max(1, std::min(work, nsm)) : nsm * kTeamCtasPerSm;
 }

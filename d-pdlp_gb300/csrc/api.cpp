@@ -418,8 +418,9 @@ cupdlpx_result_t *solve_impl(const lp_problem_t *prob, const pdhg_parameters_t *
   try {
     print_initial_info(&p, prob);
     StreamGuard sg;
-    std::unique_ptr<pdlp::DevProblem> P(pdlp::upload_problem(prob, sg.s));
-    pdlp_options_t o = opts ? *opts : env_options();
+    const pdlp_options_t o = opts ? *opts : env_options();
+    std::unique_ptr<pdlp::DevProblem> P(pdlp::upload_problem(
+        prob, sg.s, pdlp::kernel_override(), o.precision != PDLP_PRECISION_FP64));
     cupdlpx_result_t *r =
         o.precision != PDLP_PRECISION_FP64
             ? run_refined(*P, p, o, sg.s, info, t0)

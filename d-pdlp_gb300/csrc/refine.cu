@@ -209,6 +209,7 @@ cupdlpx_result_t *solve_refined(const DevProblem &P, const pdhg_parameters_t &pa
   Q.A = P.A;
   Q.AT = P.AT;
   Q.kernel = P.kernel;
+  Q.fp32 = P.fp32;
   Q.strips = P.strips;
   Q.nsm = P.nsm;
   Q.perm_m = P.perm_m;
@@ -415,6 +416,7 @@ cupdlpx_result_t *solve_refined(const DevProblem &P, const pdhg_parameters_t &pa
     W.A = P.A;
     W.AT = P.AT;
     W.kernel = P.kernel;
+    W.fp32 = P.fp32;
     W.strips = P.strips;
     W.nsm = P.nsm;
     W.perm_m = P.perm_m;

@@ -131,7 +131,9 @@ struct pdlp_server {
       } else {
         try {
           const auto tu = Clock::now();
-          std::unique_ptr<pdlp::DevProblem> P(pdlp::upload_problem(r->prob, st));
+          std::unique_ptr<pdlp::DevProblem> P(
+              pdlp::upload_problem(r->prob, st, pdlp::kernel_override(),
+                                   opts.precision != PDLP_PRECISION_FP64));
           r->upload_s = since(tu, Clock::now());
           pdlp_solve_info_t si;
           memset(&si, 0, sizeof(si));

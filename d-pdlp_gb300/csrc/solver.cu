@@ -7,6 +7,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <array>
 #include <atomic>
 #include <exception>
 #include <mutex>
@@ -101,8 +102,23 @@ __global__ void k_invert(int n, const int *__restrict__ perm, int *__restrict__ 
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
     inv[perm[i]] = (int)i;
 }
-__global__ void k_gather(int n, const double *__restrict__ src, const int *__restrict__ perm,
-                         double *__restrict__ dst) {
+// dst[i] = src[perm[i]] (null perm: src[i]) for several vectors, one to a grid row
+struct GatherList {
+  const double *src[7];
+  double *dst[7];
+  const int *perm[7];
+  int count[7];
+};
+__global__ void k_gather(const __grid_constant__ GatherList g) {
+  const int v = blockIdx.y;
+  const double *src = g.src[v];
+  const int *perm = g.perm[v];
+  for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < g.count[v];
+       i += (long)gridDim.x * blockDim.x)
+    g.dst[v][i] = src[perm ? perm[i] : i];
+}
+__global__ void k_gather_bytes(int n, const unsigned char *__restrict__ src,
+                               const int *__restrict__ perm, unsigned char *__restrict__ dst) {
   for (long i = blockIdx.x * (long)blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x)
     dst[i] = src[perm[i]];
 }
@@ -113,7 +129,7 @@ __global__ void k_scatter_back(int n, const double *__restrict__ src, const int 
 }
 void launch_gather(int n, const double *src, const int *perm, double *dst, cudaStream_t st) {
   if (n <= 0) return;
-  k_gather<<<grid_for(n), kThreads, 0, st>>>(n, src, perm, dst);
+  k_gather<<<grid_for(n), kThreads, 0, st>>>(GatherList{{src}, {dst}, {perm}, {n}});
   PDLP_LAUNCH_CHECK();
 }
 void launch_scatter(int n, const double *src, const int *perm, double *dst, cudaStream_t st) {
@@ -122,27 +138,35 @@ void launch_scatter(int n, const double *src, const int *perm, double *dst, cuda
   PDLP_LAUNCH_CHECK();
 }
 
-// The stored elements of a strip-format matrix from CSR rows sptr / scol /
-// sval: row i is the source's row perm[i] with its entries in their order,
-// column j becomes icol[j] (null permutations: the identity).  A warp per
-// front row, then a warp per strip.
+// The stored elements of a strip-format matrix from entries scol / sval in rows
+// sptr: row i is the source's row perm[i] with its entries in their order, whose
+// k-th is entry k or pos[k]; column j becomes icol[j] (null perm, pos, icol: the
+// identity).  A warp per front item, then a warp per strip.
 __global__ void __launch_bounds__(kThreads)
     k_strip_fill(StripMat<double> A, const int *__restrict__ sptr, const int *__restrict__ scol,
-                 const double *__restrict__ sval, const int *__restrict__ perm,
-                 const int *__restrict__ icol, int *__restrict__ col, double *__restrict__ val) {
+                 const double *__restrict__ sval, const int *__restrict__ pos,
+                 const int *__restrict__ perm, const int *__restrict__ icol,
+                 int *__restrict__ col, double *__restrict__ val) {
   const int lane = threadIdx.x & 31;
   const int W = gridDim.x * (kThreads / 32);
-  for (int w = (blockIdx.x * kThreads + threadIdx.x) >> 5; w < A.p.nfront + A.p.nstrip; w += W) {
-    if (w < A.p.nfront) {
-      const int a = sptr[perm ? perm[w] : w], to = A.ptr[w], len = A.ptr[w + 1] - to;
-      for (int k = lane; k < len; k += 32) {
-        const int c = scol[a + k];
-        col[to + k] = icol ? icol[c] : c;
-        val[to + k] = sval[a + k];
+  auto take = [&](int k, int &c, double &v) {
+    const int q = pos ? pos[k] : k;
+    c = scol[q];
+    if (icol) c = icol[c];
+    v = sval[q];
+  };
+  for (int w = (blockIdx.x * kThreads + threadIdx.x) >> 5; w < A.p.nitem + A.p.nstrip; w += W) {
+    if (w < A.p.nitem) {
+      const int4 b = A.p.item[w];
+      const int rows = b.y < 0 ? 1 : b.y, step = b.y < 0 ? 256 : 32;
+      for (int i = b.x; i < b.x + rows; ++i) {
+        const int from = sptr[perm ? perm[i] : i] - A.ptr[i];  // source less place
+        const int first = b.y < 0 ? b.z : A.ptr[i], end = b.y < 0 ? b.w : A.ptr[i + 1];
+        for (int k = first + lane; k < end; k += step) take(from + k, col[k], val[k]);
       }
       continue;
     }
-    const int s = w - A.p.nfront, lg = A.p.lg;
+    const int s = w - A.p.nitem, lg = A.p.lg;
     const int row = A.p.nfront + s * (32 >> lg) + (lane >> lg), sub = lane & ((1 << lg) - 1);
     int a = 0, len = 0;
     if (row < A.rows) {
@@ -156,11 +180,7 @@ __global__ void __launch_bounds__(kThreads)
       int c = -1;
       double v = 0.0;
       const int e = (k << lg) + sub;
-      if (e < len) {
-        c = scol[a + e];
-        if (icol) c = icol[c];
-        v = sval[a + e];
-      }
+      if (e < len) take(a + e, c, v);
       col[o0 + (size_t)k * 32] = c;
       val[o0 + (size_t)k * 32] = v;
     }
@@ -381,10 +401,80 @@ void parallel_slices(int T, long count, F &&f) {
 }  // namespace
 
 DevProblem::~DevProblem() {
-  if (arena) dev_free(arena, owner);
+  if (!arena) return;  // a view of another problem
+  if (fp32 && fp32->mem) dev_free(fp32->mem, owner);
+  dev_free(arena, owner);
 }
 
-DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel) {
+namespace {
+// The rows' FP32 sums of A and A^T (strip.cuh) in their original order.
+struct Fp32Host {
+  std::vector<unsigned char> A, AT;
+  bool pairs_A = false, pairs_AT = false;
+};
+Fp32Host fp32_order_host(int m, int n, const int *ptr, const int *tptr, int tile, int threads) {
+  Fp32Host h;
+  auto one = [&](int rows, const int *p, int nv, std::vector<unsigned char> &sums, bool &pairs) {
+    pairs = strip_pairs(rows, p);
+    if (pairs) strip_sums_pipe(rows, p, nv, sums);
+    else strip_sums_fused(rows, p, tile, pick_chunk(tile), sums);
+  };
+  auto of_A = [&] { one(m, ptr, 4, h.A, h.pairs_A); };
+  std::future<void> other;
+  if (threads > 1) other = std::async(std::launch::async, of_A);
+  else of_A();
+  one(n, tptr, 5, h.AT, h.pairs_AT);
+  if (other.valid()) other.get();
+  return h;
+}
+// ... and on the device in the format's order.
+void fp32_order_upload(const DevProblem &P, const Fp32Host &h, Fp32Order &o, cudaStream_t st) {
+  const size_t vm = P.m, vn = P.n;
+  Sizer z;
+  z.add<unsigned char>(vm);
+  z.add<unsigned char>(vn);
+  o.mem = dev_alloc(z.bytes, st);
+  struct Scratch {
+    void *p;
+    cudaStream_t st;
+    ~Scratch() { dev_free(p, st); }
+  } raw{dev_alloc(std::max(vm, vn), st), st};
+  Arena ar{(char *)o.mem, 0};
+  auto put = [&](const std::vector<unsigned char> &v, const int *perm, const unsigned char *&out) {
+    unsigned char *dst = ar.take<unsigned char>(v.size());
+    out = dst;
+    if (v.empty()) return;
+    PDLP_CUDA(cudaMemcpyAsync(perm ? raw.p : dst, v.data(), v.size(), cudaMemcpyHostToDevice, st));
+    if (!perm) return;
+    k_gather_bytes<<<grid_for((long)v.size()), kThreads, 0, st>>>(
+        (int)v.size(), (const unsigned char *)raw.p, perm, dst);
+    PDLP_LAUNCH_CHECK();
+  };
+  put(h.A, P.perm_m, o.A);
+  put(h.AT, P.perm_n, o.AT);
+  o.pairs_A = h.pairs_A;
+  o.pairs_AT = h.pairs_AT;
+  PDLP_CUDA(cudaStreamSynchronize(st));  // also for solves on other streams
+  o.made = true;
+}
+}  // namespace
+
+const Fp32Order &DevProblem::fp32_order(cudaStream_t st) const {
+  Fp32Order &o = *fp32;
+  std::lock_guard<std::mutex> lk(o.mu);
+  if (!o.made) {
+    if (o.mem) dev_free(o.mem, st);  // of an attempt that failed
+    o.mem = nullptr;
+    fp32_order_upload(*this, fp32_order_host(m, n, o.ptr.data(), o.tptr.data(), tile,
+                                             upload_threads(nnz)), o, st);
+    o.ptr = {};
+    o.tptr = {};
+  }
+  return o;
+}
+
+DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel,
+                           bool for_fp32) {
   const int n = prob->num_variables, m = prob->num_constraints;
   const int nnz = prob->constraint_matrix_num_nonzeros;
   // A malformed CSR must never reach the host transpose or a device gather.
@@ -450,36 +540,16 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel
   std::vector<int4> pblkA, pblkT;
   std::vector<int2> plrA, plrT;
   StripHost shA, shT;
-  auto strips_of = [&](int rows, const int *ptr, int nv, StripHost &h) {
-    std::vector<unsigned char> sums;
-    bool pairs = false;
-    auto fp32_sums = [&] {
-      pairs = strip_pairs(rows, ptr);
-      if (pairs) strip_sums_pipe(rows, ptr, nv, sums);
-      else strip_sums_fused(rows, ptr, P->tile, chunk, sums);
-    };
-    const int T = upload_threads(nnz);
-    if (T > 1) {
-      auto other = std::async(std::launch::async, fp32_sums);
-      build_strip_host(rows, ptr, nsm, chunk, h);
-      other.get();
-    } else {
-      build_strip_host(rows, ptr, nsm, chunk, h);
-      fp32_sums();
-    }
-    h.pairs = pairs;
-    if (h.identity) {
-      h.sums = std::move(sums);
-    } else {
-      h.sums.resize(rows);
-      parallel_slices(T, rows, [&](long a, long b) {
-        for (long i = a; i < b; ++i) h.sums[i] = sums[h.perm[i]];
-      });
-    }
-  };
+  std::future<Fp32Host> fp32_host;
+  if (strips && for_fp32)
+    fp32_host = std::async(upload_threads(nnz) > 1 ? std::launch::async : std::launch::deferred,
+                           [&] {
+                             return fp32_order_host(m, n, prob->constraint_matrix_row_pointers,
+                                                    tp.data(), P->tile, upload_threads(nnz));
+                           });
   auto plans_A = [&] {
     if (strips) {
-      strips_of(m, prob->constraint_matrix_row_pointers, 4, shA);
+      build_strip_host(m, prob->constraint_matrix_row_pointers, nsm, chunk, shA);
       return;
     }
     build_plan_host(m, prob->constraint_matrix_row_pointers, P->tile, blkA, lrA, chunk);
@@ -499,7 +569,7 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel
     plans_A();
   try {
     if (strips) {
-      strips_of(n, tp.data(), 5, shT);
+      build_strip_host(n, tp.data(), nsm, chunk, shT);
     } else {
       build_plan_host(n, tp.data(), P->tile, blkT, lrT, chunk);
       build_pipe_plan_host(n, tp.data(), 5, pblkT, plrT);
@@ -540,11 +610,10 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel
   Sizer z;
   if (strips) {
     for (const StripHost *h : {&shA, &shT}) {
-      z.add<int>(h->store); z.add<double>(h->store);
       z.add<int>(h->fptr.size()); z.add<int>(h->off.size());
       z.add<int4>(h->item.size()); z.add<int2>(h->lrow.size());
-      z.add<unsigned char>(h->sums.size());
-      if (!h->identity) z.add<int>(h->perm.size());
+      z.add<int>(h->perm.size());
+      z.add<int>(h->store); z.add<double>(h->store);
     }
   } else {
     z.add<int>(vm + 1); z.add<int>(nnz); z.add<double>(nnz);
@@ -594,19 +663,46 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel
     if (!plr.empty())
       PDLP_CUDA(cudaMemcpyAsync(M.pipe.lrow, plr.data(), plr.size() * 8, cudaMemcpyHostToDevice, st));
   };
+  // Host arrays on their way to consecutive places on the device.  Up to
+  // kPackBytes they go in one copy from one buffer: a small LP's upload is the
+  // number of its copies (20,000 non-zeros: 0.32 ms with 19 of them, 0.23 before
+  // there were strips).
+  constexpr size_t kPackBytes = 1 << 20;
+  struct Sending {
+    std::vector<std::array<const void *, 2>> at;  // source, place
+    std::vector<size_t> bytes;
+    std::vector<char> packed;
+    void add(void *dst, const void *src, size_t b) {
+      if (b == 0) return;
+      at.push_back({src, dst});
+      bytes.push_back(b);
+    }
+    void go(cudaStream_t st) {
+      if (at.empty()) return;
+      char *const base = (char *)at[0][1];
+      const size_t all = (const char *)at.back()[1] + bytes.back() - base;
+      if (all <= kPackBytes) {
+        packed.resize(all);
+        for (size_t i = 0; i < at.size(); ++i)
+          memcpy(packed.data() + ((const char *)at[i][1] - base), at[i][0], bytes[i]);
+        PDLP_CUDA(cudaMemcpyAsync(base, packed.data(), all, cudaMemcpyHostToDevice, st));
+        return;
+      }
+      for (size_t i = 0; i < at.size(); ++i)
+        PDLP_CUDA(cudaMemcpyAsync((void *)at[i][1], at[i][0], bytes[i], cudaMemcpyHostToDevice, st));
+    }
+  };
+  Sending index, input;
   auto up = [&](auto *&dst, const auto &src) {
     using E = typename std::remove_reference_t<decltype(src)>::value_type;
     E *p = ar.take<E>(src.size());
     dst = p;
-    if (!src.empty())
-      PDLP_CUDA(cudaMemcpyAsync(p, src.data(), src.size() * sizeof(E), cudaMemcpyHostToDevice, st));
+    index.add(p, src.data(), src.size() * sizeof(E));
   };
   auto strip = [&](DevCsr &M, int rows, int cols, const StripHost &h, const int *&perm) {
     M.rows = rows;
     M.cols = cols;
     M.nnz = nnz;
-    M.col = ar.take<int>(h.store);
-    M.val = ar.take<double>(h.store);
     StripPlan &p = M.strip;
     p.on = 1;
     p.nfront = (int)h.fptr.size() - 1;
@@ -617,19 +713,22 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel
     p.store = h.store;
     const long warps = (long)p.nitem + p.nstrip, per = kThreads / 32;
     p.grid = (int)((warps + per - 1) / per);
-    p.pairs = h.pairs;
     up(M.ptr, h.fptr);
     up(p.off, h.off);
     up(p.item, h.item);
     up(p.lrow, h.lrow);
-    up(p.sums, h.sums);
-    if (!h.identity) up(perm, h.perm);
+    if (!h.perm.empty()) up(perm, h.perm);
   };
   if (strips) {
     strip(P->A, m, n, shA, P->perm_m);
     strip(P->AT, n, m, shT, P->perm_n);
+    for (DevCsr *M : {&P->A, &P->AT}) {
+      M->col = ar.take<int>(M->strip.store);
+      M->val = ar.take<double>(M->strip.store);
+    }
     P->A.strip.unit_parts = P->AT.strip.unit_parts =
         team_ctas(nnz, P->A.strip, P->AT.strip, nsm) > 0;
+    index.go(st);
   } else {
     mat(P->A, m, n, blkA, lrA, pblkA, plrA);
     mat(P->AT, n, m, blkT, lrT, pblkT, plrT);
@@ -639,78 +738,108 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel
   P->uv = ar.take<double>(vn);
   P->lc = ar.take<double>(vm);
   P->uc = ar.take<double>(vm);
-  auto h2d = [&](void *dst, const void *src, size_t b) {
-    if (b) PDLP_CUDA(cudaMemcpyAsync(dst, src, b, cudaMemcpyHostToDevice, st));
+  if (prob->primal_start) P->xs = ar.take<double>(vn);
+  if (prob->dual_start) P->ys = ar.take<double>(vm);
+  struct Vec {
+    double *dst;
+    const double *src;
+    size_t count;
+    const int *perm;
   };
-  // device scratch of the upload, released on its stream
+  std::vector<Vec> vecs = {{P->c, prob->objective_vector, vn, P->perm_n},
+                           {P->lv, prob->variable_lower_bound, vn, P->perm_n},
+                           {P->uv, prob->variable_upper_bound, vn, P->perm_n},
+                           {P->lc, prob->constraint_lower_bound, vm, P->perm_m},
+                           {P->uc, prob->constraint_upper_bound, vm, P->perm_m}};
+  if (P->xs) vecs.push_back({P->xs, prob->primal_start, vn, P->perm_n});
+  if (P->ys) vecs.push_back({P->ys, prob->dual_start, vm, P->perm_m});
+  auto direct = [&](const Vec &v) { return !v.perm && v.count * 8 > kPackBytes; };
+  // device scratch of the upload, released on its stream: A as given, what its
+  // stable transpose (reference: cusparseCsr2cscEx2, src/pdlp_core_op.cu:109-130)
+  // needs beside the places of the strips, and the vectors as given
   struct Scratch {
-    void *p = nullptr;
+    void *p;
     cudaStream_t st;
     ~Scratch() { dev_free(p, st); }
   };
-  {
-    // A as given, then its stable transpose on the device (reference:
-    // cusparseCsr2cscEx2, src/pdlp_core_op.cu:109-130); in the strip format
-    // both are then laid out in the order of their rows' lengths
-    Sizer zs;
-    if (strips) {
-      zs.add<int>(vm + 1); zs.add<int>(nnz); zs.add<double>(nnz);
-      zs.add<int>(vn + 1); zs.add<int>(nnz); zs.add<double>(nnz);
-      zs.add<int>(vm); zs.add<int>(vn);
-    }
+  Sizer zs;
+  if (strips) {
+    zs.add<int>(vm + 1); zs.add<int>(nnz); zs.add<double>(nnz);
+    for (const Vec &v : vecs)
+      if (!direct(v)) zs.add<double>(v.count);
+    zs.add<int>(vn + 1); zs.add<int>(vm); zs.add<int>(vn);
+    zs.add<char>(column_sort_hist_bytes(nnz));
+  } else {
     zs.add<char>(device_transpose_scratch_bytes(n, nnz));
-    Scratch sc{dev_alloc(zs.bytes, st), st};
-    Arena sa{(char *)sc.p, 0};
-    int *ptr = P->A.ptr, *col = P->A.col, *tptr = P->AT.ptr, *tcol = P->AT.col;
-    double *val = P->A.val, *tval = P->AT.val;
-    int *inv_m = nullptr, *inv_n = nullptr;
-    if (strips) {
-      ptr = sa.take<int>(vm + 1); col = sa.take<int>(nnz); val = sa.take<double>(nnz);
-      tptr = sa.take<int>(vn + 1); tcol = sa.take<int>(nnz); tval = sa.take<double>(nnz);
-      inv_m = sa.take<int>(vm); inv_n = sa.take<int>(vn);
-    }
-    h2d(ptr, prob->constraint_matrix_row_pointers, (vm + 1) * 4);
-    h2d(col, prob->constraint_matrix_col_indices, (size_t)nnz * 4);
-    h2d(val, prob->constraint_matrix_values, (size_t)nnz * 8);
-    device_transpose(m, n, nnz, ptr, col, val, tptr, tcol, tval,
-                     sa.take<char>(device_transpose_scratch_bytes(n, nnz)), st);
-    if (strips) {
-      if (P->perm_m) k_invert<<<grid_for(m), kThreads, 0, st>>>(m, P->perm_m, inv_m);
-      if (P->perm_n) k_invert<<<grid_for(n), kThreads, 0, st>>>(n, P->perm_n, inv_n);
-      auto fill = [&](DevCsr &M, const int *sp, const int *sc, const double *sv, const int *perm,
-                      const int *icol) {
-        const long warps = (long)M.strip.nfront + M.strip.nstrip;
-        if (warps == 0) return;
-        k_strip_fill<<<grid_for(warps * 32), kThreads, 0, st>>>(strip_mat(M), sp, sc, sv, perm,
-                                                               icol, M.col, M.val);
-        PDLP_LAUNCH_CHECK();
-      };
-      fill(P->A, ptr, col, val, P->perm_m, P->perm_n ? inv_n : nullptr);
-      fill(P->AT, tptr, tcol, tval, P->perm_n, P->perm_m ? inv_m : nullptr);
-    }
   }
-  {
-    // the vectors, in the order of the format
-    const size_t most = std::max(vn, vm);
-    Scratch sc{P->perm_m || P->perm_n ? dev_alloc(most * 8, st) : nullptr, st};
-    auto vec = [&](double *dst, const double *src, int count, const int *perm) {
-      if (count == 0) return;
-      h2d(perm ? sc.p : dst, src, (size_t)count * 8);
-      if (perm) launch_gather(count, (const double *)sc.p, perm, dst, st);
+  const Scratch scratch{dev_alloc(zs.bytes, st), st};
+  Arena sa{(char *)scratch.p, 0};
+  if (strips) {
+    int *const ptr = sa.take<int>(vm + 1), *const col = sa.take<int>(nnz);
+    double *const val = sa.take<double>(nnz);
+    input.add(ptr, prob->constraint_matrix_row_pointers, (vm + 1) * 4);
+    input.add(col, prob->constraint_matrix_col_indices, (size_t)nnz * 4);
+    input.add(val, prob->constraint_matrix_values, (size_t)nnz * 8);
+    GatherList list{};
+    int lists = 0;
+    size_t most = 0;
+    for (const Vec &v : vecs) {
+      if (direct(v)) {
+        PDLP_CUDA(cudaMemcpyAsync(v.dst, v.src, v.count * 8, cudaMemcpyHostToDevice, st));
+        continue;
+      }
+      double *const raw = sa.take<double>(v.count);
+      input.add(raw, v.src, v.count * 8);
+      list.src[lists] = raw;
+      list.dst[lists] = v.dst;
+      list.perm[lists] = v.perm;
+      list.count[lists++] = (int)v.count;
+      most = std::max(most, v.count);
+    }
+    input.go(st);
+    int *const tptr = sa.take<int>(vn + 1);
+    int *const inv_m = sa.take<int>(vm), *const inv_n = sa.take<int>(vn);
+    int *const hist = (int *)sa.take<char>(column_sort_hist_bytes(nnz));
+    // the sort's arrays are where the strips will be: its result (positions and
+    // rows) in A's place, which is filled last, its keys in A^T's
+    int *const inA = P->A.col, *const inT = P->AT.col;
+    const size_t nz = nnz;
+    const ColumnSort sort{inT, inT + nz, inA, inA + nz, inA + 2 * nz, hist};
+    const int *const pos = device_column_sort(m, n, nnz, ptr, col, sort, tptr, st);
+    if (P->perm_m) k_invert<<<grid_for(m), kThreads, 0, st>>>(m, P->perm_m, inv_m);
+    if (P->perm_n) k_invert<<<grid_for(n), kThreads, 0, st>>>(n, P->perm_n, inv_n);
+    auto fill = [&](DevCsr &M, const int *sp, const int *sc, const double *sv, const int *at,
+                    const int *perm, const int *icol) {
+      const long warps = (long)M.strip.nitem + M.strip.nstrip;
+      if (warps == 0) return;
+      k_strip_fill<<<grid_for(warps * 32), kThreads, 0, st>>>(strip_mat(M), sp, sc, sv, at, perm,
+                                                             icol, M.col, M.val);
+      PDLP_LAUNCH_CHECK();
     };
-    vec(P->c, prob->objective_vector, n, P->perm_n);
-    vec(P->lv, prob->variable_lower_bound, n, P->perm_n);
-    vec(P->uv, prob->variable_upper_bound, n, P->perm_n);
-    vec(P->lc, prob->constraint_lower_bound, m, P->perm_m);
-    vec(P->uc, prob->constraint_upper_bound, m, P->perm_m);
-    if (prob->primal_start) {
-      P->xs = ar.take<double>(vn);
-      vec(P->xs, prob->primal_start, n, P->perm_n);
+    fill(P->AT, tptr, sort.rowk, val, pos, P->perm_n, P->perm_m ? inv_m : nullptr);
+    fill(P->A, ptr, col, val, nullptr, P->perm_m, P->perm_n ? inv_n : nullptr);
+    if (most > 0) {
+      k_gather<<<dim3(grid_for((long)most), lists), kThreads, 0, st>>>(list);
+      PDLP_LAUNCH_CHECK();
     }
-    if (prob->dual_start) {
-      P->ys = ar.take<double>(vm);
-      vec(P->ys, prob->dual_start, m, P->perm_m);
+    P->fp32 = std::make_shared<Fp32Order>();
+    if (for_fp32) {
+      fp32_order_upload(*P, fp32_host.get(), *P->fp32, st);
+    } else {
+      P->fp32->ptr.assign(prob->constraint_matrix_row_pointers,
+                          prob->constraint_matrix_row_pointers + m + 1);
+      P->fp32->tptr = std::move(tp);
     }
+  } else {
+    auto h2d = [&](void *dst, const void *src, size_t b) {
+      if (b) PDLP_CUDA(cudaMemcpyAsync(dst, src, b, cudaMemcpyHostToDevice, st));
+    };
+    h2d(P->A.ptr, prob->constraint_matrix_row_pointers, (vm + 1) * 4);
+    h2d(P->A.col, prob->constraint_matrix_col_indices, (size_t)nnz * 4);
+    h2d(P->A.val, prob->constraint_matrix_values, (size_t)nnz * 8);
+    device_transpose(m, n, nnz, P->A.ptr, P->A.col, P->A.val, P->AT.ptr, P->AT.col, P->AT.val,
+                     scratch.p, st);
+    for (const Vec &v : vecs) h2d(v.dst, v.src, v.count * 8);
   }
   PDLP_CUDA(cudaStreamSynchronize(st));  // host staging (plans) must outlive the copies
   return P.release();

@@ -10,6 +10,7 @@
 #include <array>
 #include <map>
 #include <memory>
+#include <mutex>
 #include <new>
 #include <string>
 #include <utility>
@@ -156,6 +157,7 @@ __host__ __device__ inline IterFlags iteration_flags(int t, int F) {
 // but its inputs and results.  Read-only once built; any number of solves can run from it.  A derived
 // problem (refinement) shares the matrices of its parent and owns only its
 // vectors.
+struct Fp32Order;
 struct DevProblem {
   int m = 0, n = 0, nnz = 0, tile = 0;
   DevCsr A, AT;  // original values; plan scratch (lcnt/lsum) is per solve
@@ -180,6 +182,10 @@ struct DevProblem {
   // the kernel of its products: -1 strips, or on plain CSR 0 fused, 1 pipelined
   int kernel = -1;
   bool strips = true;  // strip format (kernel < 0)
+  // how FP32 solves sum its rows, made when first asked for (a view shares its
+  // parent's)
+  std::shared_ptr<Fp32Order> fp32;
+  const Fp32Order &fp32_order(cudaStream_t st) const;
   int nsm = kNumSms;  // SMs of the device it was uploaded to
   ~DevProblem();
 };
@@ -189,8 +195,21 @@ int kernel_override();
 
 // Validate, transpose, plan and upload for the products' kernel (DevProblem::
 // kernel).  Throws on a malformed CSR.
+// for_fp32: with the order of its FP32 sums.
 DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st,
-                           int kernel = kernel_override());
+                           int kernel = kernel_override(), bool for_fp32 = false);
+
+// The order of a problem's FP32 sums ("FP32 sums" in strip.cuh) on the device.
+// FP64 solves do without it, so an upload that is not for an FP32 solve leaves it
+// to the first one and keeps the row pointers it follows from.
+struct Fp32Order {
+  std::mutex mu;
+  bool made = false;
+  std::vector<int> ptr, tptr;  // of A and A^T, until it is made
+  void *mem = nullptr;
+  const unsigned char *A = nullptr, *AT = nullptr;  // StripPlan::sums
+  bool pairs_A = false, pairs_AT = false;
+};
 
 // KKT measures of a point, in the reference's definitions.
 struct Kkt {
@@ -405,6 +424,15 @@ using host_buf = std::vector<T, uninit_alloc<T>>;
 // bit for bit the host transpose below; scratch of
 // device_transpose_scratch_bytes(n, nnz) bytes, all work on stream st.
 size_t device_transpose_scratch_bytes(int n, int nnz);
+// Its first part: the entries by column (rows ascending).  Returns the positions
+// of the entries in that order (in v0 or v1), fills rowk (the row of every entry)
+// and tptr.  k0, k1, v0, v1, rowk: nnz ints each.
+struct ColumnSort {
+  int *k0, *k1, *v0, *v1, *rowk, *hist;
+};
+size_t column_sort_hist_bytes(int nnz);
+const int *device_column_sort(int m, int n, int nnz, const int *ptr, const int *col,
+                              const ColumnSort &b, int *tptr, cudaStream_t st);
 void device_transpose(int m, int n, int nnz, const int *ptr, const int *col, const double *val,
                       int *tptr, int *tcol, double *tval, void *scratch, cudaStream_t st);
 

@@ -616,6 +616,14 @@ void Solve<T, M>::alloc() {
   };
   matT(A_, A64_);
   matT(AT_, AT64_);
+  if constexpr (!M64)
+    if (P_.strips) {
+      const Fp32Order &o = P_.fp32_order(st_);
+      A_.strip.sums = o.A;
+      A_.strip.pairs = o.pairs_A;
+      AT_.strip.sums = o.AT;
+      AT_.strip.pairs = o.pairs_AT;
+    }
 
   Dev<T> &d = d_;
   d.n = n;
@@ -694,9 +702,9 @@ void Solve<T, M>::apply_kernels(bool pipe) {
   Dev<T> &d = d_;
   A64_.pipe_on = A_.pipe_on = pipe && P_.A.pipe.ntile > 0;
   AT64_.pipe_on = AT_.pipe_on = pipe && P_.AT.pipe.ntile > 0;
-  d.fp32_sums = (P_.strips ? P_.A.strip.pairs != 0 : pipe) ? kFp32Pairs
-                : P_.tile == 512                              ? kFp32Tiles512
-                                                              : kFp32Tiles;
+  d.fp32_sums = (P_.strips ? A_.strip.pairs != 0 : pipe) ? kFp32Pairs
+                : P_.tile == 512                           ? kFp32Tiles512
+                                                           : kFp32Tiles;
   d.nblkA = (int)spmv_partials(A64_);
   d.nlongA = (int)spmv_long_rows(A64_);
   d.nblkT = (int)spmv_partials(AT64_);

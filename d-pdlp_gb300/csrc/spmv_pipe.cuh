@@ -157,7 +157,11 @@ inline void build_pipe_plan_host(int rows, const int *ptr, int NV, std::vector<i
       while (r < rows && r - r0 < kPipeRows) {
         const int l2 = ptr[r + 1] - ptr[r];
         if (l2 > kPipeMedRows || ptr[r + 1] - ptr[r0] > kPipeTile) break;
-        if (pipe_tile_bytes(make_int4(r0, r + 1, ptr[r0], ptr[r + 1]), NV) > kPipeTileBytes) break;
+        // (the bound first: the exact bytes matter near the limit only)
+        if (4 * (r + 2 - r0) + 12 * (ptr[r + 1] - ptr[r0]) + NV * 8 * (r + 3 - r0) + 96 >
+                kPipeTileBytes &&
+            pipe_tile_bytes(make_int4(r0, r + 1, ptr[r0], ptr[r + 1]), NV) > kPipeTileBytes)
+          break;
         ++r;
       }
     }

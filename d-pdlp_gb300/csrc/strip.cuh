@@ -42,6 +42,8 @@
 // kernel strides a long row with.
 #pragma once
 
+#include <limits.h>
+
 #include <algorithm>
 #include <vector>
 
@@ -76,14 +78,11 @@ struct StripPlan {
 };
 
 struct StripHost {
-  std::vector<int> perm;       // position -> original row
-  bool identity = true;        // perm is 0, 1, 2, ...
+  std::vector<int> perm;       // position -> original row (empty: the same)
   std::vector<int> fptr;       // element offsets of the front's rows
   std::vector<int4> item;
   std::vector<int2> lrow;
   std::vector<int> off;
-  std::vector<unsigned char> sums;  // how each row is summed in FP32
-  bool pairs = false;
   int lg = 0;
   long store = 0;
 };
@@ -168,28 +167,32 @@ inline void strip_sums_pipe(int rows, const int *ptr, int nv, std::vector<unsign
 inline void build_strip_host(int rows, const int *ptr, int sms, int chunk, StripHost &h) {
   h = StripHost();
   h.lg = strip_lanes(rows, sms);
-  h.perm.resize(rows);
   // stable order by decreasing length: the front by sorting, the rest by
   // counting
   std::vector<int> front;
   std::vector<int> count(kStripRow + 2, 0);
-  for (int r = 0; r < rows; ++r) {
+  bool sorted = true;
+  for (int r = 0, before = INT_MAX; r < rows; ++r) {
     const int len = ptr[r + 1] - ptr[r];
+    sorted &= len <= before;
+    before = len;
     if (len > kStripRow) front.push_back(r);
     else ++count[kStripRow - len + 1];
   }
-  std::stable_sort(front.begin(), front.end(), [&](int a, int b) {
-    return ptr[a + 1] - ptr[a] > ptr[b + 1] - ptr[b];
-  });
   const int nfront = (int)front.size();
-  std::copy(front.begin(), front.end(), h.perm.begin());
-  count[0] = nfront;
-  for (int l = 1; l <= kStripRow + 1; ++l) count[l] += count[l - 1];
-  for (int r = 0; r < rows; ++r) {
-    const int len = ptr[r + 1] - ptr[r];
-    if (len <= kStripRow) h.perm[count[kStripRow - len]++] = r;
+  if (!sorted) {
+    h.perm.resize(rows);
+    std::stable_sort(front.begin(), front.end(), [&](int a, int b) {
+      return ptr[a + 1] - ptr[a] > ptr[b + 1] - ptr[b];
+    });
+    std::copy(front.begin(), front.end(), h.perm.begin());
+    count[0] = nfront;
+    for (int l = 1; l <= kStripRow + 1; ++l) count[l] += count[l - 1];
+    for (int r = 0; r < rows; ++r) {
+      const int len = ptr[r + 1] - ptr[r];
+      if (len <= kStripRow) h.perm[count[kStripRow - len]++] = r;
+    }
   }
-  for (int i = 0; i < rows && h.identity; ++i) h.identity = h.perm[i] == i;
   // front: items and chunks.  Items of a small front are smaller, down to a
   // row each: as many as keep them within 8 warps of each SM (a transport LP
   // of 854 x 94, 800 FP64 iterations and the set-up: 22.0 -> 17.4 ms)
@@ -221,8 +224,8 @@ inline void build_strip_host(int rows, const int *ptr, int sms, int chunk, Strip
   const int lanes = 1 << h.lg;
   for (int r = nfront; r < rows; r += 32 / lanes) {
     h.off.push_back((int)at);
-    // its first row is its longest
-    at += (ptr[h.perm[r] + 1] - ptr[h.perm[r]] + lanes - 1) / lanes;
+    const int first = sorted ? r : h.perm[r];  // its longest row
+    at += (ptr[first + 1] - ptr[first] + lanes - 1) / lanes;
   }
   h.off.push_back((int)at);
   h.store = at * 32;

@@ -147,11 +147,9 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
-// A^T: row pointers from the sorted keys, columns (rows of A) and values
-__global__ void k_transpose_out(int n, int nnz, const int *__restrict__ skeys,
-                                const int *__restrict__ spos, const int *__restrict__ rowk,
-                                const double *__restrict__ val, int *__restrict__ tptr,
-                                int *__restrict__ tcol, double *__restrict__ tval) {
+// A^T: row pointers from the sorted keys ...
+__global__ void k_column_ptr(int n, int nnz, const int *__restrict__ skeys,
+                             int *__restrict__ tptr) {
   const long stride = (long)gridDim.x * blockDim.x;
   for (long j = blockIdx.x * (long)blockDim.x + threadIdx.x; j <= n; j += stride) {
     int lo = 0, hi = nnz;  // first position with key >= j
@@ -162,6 +160,13 @@ __global__ void k_transpose_out(int n, int nnz, const int *__restrict__ skeys,
     }
     tptr[j] = lo;
   }
+}
+
+// ... columns (rows of A) and values
+__global__ void k_transpose_out(int nnz, const int *__restrict__ spos,
+                                const int *__restrict__ rowk, const double *__restrict__ val,
+                                int *__restrict__ tcol, double *__restrict__ tval) {
+  const long stride = (long)gridDim.x * blockDim.x;
   for (long p = blockIdx.x * (long)blockDim.x + threadIdx.x; p < nnz; p += stride) {
     const int k = spos[p];
     tcol[p] = rowk[k];
@@ -171,41 +176,57 @@ __global__ void k_transpose_out(int n, int nnz, const int *__restrict__ skeys,
 
 }  // namespace
 
+size_t column_sort_hist_bytes(int nnz) {
+  const long ntiles = ((long)nnz + kTileKeys - 1) / kTileKeys;
+  return (size_t)kDigits * (ntiles > 0 ? ntiles : 1) * 4;
+}
+
 size_t device_transpose_scratch_bytes(int n, int nnz) {
   (void)n;
-  const long ntiles = ((long)nnz + kTileKeys - 1) / kTileKeys;
-  return 5 * ((size_t)nnz * 4 + 256) + (size_t)kDigits * (ntiles > 0 ? ntiles : 1) * 4 + 256;
+  return 5 * ((size_t)nnz * 4 + 256) + column_sort_hist_bytes(nnz) + 256;
+}
+
+const int *device_column_sort(int m, int n, int nnz, const int *ptr, const int *col,
+                              const ColumnSort &b, int *tptr, cudaStream_t st) {
+  int *k0 = b.k0, *k1 = b.k1, *v0 = b.v0, *v1 = b.v1;
+  const int ntiles = (int)(((long)nnz + kTileKeys - 1) / kTileKeys);
+  const int g = grid_for(nnz > n + 1 ? nnz : n + 1);
+  if (nnz > 0) {
+    PDLP_CUDA(cudaMemcpyAsync(k0, col, (size_t)nnz * 4, cudaMemcpyDeviceToDevice, st));
+    k_iota<<<g, kThreads, 0, st>>>(nnz, v0);
+    k_row_of<<<g, kThreads, 0, st>>>(m, nnz, ptr, b.rowk);
+    PDLP_LAUNCH_CHECK();
+    int bits = 0;
+    while (bits < 31 && (1L << bits) < (long)n) ++bits;
+    for (int shift = 0; shift < bits; shift += kRadixBits) {
+      k_digit_hist<<<ntiles, kThreads, 0, st>>>(nnz, shift, k0, ntiles, b.hist);
+      k_scan_hist<<<1, 1024, 0, st>>>((long)kDigits * ntiles, b.hist);
+      k_scatter<<<ntiles, kThreads, 0, st>>>(nnz, shift, k0, v0, k1, v1, ntiles, b.hist);
+      PDLP_LAUNCH_CHECK();
+      std::swap(k0, k1);
+      std::swap(v0, v1);
+    }
+  }
+  k_column_ptr<<<g, kThreads, 0, st>>>(n, nnz, k0, tptr);
+  PDLP_LAUNCH_CHECK();
+  return v0;
 }
 
 void device_transpose(int m, int n, int nnz, const int *ptr, const int *col, const double *val,
                       int *tptr, int *tcol, double *tval, void *scratch, cudaStream_t st) {
   auto a256 = [](size_t b) { return (b + 255) & ~(size_t)255; };
   char *p = (char *)scratch;
-  int *k0 = (int *)p; p += a256((size_t)nnz * 4);
-  int *k1 = (int *)p; p += a256((size_t)nnz * 4);
-  int *v0 = (int *)p; p += a256((size_t)nnz * 4);
-  int *v1 = (int *)p; p += a256((size_t)nnz * 4);
-  int *rowk = (int *)p; p += a256((size_t)nnz * 4);
-  int *hist = (int *)p;
-  const int ntiles = (int)(((long)nnz + kTileKeys - 1) / kTileKeys);
-  const int g = grid_for(nnz > n + 1 ? nnz : n + 1);
-  if (nnz > 0) {
-    PDLP_CUDA(cudaMemcpyAsync(k0, col, (size_t)nnz * 4, cudaMemcpyDeviceToDevice, st));
-    k_iota<<<g, kThreads, 0, st>>>(nnz, v0);
-    k_row_of<<<g, kThreads, 0, st>>>(m, nnz, ptr, rowk);
-    PDLP_LAUNCH_CHECK();
-    int bits = 0;
-    while (bits < 31 && (1L << bits) < (long)n) ++bits;
-    for (int shift = 0; shift < bits; shift += kRadixBits) {
-      k_digit_hist<<<ntiles, kThreads, 0, st>>>(nnz, shift, k0, ntiles, hist);
-      k_scan_hist<<<1, 1024, 0, st>>>((long)kDigits * ntiles, hist);
-      k_scatter<<<ntiles, kThreads, 0, st>>>(nnz, shift, k0, v0, k1, v1, ntiles, hist);
-      PDLP_LAUNCH_CHECK();
-      std::swap(k0, k1);
-      std::swap(v0, v1);
-    }
-  }
-  k_transpose_out<<<g, kThreads, 0, st>>>(n, nnz, k0, v0, rowk, val, tptr, tcol, tval);
+  auto take = [&] {
+    int *q = (int *)p;
+    p += a256((size_t)nnz * 4);
+    return q;
+  };
+  ColumnSort b;
+  b.k0 = take(); b.k1 = take(); b.v0 = take(); b.v1 = take(); b.rowk = take();
+  b.hist = (int *)p;
+  const int *pos = device_column_sort(m, n, nnz, ptr, col, b, tptr, st);
+  if (nnz == 0) return;
+  k_transpose_out<<<grid_for(nnz), kThreads, 0, st>>>(nnz, pos, b.rowk, val, tcol, tval);
   PDLP_LAUNCH_CHECK();
 }
 

@@ -110,6 +110,8 @@ HostFlag *hostflag_acquire();
 void hostflag_release(HostFlag *f);
 // Return the pool's cached blocks to the device.
 void release_pooled_memory();
+// most bytes of the device's pool in use at once since the last reset
+long long pooled_memory_high(bool reset);
 
 __device__ __forceinline__ unsigned long long global_ns() {
   unsigned long long t;

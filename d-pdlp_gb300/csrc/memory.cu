@@ -90,6 +90,20 @@ void hostflag_release(HostFlag *f) {
   }
 }
 
+long long pooled_memory_high(bool reset) {
+  try {
+    cudaMemPool_t p = device_pool();
+    unsigned long long v = 0;
+    PDLP_CUDA(cudaMemPoolGetAttribute(p, cudaMemPoolAttrUsedMemHigh, &v));
+    unsigned long long zero = 0;
+    if (reset) PDLP_CUDA(cudaMemPoolSetAttribute(p, cudaMemPoolAttrUsedMemHigh, &zero));
+    return (long long)v;
+  } catch (const std::exception &) {
+    cudaGetLastError();
+    return -1;
+  }
+}
+
 void release_pooled_memory() {
   std::lock_guard<std::mutex> lk(g_pool_mu);
   for (auto &p : g_pool)

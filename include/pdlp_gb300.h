@@ -228,6 +228,9 @@ long long pdlp_server_submit_bytes(pdlp_server_t *s, const void *buf, long long 
 
 /* Return the device memory cached by the library's pool. */
 void pdlp_release_pooled_memory(void);
+/* Most bytes of the current device's pool in use at once since the last call
+ * with a non-zero `reset`; -1 on a CUDA error. */
+long long pdlp_pooled_memory_high(int reset);
 
 /* Message of the last failure in this thread ("" if none). */
 const char *pdlp_last_error(void);

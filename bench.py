@@ -222,16 +222,19 @@ def kernel_bytes(m, n, nnz, s=8):
     return primal, dual
 
 
-def load_traffic(workload, precision, kernel):
-    """DRAM bytes per launch of a step kernel from one ncu capture
-    (profiles/ncu_traffic.json), or None."""
+SPMV_KERNELS = ["fused", "pipelined", "strip"]  # pdlp_solve_info_t.spmv_kernel_A / _AT
+
+
+def load_traffic(workload, precision, step, kernel):
+    """DRAM bytes per launch of a step on one of SPMV_KERNELS from an ncu capture
+    (profiles/ncu_traffic.json), or None where none of that kernel is recorded."""
     path = os.path.join(ROOT, "profiles", "ncu_traffic.json")
     if not os.path.exists(path):
         return None
     try:
         with open(path) as f:
             d = json.load(f)
-        e = d.get(workload, {}).get(precision, {}).get(kernel)
+        e = d.get(workload, {}).get(precision, {}).get(step, {}).get(kernel)
         return None if e is None else float(e["dram_bytes_per_launch"])
     except (ValueError, KeyError, TypeError):
         return None
@@ -381,9 +384,12 @@ def run_ours(args, cp, rank, world, local):
     dom = max(kernels, key=lambda k: kernels[k][0])
     peak, peak_kind = load_peaks()
     ach = kernels[dom][1] / (kernels[dom][0] * 1e-3) / 1e9
+    on_kernel = {"A": SPMV_KERNELS[out.info["spmv_kernel_A"]],
+                 "A^T": SPMV_KERNELS[out.info["spmv_kernel_AT"]]}
     iters, pm_iters = r["total_count"], last.info["power_iterations"]
-    # uploaded by solve_lp_problem: A and A^T (CSR), c, bounds, power start vector
-    h2d = 4 * (m + 1) + 4 * (n + 1) + 24 * nnz + 24 * n + 16 * m + 8 * m
+    # uploaded by solve_lp_problem: A in CSR (A^T is built on the device), c, bounds,
+    # power start vector; the format's tables (a few bytes a row) are not counted
+    h2d = 4 * (m + 1) + 12 * nnz + 24 * n + 16 * m + 8 * m
     d2h = 8 * (2 * n + m)  # primal, reduced cost, dual
     line = {
         "metric": METRIC, "value": round(value, 4), "unit": "s", "n_gpus": world,
@@ -404,7 +410,8 @@ def run_ours(args, cp, rank, world, local):
         "gpu_launches": int(launches),
         "roofline": {"bound": "hbm", "kernel": dom, "achieved": round(ach, 1), "peak": peak,
                      "unit": "GB/s", "frac": round(ach / peak, 4),
-                     "traffic": load_traffic(name, args.precision, dom),
+                     "traffic": load_traffic(name, args.precision, dom,
+                                             on_kernel["A" if dom == "dual_step" else "A^T"]),
                      "peak_source": f"{peak_kind} hbm_gbs (STREAM copy; the only HBM figure "
                                     "measured)",
                      "algorithmic_bytes_per_launch": kernels[dom][1],
@@ -415,8 +422,7 @@ def run_ours(args, cp, rank, world, local):
                      "timing": timing,
                      "isolated_ms": {"primal_step": round(ms[0], 4), "dual_step": round(ms[1], 4),
                                      "eval_A": round(ms[2], 4), "eval_AT": round(ms[3], 4)}},
-        "spmv_kernels": {"A": ["fused", "pipelined", "strip"][out.info["spmv_kernel_A"]],
-                         "A^T": ["fused", "pipelined", "strip"][out.info["spmv_kernel_AT"]]},
+        "spmv_kernels": on_kernel,
         "solve": {"status": r["status"], "iterations": iters, "power_iterations": pm_iters,
                   "rel_primal": r["relative_primal_residual"],
                   "rel_dual": r["relative_dual_residual"], "rel_gap": r["relative_objective_gap"],

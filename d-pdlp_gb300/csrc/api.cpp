@@ -671,11 +671,17 @@ int pdlp_gpu_rescale(const lp_problem_t *prob, const pdhg_parameters_t *params, 
       fetch(off.data(), M.strip.off, off.size());
       const int *rp = prob->constraint_matrix_row_pointers;
       for (int i = 0; i < m; ++i) {
-        const int r = om[i], q = i - M.strip.nfront, lg = M.strip.lg, H = 32 >> lg;
+        const pdlp::StripPlan &p = M.strip;
+        const int r = om[i], q = i - p.nfront;
+        // its strip, if it has one
+        const bool wide = i < p.wide_end;
+        const int lg = wide ? p.lgw : p.lg, H = 32 >> lg;
+        const int place = wide ? q : i - p.wide_end, strip = (wide ? 0 : p.nwide) + place / H;
         for (int k = 0; k < rp[r + 1] - rp[r]; ++k)
           vals[rp[r] + k] =
               q < 0 ? v[front[i] + k]
-                    : v[((size_t)off[q / H] + (k >> lg)) * 32 + ((q % H) << lg) + (k & ((1 << lg) - 1))];
+                    : v[((size_t)off[strip] + (k >> lg)) * 32 + ((place % H) << lg) +
+                        (k & ((1 << lg) - 1))];
       }
     } else {
       fetch(vals, M.val, M.nnz);

@@ -150,10 +150,10 @@ __global__ void __launch_bounds__(kThreads)
   }
   for (int s = w0; s < A.p.nstrip; s += W) {
     const int o0 = A.p.off[s], n = A.p.off[s + 1] - o0;
-    const int lg = A.p.lg, G = 1 << lg;
-    const int row = A.p.nfront + s * (32 >> lg) + (lane >> lg);
+    const StripPlace place = strip_place(A.p, A.rows, s);
+    const int lg = place.lg, G = 1 << lg, row = place.row + (lane >> lg);
     const size_t at = (size_t)o0 * 32 + lane;
-    const bool live = row < A.rows;
+    const bool live = row < place.end;
     const double a = SCALE && live ? rs[row] : 1.0;
     U64 mx = 0;
     double sum = 0.0;

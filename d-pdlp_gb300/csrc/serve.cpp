@@ -173,27 +173,29 @@ extern "C" {
 long long pdlp_estimate_device_bytes(int m, int n, long long nnz, int precision) {
   if (m < 0 || n < 0 || nnz < 0) return -1;
   const long long vm = m, vn = n, slack = 8 << 20;  // small buffers, padding of rows with several lanes
-  // both matrices' units: items of rows longer than 64 (at most one to 65 non-zeros) and
-  // strips of 32 rows (or a few thousand smaller ones)
-  const long long units = 2 * (nnz / 65) + (vm + vn) / 32 + 4096;
+  // a matrix's stored elements: rows longer than 64 are padded to a multiple of 8
+  const long long kept = nnz + nnz / 9;
+  // both matrices' units: items of rows longer than 256 (at most one to 128 non-zeros),
+  // strips of four rows longer than 64 and of 32 others (or a few thousand smaller ones)
+  const long long units = 2 * (nnz / 128) + 2 * (nnz / 260) + (vm + vn) / 32 + 4096;
   // resident problem: A and A^T in strips, item and strip tables, order of the
   // rows, their FP32 sums, objective, bounds and start values
-  const long long resident = 24 * nnz + 20 * units + 5 * (vm + vn) + 32 * vn + 24 * vm + slack;
+  const long long resident = 24 * kept + 20 * units + 5 * (vm + vn) + 32 * vn + 24 * vm + slack;
   // FP64 solve: scaled values, scaled vectors, iterates, power method and output vectors,
   // item sums and partial sums (per 8 units), and for LPs that a team may run the
   // iterates once more and partial sums per unit.  The upload's scratch (A in CSR,
   // the vectors as given) is gone by then.
   const long long team_rows = 2 * 2432 * 32;
   const long long state = 64 * std::min(vn, team_rows) + 48 * std::min(vm, team_rows);
-  const long long solve = 16 * nnz + 136 * vn + 112 * vm + 24 * units + state + slack;
+  const long long solve = 16 * kept + 136 * vn + 112 * vm + 24 * units + state + slack;
   // (the CSR of a kernel that PDLP_STEP_KERNEL forces: the transpose's 21 instead)
   const long long upload =
       (pdlp::kernel_override() < 0 ? 13 : 21) * nnz + 36 * vn + 32 * vm + slack;
   if (precision == PDLP_PRECISION_FP64) return resident + std::max(solve, upload);
   // mixed precision: an FP32 copy of the values, the snapshot of the best point, the
   // refinement's own vectors and the FP64 evaluator beside the round's solve
-  return resident + solve + 8 * nnz + 16 * vn + 8 * vm + state +
-         (16 * nnz + 136 * vn + 112 * vm + 24 * units + slack) + 72 * vn + 56 * vm + 16 * units;
+  return resident + solve + 8 * kept + 16 * vn + 8 * vm + state +
+         (16 * kept + 136 * vn + 112 * vm + 24 * units + slack) + 72 * vn + 56 * vm + 16 * units;
 }
 
 pdlp_server_t *pdlp_server_create(const pdhg_parameters_t *params, const pdlp_options_t *opts,

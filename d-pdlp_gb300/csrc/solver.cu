@@ -166,10 +166,11 @@ __global__ void __launch_bounds__(kThreads)
       }
       continue;
     }
-    const int s = w - A.p.nitem, lg = A.p.lg;
-    const int row = A.p.nfront + s * (32 >> lg) + (lane >> lg), sub = lane & ((1 << lg) - 1);
+    const int s = w - A.p.nitem;
+    const StripPlace place = strip_place(A.p, A.rows, s);
+    const int lg = place.lg, row = place.row + (lane >> lg), sub = lane & ((1 << lg) - 1);
     int a = 0, len = 0;
-    if (row < A.rows) {
+    if (row < place.end) {
       const int r = perm ? perm[row] : row;
       a = sptr[r];
       len = sptr[r + 1] - a;
@@ -709,7 +710,10 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel
     p.nitem = (int)h.item.size();
     p.nlong = (int)h.lrow.size();
     p.nstrip = (int)h.off.size() - 1;
+    p.nwide = h.nwide;
+    p.wide_end = h.wide_end;
     p.lg = h.lg;
+    p.lgw = h.lgw;
     p.store = h.store;
     const long warps = (long)p.nitem + p.nstrip, per = kThreads / 32;
     p.grid = (int)((warps + per - 1) / per);

@@ -20,6 +20,9 @@
 //     to give the chip's warps a strip each has 2, 4 or 8 lanes to a row (and
 //     16, 8 or 4 rows to a strip): there the time is the chain of a strip's
 //     loads (about 1,300 cycles for four elements), not the issue slots;
+//   * rows of up to kWideRow have 8 lanes each in strips of their own (wide
+//     strips, which stand before the others), or 16 or 32 in a small matrix:
+//     one reduction over 8 lanes for four rows instead of one over 32 for each;
 //   * longer rows come first (the front), in CSR order: a warp takes items of
 //     consecutive rows of together up to kStripItem non-zeros (lanes stride a
 //     row, its lane sums are added across lanes in FP64, and the item's rows
@@ -54,13 +57,15 @@
 namespace pdlp {
 
 constexpr int kStripRow = 64;     // longest row of a strip
+constexpr int kWideRow = 256;     // longest row of a wide strip
 constexpr int kStripItem = 1024;  // non-zeros of a front item
 
 struct StripPlan {
   int on = 0;                  // the matrix is stored in this format
-  int nfront = 0;              // rows longer than kStripRow (they come first)
+  int nfront = 0;              // rows longer than kWideRow (they come first)
+  int nwide = 0, wide_end = 0; // wide strips and the end of their rows
   int nitem = 0, nlong = 0, nstrip = 0;
-  int lg = 0;                  // a strip's rows have 1 << lg lanes each
+  int lg = 0, lgw = 0;         // a strip's (wide strip's) rows have 1 << lg lanes each
   // reduction partials: one per strip, whatever warp took it, for LPs that a
   // team may run (team.cuh); else one per block
   int unit_parts = 0;
@@ -83,15 +88,26 @@ struct StripHost {
   std::vector<int4> item;
   std::vector<int2> lrow;
   std::vector<int> off;
-  int lg = 0;
+  int nwide = 0, wide_end = 0;
+  int lg = 0, lgw = 0;
   long store = 0;
 };
 
+// Strip s of a matrix: the lanes of its rows, its first row and the end of the
+// rows of its kind.
+struct StripPlace {
+  int lg, row, end;
+};
+__host__ __device__ inline StripPlace strip_place(const StripPlan &p, int rows, int s) {
+  if (s < p.nwide) return {p.lgw, p.nfront + s * (32 >> p.lgw), p.wide_end};
+  return {p.lg, p.wide_end + (s - p.nwide) * (32 >> p.lg), rows};
+}
+
 // Lanes of a row (as their logarithm): as many as keep the strips within 8
 // warps of each of `sms` SMs.
-inline int strip_lanes(long rows, int sms) {
-  int lg = 0;
-  while (lg < 3 && (rows << (lg + 1)) <= 32L * 8 * sms) ++lg;
+inline int strip_lanes(long rows, int sms, int least = 0, int most = 3) {
+  int lg = least;
+  while (lg < most && (rows << (lg + 1)) <= 32L * 8 * sms) ++lg;
   return lg;
 }
 
@@ -170,16 +186,19 @@ inline void build_strip_host(int rows, const int *ptr, int sms, int chunk, Strip
   // stable order by decreasing length: the front by sorting, the rest by
   // counting
   std::vector<int> front;
-  std::vector<int> count(kStripRow + 2, 0);
+  std::vector<int> count(kWideRow + 2, 0);
   bool sorted = true;
   for (int r = 0, before = INT_MAX; r < rows; ++r) {
     const int len = ptr[r + 1] - ptr[r];
     sorted &= len <= before;
     before = len;
-    if (len > kStripRow) front.push_back(r);
-    else ++count[kStripRow - len + 1];
+    if (len > kWideRow) front.push_back(r);
+    else ++count[kWideRow - len + 1];
   }
   const int nfront = (int)front.size();
+  h.wide_end = nfront;
+  for (int l = 1; l <= kWideRow - kStripRow; ++l) h.wide_end += count[l];
+  h.lgw = strip_lanes(h.wide_end - nfront, sms, 3, 5);
   if (!sorted) {
     h.perm.resize(rows);
     std::stable_sort(front.begin(), front.end(), [&](int a, int b) {
@@ -187,10 +206,10 @@ inline void build_strip_host(int rows, const int *ptr, int sms, int chunk, Strip
     });
     std::copy(front.begin(), front.end(), h.perm.begin());
     count[0] = nfront;
-    for (int l = 1; l <= kStripRow + 1; ++l) count[l] += count[l - 1];
+    for (int l = 1; l <= kWideRow + 1; ++l) count[l] += count[l - 1];
     for (int r = 0; r < rows; ++r) {
       const int len = ptr[r + 1] - ptr[r];
-      if (len <= kStripRow) h.perm[count[kStripRow - len]++] = r;
+      if (len <= kWideRow) h.perm[count[kWideRow - len]++] = r;
     }
   }
   // front: items and chunks.  Items of a small front are smaller, down to a
@@ -221,12 +240,16 @@ inline void build_strip_host(int rows, const int *ptr, int sms, int chunk, Strip
   }
   // strips
   long at = ((long)h.fptr.back() + 31) / 32;
-  const int lanes = 1 << h.lg;
-  for (int r = nfront; r < rows; r += 32 / lanes) {
-    h.off.push_back((int)at);
-    const int first = sorted ? r : h.perm[r];  // its longest row
-    at += (ptr[first + 1] - ptr[first] + lanes - 1) / lanes;
-  }
+  auto strips = [&](int begin, int end, int lanes) {
+    for (int r = begin; r < end; r += 32 / lanes) {
+      h.off.push_back((int)at);
+      const int first = sorted ? r : h.perm[r];  // its longest row
+      at += (ptr[first + 1] - ptr[first] + lanes - 1) / lanes;
+    }
+  };
+  strips(nfront, h.wide_end, 1 << h.lgw);
+  h.nwide = (int)h.off.size();
+  strips(h.wide_end, rows, 1 << h.lg);
   h.off.push_back((int)at);
   h.store = at * 32;
 }
@@ -298,6 +321,15 @@ struct StripSum<float, PAIR> {
     if constexpr (PAIR) return isfinite(all.lo()) ? all.rounded() : all.hi();
     else return all;
   }
+  // pairs of a row's lanes, after total()
+  __device__ __forceinline__ float across(int lanes) {
+    for (int o = 1; o < lanes; o <<= 1) {
+      const float h = __shfl_xor_sync(0xffffffffu, all.hi(), o);
+      const float l = __shfl_xor_sync(0xffffffffu, all.lo(), o);
+      all.add_pair(h, l);
+    }
+    return isfinite(all.lo()) ? all.rounded() : all.hi();
+  }
 };
 
 template <class Epi, class M>
@@ -345,15 +377,6 @@ __device__ __forceinline__ void strip_head(const StripMat<M> &A, int s, StripHea
   strip_load<STREAM>(A.col + at, A.val + at, x.n, x.q);
 }
 
-// Row of this lane in strip s, and whether it is the lane that ends the row.
-template <class M>
-__device__ __forceinline__ int strip_row(const StripMat<M> &A, int s, bool &ends) {
-  const int lane = threadIdx.x & 31, lg = A.p.lg;
-  const int row = A.p.nfront + s * (32 >> lg) + (lane >> lg);
-  ends = row < A.rows && (lane & ((1 << lg) - 1)) == 0;
-  return row;
-}
-
 // Sums of the strip rows (FP32) that the fused kernel strides with several
 // lanes (see "FP32 sums"), by the whole warp, row by row: its lanes take those
 // lanes' parts of the row.  total: this lane's row's sum.  Such a row stands
@@ -393,14 +416,15 @@ __device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi,
                                            int s, const StripHead<M> &head) {
   const int lane = threadIdx.x & 31, o0 = head.o0, n = head.n;
   StripQuad<M> q = head.q;
-  bool ends;
-  const int row = strip_row(A, s, ends);
+  // the row of this lane, and whether it is the lane that ends the row
+  const StripPlace place = strip_place(A.p, A.rows, s);
+  const int lg = place.lg, row = place.row + (lane >> lg);
+  const bool ends = row < place.end && (lane & ((1 << lg) - 1)) == 0;
   const int *col = A.col + (size_t)o0 * 32 + lane;
   const M *val = A.val + (size_t)o0 * 32 + lane;
   typename pre_of<Epi>::type pre;
   if constexpr (has_preload<Epi>::value)
     if (ends) epi.preload(row, pre);
-  const int lg = A.p.lg;
   int how = 0;
   if constexpr (sizeof(M) == 4) how = row < A.rows ? __ldg(A.p.sums + row) : 8 << 4;
   StripSum<M, PAIR> sum(how);
@@ -423,7 +447,7 @@ __device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi,
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       if (k + u >= n) break;  // the same for every lane
-      if (sizeof(M) == 8 || lg == 0) {
+      if (sizeof(M) == 8 || PAIR || lg == 0) {
         if (sizeof(M) == 8 || q.c[u] >= 0) sum.add(u % 2 && n > 2, q.v[u], x[u]);
       } else {
         // a row's elements in their order, by every lane of the row
@@ -443,6 +467,8 @@ __device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi,
   M total = sum.total(n > 2);
   if constexpr (sizeof(M) == 8)
     for (int o = 1; o < (1 << lg); o <<= 1) total += __shfl_xor_sync(0xffffffffu, total, o);
+  if constexpr (sizeof(M) == 4 && PAIR)
+    if (lg > 0) total = sum.across(1 << lg);
   if constexpr (sizeof(M) == 4 && !PAIR)
     if (n > 1 || lg > 0) strip_strided<STREAM>(epi, col - lane, val - lane, n, lg, ends, how, total);
   if (ends) strip_epilogue(epi, row, total, pre, acc);

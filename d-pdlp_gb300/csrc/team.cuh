@@ -155,7 +155,7 @@ class TeamTurn {
 };
 
 // CTAs of the team for an LP's matrices; 0: no team.  A matrix with a front (rows
-// of more than 64 entries) has none: its items and their sums need a barrier
+// of more than 256 entries) has none: its items and their sums need a barrier
 // more per product and leave most warps of a team idle (an LP with such rows:
 // 25 ms against 17 ms with a kernel per product).  Nor has one with more than
 // two strips for a warp: the barriers no longer show beside the strips, but every

@@ -51,6 +51,10 @@ LENGTHS = {
     "short_alone": ([40, 500] * 60, 700),
     "last_tile_one_row": ([16] * 32 + [7], 300),
     "edges": ([63, 64, 65, 0, 1, 31, 32, 33] * 20 + [511, 512, 513, 1023, 1024, 1025, 5000], 6000),
+    # rows of 65 to 256 have 32, 16 and 8 lanes
+    "wide_32_lanes": ([65, 127, 128, 255, 256, 257, 30] * 20, 9000),
+    "wide_16_lanes": ([65, 100, 256, 3] * 600, 9000),
+    "wide_8_lanes": ([65, 73, 256, 260, 7] * 1200, 90000),
     "eight_lanes": ([9] * 3000, 5003),
     "four_lanes": ([9] * 9000, 12000),
     "one_lane": ([6] * 45001, 50021),

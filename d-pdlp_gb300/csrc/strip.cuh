@@ -636,13 +636,14 @@ __device__ __forceinline__ void strip_block_partials(const double (&acc)[NA], do
 // the compiler keeps a dozen vector pointers in registers (spills at 48), at
 // the price of the gathers in flight.
 // Bound by FP64 issue (16 cycles per warp instruction and SM) and by the
-// gathers' L2 requests.  20M non-zeros, ms per launch, before (the faster of
-// the CSR kernels) and now: power-law dual step 0.121 -> 0.083 (FP32 0.101 ->
-// 0.053), primal step 0.152 -> 0.146 (FP32 0.103 -> 0.132: the segments of its
-// sums); transport evaluation over A^T 0.375 -> 0.305, primal step, whose rows
-// have two entries, 0.185 -> 0.203.  5 blocks per SM: 6 spill more (FP32 primal
-// step 0.139; FP32 pairs, which need fewer registers, run at 6), 4 (no spills)
-// take the transport primal step to 0.258.
+// gathers' L2 requests.  20M non-zeros, ms per launch inside a solve, before (the
+// faster of the CSR kernels), with a block's warps far apart in the list, and
+// now: power-law primal step 0.155, 0.147, 0.120 (FP32 0.106, 0.123, 0.102), dual
+// step 0.128, 0.089, 0.084 (FP32 0.104, 0.057, 0.051); transport primal step
+// 0.185, 0.206, 0.204 (FP32 0.132, 0.118, 0.118), dual step 0.108, 0.112, 0.096
+// (FP32 0.084, 0.104, 0.074).  5 blocks per SM: 6 spill more (FP32 power-law
+// primal step 0.139 against 0.132 ms; FP32 pairs, which need fewer registers, run
+// at 6), 4 (no spills) took the transport primal step to 0.258.
 template <class Epi, bool STREAM, bool PAIR>
 __global__ void __launch_bounds__(kThreads, sizeof(typename Epi::val_t) == 8 || !PAIR ? 5 : 6)
     spmv_strip(const __grid_constant__ StripMat<typename Epi::val_t> A,
@@ -650,8 +651,9 @@ __global__ void __launch_bounds__(kThreads, sizeof(typename Epi::val_t) == 8 || 
   using M = typename Epi::val_t;
   constexpr int NF = Epi::NF;
   __shared__ double sc[4];
-  // the warps of a block are far apart in the (longest first) list
-  const int w = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+  // a block's warps are neighbours in the list: of one length, so that none
+  // holds the block's place on the SM for long, and with gathers in common
+  const int w = blockIdx.x * (kThreads / 32) + (threadIdx.x >> 5);
   const int units = A.p.nitem + A.p.nstrip;
   if (!epi.init()) return;
   if (threadIdx.x == 0) epi.prologue(sc);

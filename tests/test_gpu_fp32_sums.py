@@ -55,6 +55,8 @@ LENGTHS = {
     "wide_32_lanes": ([65, 127, 128, 255, 256, 257, 30] * 20, 9000),
     "wide_16_lanes": ([65, 100, 256, 3] * 600, 9000),
     "wide_8_lanes": ([65, 73, 256, 260, 7] * 1200, 90000),
+    # a front in which rows of up to 2,048 are not cut
+    "whole_rows": ([2048] * 700 + [2049] * 600 + [1025, 1500, 3000] * 40, 20000),
     "eight_lanes": ([9] * 3000, 5003),
     "four_lanes": ([9] * 9000, 12000),
     "one_lane": ([6] * 45001, 50021),

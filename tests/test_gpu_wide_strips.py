@@ -19,6 +19,8 @@ SHAPES = {
     "8_lanes": ([65, 71, 72, 73, 256, 2] * 600, 90000, True),
     "8_lanes_no_team": ([65, 130, 256, 257, 300, 2] * 600 + [1500, 1024, 1025], 90000, False),
     "only_wide": ([100] * 37, 500, True),
+    # a front in which rows of up to 2,048 are not cut
+    "whole_rows": ([2048] * 700 + [2049] * 600 + [1025, 1500, 3000] * 40, 20000, False),
 }
 
 

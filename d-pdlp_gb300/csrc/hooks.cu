@@ -30,6 +30,13 @@ struct RowSumEpi {
   __device__ void row(int r, T s, double *) const { y[r] = s; }
 };
 using PlainEpi = RowSumEpi<double>;
+// ... in the kernels of the step epilogues, which load their rows' vectors ahead
+template <class T>
+struct RowSumPreEpi : RowSumEpi<T> {
+  struct Pre {};
+  __device__ void preload(int, Pre &) const {}
+  __device__ void row_pre(int r, T s, const Pre &, double *) const { this->y[r] = s; }
+};
 
 }  // namespace pdlp
 
@@ -156,7 +163,7 @@ extern "C" int pdlp_gpu_products_fp32(const lp_problem_t *prob, int kernel, cons
       float *da = mem.p, *db = mem.p + a.size();
       if (!a.empty())
         PDLP_CUDA(cudaMemcpyAsync(da, a.data(), a.size() * 4, cudaMemcpyHostToDevice, st));
-      launch_spmv(M, RowSumEpi<float>{da, db}, nullptr, nullptr, st);
+      launch_spmv(M, RowSumPreEpi<float>{{da, db}}, nullptr, nullptr, st);
       if (!b.empty())
         PDLP_CUDA(cudaMemcpyAsync(b.data(), db, b.size() * 4, cudaMemcpyDeviceToHost, st));
       PDLP_CUDA(cudaStreamSynchronize(st));

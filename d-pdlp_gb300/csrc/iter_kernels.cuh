@@ -462,8 +462,14 @@ void launch_spmv(const DevCsrT<V> &M, const Epi &epi, double *part, double *lpar
   if (M.strip.on) {
     if (M.strip.grid == 0) return;
     auto go = [&](auto stream, auto pair) {
-      spmv_strip<Epi, decltype(stream)::value, decltype(pair)::value>
-          <<<M.strip.grid, kThreads, 0, st>>>(strip_mat(M), part, lpart, epi);
+      constexpr bool S = decltype(stream)::value, P = decltype(pair)::value;
+      if constexpr (has_preload<Epi>::value && S)
+        if (M.strip.narrow) {
+          spmv_strip<Epi, S, P, true>
+              <<<M.strip.grid, kThreads, 0, st>>>(strip_mat(M), part, lpart, epi);
+          return;
+        }
+      spmv_strip<Epi, S, P><<<M.strip.grid, kThreads, 0, st>>>(strip_mat(M), part, lpart, epi);
     };
     using Yes = std::true_type;
     using No = std::false_type;

@@ -715,6 +715,9 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel
     p.lg = h.lg;
     p.lgw = h.lgw;
     p.store = h.store;
+    // (rows stand in decreasing length: the first strip is the widest)
+    p.narrow = p.nitem == 0 && p.nwide == 0 && p.lg == 0 && p.nstrip > 0 &&
+               h.off[1] - h.off[0] <= kNarrow;
     const long warps = (long)p.nitem + p.nstrip, per = kThreads / 32;
     p.grid = (int)((warps + per - 1) / per);
     up(M.ptr, h.fptr);

@@ -60,6 +60,7 @@ namespace pdlp {
 constexpr int kStripRow = 64;     // longest row of a strip
 constexpr int kWideRow = 256;     // longest row of a wide strip
 constexpr int kStripItem = 1024;  // non-zeros of a front item (of several rows)
+constexpr int kNarrow = 2;        // elements of a narrow matrix's strips
 
 struct StripPlan {
   int on = 0;                  // the matrix is stored in this format
@@ -71,6 +72,7 @@ struct StripPlan {
   // team may run (team.cuh); else one per block
   int unit_parts = 0;
   int pairs = 0;               // FP32 sums in pairs (see above)
+  int narrow = 0;              // strips of up to kNarrow elements only, a lane a row
   int grid = 0;                // blocks of the product kernel (8 items or strips each)
   long store = 0;              // stored elements, padding included
   int *off = nullptr;          // strip s: 32-element columns off[s] .. off[s + 1]
@@ -371,7 +373,7 @@ struct StripHead {
   int o0, n;
   StripQuad<M> q;
 };
-template <bool STREAM, class M>
+template <bool STREAM, int MOST = 4, class M>
 __device__ __forceinline__ void strip_head(const StripMat<M> &A, int s, StripHead<M> &x) {
   x.o0 = x.n = 0;
   if (s < A.p.nstrip) {
@@ -379,7 +381,7 @@ __device__ __forceinline__ void strip_head(const StripMat<M> &A, int s, StripHea
     x.n = __ldg(A.p.off + s + 1) - x.o0;
   }
   const size_t at = (size_t)x.o0 * 32 + (threadIdx.x & 31);
-  strip_load<STREAM>(A.col + at, A.val + at, x.n, x.q);
+  strip_load<STREAM>(A.col + at, A.val + at, MOST < 4 ? min(x.n, MOST) : x.n, x.q);
 }
 
 // Sums of the strip rows (FP32) that the fused kernel strides with several
@@ -415,15 +417,15 @@ __device__ __forceinline__ void strip_strided(const Epi &epi, const int *col, co
   }
 }
 
-// Strip s, by a warp; `head` as strip_head loaded it.
-template <bool STREAM, bool PAIR, class Epi, class M>
+// Strip s, by a warp; `head` as strip_head loaded it.  NARROW: of a narrow matrix.
+template <bool STREAM, bool PAIR, bool NARROW = false, class Epi, class M>
 __device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi, double *acc,
                                            int s, const StripHead<M> &head) {
   const int lane = threadIdx.x & 31, o0 = head.o0, n = head.n;
   StripQuad<M> q = head.q;
   // the row of this lane, and whether it is the lane that ends the row
   const StripPlace place = strip_place(A.p, A.rows, s);
-  const int lg = place.lg, row = place.row + (lane >> lg);
+  const int lg = NARROW ? 0 : place.lg, row = place.row + (lane >> lg);
   const bool ends = row < place.end && (lane & ((1 << lg) - 1)) == 0;
   const int *col = A.col + (size_t)o0 * 32 + lane;
   const M *val = A.val + (size_t)o0 * 32 + lane;
@@ -436,13 +438,14 @@ __device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi,
   // four elements ahead, but not in FP32 kernels that stream: at their 40
   // registers it spills (power-law dual step 0.088 ms ahead, 0.053 without;
   // FP64 0.083 ahead, 0.087 without)
-  constexpr bool kAhead = sizeof(M) == 8 || !STREAM;
+  constexpr bool kAhead = (sizeof(M) == 8 || !STREAM) && !NARROW;
+  constexpr int kLoad = NARROW ? kNarrow : 4;
 #pragma unroll 1
-  for (int k = 0; k < n; k += 4) {
-    M x[4];
+  for (int k = 0; k < (NARROW ? 1 : n); k += 4) {
+    M x[kLoad];
     // padding: no load, and 0 times the padding's 0
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < kLoad; ++u) {
       x[u] = M(0);
       if (q.c[u] >= 0) x[u] = epi.gather(q.c[u]);
     }
@@ -450,7 +453,7 @@ __device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi,
     if constexpr (kAhead)
       strip_load<STREAM>(col + (k + 4) * 32, val + (k + 4) * 32, n - k - 4, next);
 #pragma unroll
-    for (int u = 0; u < 4; ++u) {
+    for (int u = 0; u < kLoad; ++u) {
       if (k + u >= n) break;  // the same for every lane
       if (sizeof(M) == 8 || PAIR || lg == 0) {
         if (sizeof(M) == 8 || q.c[u] >= 0) sum.add(u % 2 && n > 2, q.v[u], x[u]);
@@ -466,7 +469,7 @@ __device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi,
     }
     if constexpr (kAhead)
       q = next;
-    else
+    else if constexpr (!NARROW)
       strip_load<STREAM>(col + (k + 4) * 32, val + (k + 4) * 32, n - k - 4, q);
   }
   M total = sum.total(n > 2);
@@ -649,8 +652,15 @@ __device__ __forceinline__ void strip_block_partials(const double (&acc)[NA], do
 // (FP32 0.084, 0.104, 0.074).  5 blocks per SM: 6 spill more (FP32 power-law
 // primal step 0.139 against 0.132 ms; FP32 pairs, which need fewer registers, run
 // at 6), 4 (no spills) took the transport primal step to 0.258.
-template <class Epi, bool STREAM, bool PAIR>
-__global__ void __launch_bounds__(kThreads, sizeof(typename Epi::val_t) == 8 || !PAIR ? 5 : 6)
+// NARROW: the step kernels of a large matrix whose rows have at most two entries
+// (a transport LP's columns).  There is no loop and nothing but one strip, so 8
+// blocks fit an SM, and their vectors' loads are what such a step is: transport
+// primal step 0.204 -> 0.201 ms (6 blocks 0.207), FP32 0.118 -> 0.096, FP32
+// matrix 0.218 -> 0.181 (before the strips 0.185, 0.132 and 0.201).
+template <class Epi, bool STREAM, bool PAIR, bool NARROW = false>
+__global__ void __launch_bounds__(kThreads, NARROW ? 8
+                                            : sizeof(typename Epi::val_t) == 8 || !PAIR ? 5
+                                                                                        : 6)
     spmv_strip(const __grid_constant__ StripMat<typename Epi::val_t> A,
                double *__restrict__ part, double *__restrict__ lpart, Epi epi) {
   using M = typename Epi::val_t;
@@ -668,6 +678,15 @@ __global__ void __launch_bounds__(kThreads, sizeof(typename Epi::val_t) == 8 || 
 #pragma unroll
   for (int f = 0; f < (NF > 0 ? NF : 1); ++f) acc[f] = 0.0;
   const int lane = threadIdx.x & 31;
+  if constexpr (NARROW) {
+    if (w < units) {
+      StripHead<M> head;
+      strip_head<STREAM, kNarrow>(A, w, head);
+      strip_rows<STREAM, PAIR, true>(A, epi, acc, w, head);
+    }
+    if constexpr (NF > 0) strip_block_partials<NF, Epi::MAXMASK>(acc, part);
+    return;
+  }
   auto unit = [&](int i) {
     if (i >= A.p.nitem) {
       StripHead<M> head;

@@ -80,6 +80,8 @@ PAIRS = {
     "one_long_row": ([21] * 200000 + [70, 300], 400000),
     "front_of_100": ([100] * 43000, 400000),
     "rows_of_500": ([500] * 8500, 400000),
+    # the step kernels of matrices whose rows have at most two entries
+    "narrow": ([2, 2, 1, 0, 2] * 1000000, 90000),
 }
 
 

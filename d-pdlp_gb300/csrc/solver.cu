@@ -550,7 +550,7 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel
                            });
   auto plans_A = [&] {
     if (strips) {
-      build_strip_host(m, prob->constraint_matrix_row_pointers, nsm, chunk, shA);
+      build_strip_host(m, prob->constraint_matrix_row_pointers, nsm, P->tile, chunk, shA);
       return;
     }
     build_plan_host(m, prob->constraint_matrix_row_pointers, P->tile, blkA, lrA, chunk);
@@ -570,7 +570,7 @@ DevProblem *upload_problem(const lp_problem_t *prob, cudaStream_t st, int kernel
     plans_A();
   try {
     if (strips) {
-      build_strip_host(n, tp.data(), nsm, chunk, shT);
+      build_strip_host(n, tp.data(), nsm, P->tile, chunk, shT);
     } else {
       build_plan_host(n, tp.data(), P->tile, blkT, lrT, chunk);
       build_pipe_plan_host(n, tp.data(), 5, pblkT, plrT);

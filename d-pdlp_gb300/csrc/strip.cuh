@@ -181,9 +181,11 @@ inline void strip_sums_pipe(int rows, const int *ptr, int nv, std::vector<unsign
   }
 }
 
-// Host: order and cut the rows of a CSR matrix; chunk: elements of a long
-// row's chunk (a multiple of 256).
-inline void build_strip_host(int rows, const int *ptr, int sms, int chunk, StripHost &h) {
+// Host: order and cut the rows of a CSR matrix; tile: the longest row that the
+// fused kernel does not cut, chunk: elements of a long row's chunk (a multiple
+// of 256).
+inline void build_strip_host(int rows, const int *ptr, int sms, int tile, int chunk,
+                             StripHost &h) {
   h = StripHost();
   h.lg = strip_lanes(rows, sms);
   // stable order by decreasing length: the front by sorting, the rest by
@@ -224,8 +226,9 @@ inline void build_strip_host(int rows, const int *ptr, int sms, int chunk, Strip
   const int most = std::min(kStripItem, h.fptr.back() / (8 * sms));
   // a row of more than this is cut: in a large front, whose rows fill the chip as
   // they are, only above twice an item (5,300 rows of 1,500, FP32 dual step 0.061
-  // -> 0.043 ms: no sums to store and count)
-  const int whole = std::max(kStripItem, std::min(2 * kStripItem, h.fptr.back() / (8 * sms)));
+  // -> 0.043 ms: no sums to store and count); in a small one all rows that the
+  // fused kernel cuts too, so that a warp's rounds of loads are few
+  const int whole = std::max(tile, std::min(2 * kStripItem, h.fptr.back() / (8 * sms)));
   for (int i = 0; i < nfront;) {
     const int a = h.fptr[i], e = h.fptr[i + 1];
     if (e - a > whole) {
@@ -554,8 +557,36 @@ __device__ __forceinline__ float strip_row_sum(const StripMat<float> &A, const E
   if (how >= kSumStrided) {
     const int lanes = 1 << (how - kSumStrided);
     double t = 0.0;
-    for (int j = lane; j < lanes; j += 32)
-      t += (double)strip_chain<STREAM>(A, epi, a + j, e, lanes, 0.f);
+    if (lanes <= 32) {
+      if (lane < lanes) t = (double)strip_chain<STREAM>(A, epi, a + lane, e, lanes, 0.f);
+    } else {
+      // four of the lanes' chains side by side: a row that 256 lanes take has a
+      // few elements for each
+      constexpr int U = 4;
+#pragma unroll 1
+      for (int j = lane; j < lanes; j += 32 * U) {
+        float s[U] = {};
+#pragma unroll 1
+        for (int k = a + j; k < e; k += lanes) {
+          int c[U];
+          float v[U], x[U];
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (j + 32 * u < lanes && k + 32 * u < e) {
+              c[u] = ld_matrix<STREAM>(A.col + k + 32 * u);
+              v[u] = ld_matrix<STREAM>(A.val + k + 32 * u);
+            }
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (j + 32 * u < lanes && k + 32 * u < e) x[u] = epi.gather(c[u]);
+#pragma unroll
+          for (int u = 0; u < U; ++u)
+            if (j + 32 * u < lanes && k + 32 * u < e) s[u] = fmaf(v[u], x[u], s[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u) t += (double)s[u];
+      }
+    }
     return (float)warp_sum(t);
   }
   // segments: a lane each, added in order

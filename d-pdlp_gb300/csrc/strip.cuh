@@ -420,6 +420,93 @@ __device__ __forceinline__ void strip_strided(const Epi &epi, const int *col, co
   }
 }
 
+// Sum of this lane's row in a wide strip (FP32) where the fused kernel strides it
+// with at least its 1 << lg lanes here: element k of lane j is element (k << lg) + j
+// of the row, so that a lane's elements are those of one, two or four of the fused
+// kernel's lanes in turn, or, of 256, of a lane each.
+template <bool STREAM, class Epi>
+__device__ __forceinline__ float strip_wide_strided(const Epi &epi, const int *col,
+                                                    const float *val, int n, int lg, int how) {
+  const int turns = 1 << max(0, how - kSumStrided - lg);  // the fused kernel's lanes of a lane
+  float s[4] = {};
+  double t = 0.0;
+#pragma unroll 1
+  for (int k = 0; k < n; k += 4) {
+    StripQuad<float> q;
+    strip_load<STREAM>(col + k * 32, val + k * 32, n - k, q);
+    float x[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (q.c[u] >= 0) x[u] = epi.gather(q.c[u]);
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (q.c[u] >= 0) {
+        if (turns > 4) t += (double)fmaf(q.v[u], x[u], 0.f);
+        else if (turns == 4) s[u] = fmaf(q.v[u], x[u], s[u]);
+        else if (turns == 2) s[u & 1] = fmaf(q.v[u], x[u], s[u & 1]);
+        else s[0] = fmaf(q.v[u], x[u], s[0]);
+      }
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) t += (double)s[u];
+  for (int o = 1; o < (1 << lg); o <<= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  return (float)t;
+}
+
+// Sum of this lane's row in a wide strip (FP32, not in pairs), by the row's 1 << lg
+// lanes: a lane folds every (1 << lg)th segment, eight elements' loads at a time,
+// and the segments are added in order.  Element by element, every lane of the row
+// would add all of them with three shuffles each.  col, val: of the row's first
+// lane.
+template <bool STREAM, class Epi>
+__device__ __forceinline__ float strip_segments(const Epi &epi, const int *col, const float *val,
+                                                int n, int lg, int how) {
+  const int lane = threadIdx.x & 31, G = 1 << lg, base = lane & ~(G - 1);
+  const int len = how >= kSumStrided ? 8 : how >> 4, phase = how >= kSumStrided ? 0 : how & 15;
+  const int all_elements = n << lg;
+  // rounds of the row with the most segments in the strip
+  const int rounds = (all_elements + 7 + 3) / 4 / G + 1;
+  float all = -0.f;
+#pragma unroll 1
+  for (int r = 0; r < rounds; ++r) {
+    const int first = (r * G + lane - base) * len - phase;
+    float s = 0.f;
+    bool any = false;
+    constexpr int U = 4;
+#pragma unroll
+    for (int h = 0; h < 8; h += U) {
+      int c[U];
+      float v[U], x[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const int e = first + h + u;
+        c[u] = -1;
+        if (h + u < len && e >= 0 && e < all_elements) {
+          const int at = (e >> lg) * 32 + (e & (G - 1));
+          c[u] = ld_matrix<STREAM>(col + at);
+          v[u] = ld_matrix<STREAM>(val + at);
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (c[u] >= 0) x[u] = epi.gather(c[u]);
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (c[u] >= 0) {
+          s = fmaf(v[u], x[u], s);
+          any = true;
+        }
+    }
+    const unsigned real = __ballot_sync(0xffffffffu, any);
+    if (real == 0u) break;
+    for (int g = 0; g < G; ++g) {
+      const float add = __shfl_sync(0xffffffffu, s, base + g);
+      if ((real >> (base + g)) & 1u) all += add;
+    }
+  }
+  return all;
+}
+
 // Strip s, by a warp; `head` as strip_head loaded it.  NARROW: of a narrow matrix.
 template <bool STREAM, bool PAIR, bool NARROW = false, class Epi, class M>
 __device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi, double *acc,
@@ -437,6 +524,22 @@ __device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi,
     if (ends) epi.preload(row, pre);
   int how = 0;
   if constexpr (sizeof(M) == 4) how = row < A.rows ? __ldg(A.p.sums + row) : 8 << 4;
+  if constexpr (sizeof(M) == 4 && !PAIR && !NARROW)
+    if (s < A.p.nwide) {
+      const int up = lane & ((1 << lg) - 1);
+      const bool strided = how >= kSumStrided;
+      M total = M(0);
+      if (__any_sync(0xffffffffu, !strided))
+        total = strip_segments<STREAM>(epi, col - up, val - up, n, lg, how);
+      if (__any_sync(0xffffffffu, strided)) {
+        const M t = strip_wide_strided<STREAM>(epi, col, val, n, lg, how);
+        if (strided) total = t;
+        strip_strided<STREAM>(epi, col - lane, val - lane, n, lg,
+                              ends && how - kSumStrided < lg, how, total);
+      }
+      if (ends) strip_epilogue(epi, row, total, pre, acc);
+      return;
+    }
   StripSum<M, PAIR> sum(how);
   // four elements ahead, but not in FP32 kernels that stream: at their 40
   // registers it spills (power-law dual step 0.088 ms ahead, 0.053 without;

@@ -188,7 +188,9 @@ __global__ void __launch_bounds__(kThreads)
   }
 }
 
+template <bool WIDE>
 struct TeamPower {
+  static constexpr bool kWide = WIDE;
   PowDev d;
   StripMat<double> A, AT;
 };
@@ -197,11 +199,12 @@ struct TeamPower {
 // residual is below sv_tol or `maxit` are done, two barriers each.  Every CTA
 // folds the sums itself; the residual of an iteration is checked after the
 // next one's A^T product, which writes nothing the result depends on.
+template <bool WIDE>
 __global__ void __launch_bounds__(kTeamThreads, kTeamCtasPerSm)
-    team_power(const __grid_constant__ TeamPower data, const __grid_constant__ TeamBar bar,
+    team_power(const __grid_constant__ TeamPower<WIDE> data, const __grid_constant__ TeamBar bar,
                int maxit) {
   __shared__ TeamSmem sm;
-  __shared__ TeamPower sd;
+  __shared__ TeamPower<WIDE> sd;
   Ctl *c = data.d.ctl;
   if (ld_flag(&c->pm_done)) return;
   team_copy(data, sd, sm);
@@ -214,8 +217,8 @@ __global__ void __launch_bounds__(kTeamThreads, kTeamCtasPerSm)
   for (;;) {
     if (it < maxit)
       team_phase<0, 0u>(
-          sd, [](const TeamPower &x) -> const auto & { return x.AT; },
-          [=](const TeamPower &x) {
+          sd, [](const TeamPower<WIDE> &x) -> const auto & { return x.AT; },
+          [=](const TeamPower<WIDE> &x) {
             return PowAtEpi<const PowDev &>{x.d, (it & 1) ? x.d.v[1] : x.d.v[0], inv};
           },
           nullptr, xT);
@@ -230,8 +233,8 @@ __global__ void __launch_bounds__(kTeamThreads, kTeamCtasPerSm)
     // `>=`: a limit below zero ends it here too (a launch must always end)
     if (it >= maxit || (check && res < d.sv_tol)) break;
     team_phase<2, 0u>(
-        sd, [](const TeamPower &x) -> const auto & { return x.A; },
-        [=](const TeamPower &x) {
+        sd, [](const TeamPower<WIDE> &x) -> const auto & { return x.A; },
+        [=](const TeamPower<WIDE> &x) {
           return PowAEpi<const PowDev &>{x.d, (it & 1) ? x.d.v[1] : x.d.v[0],
                                          (it & 1) ? x.d.v[0] : x.d.v[1], inv};
         },
@@ -270,13 +273,15 @@ __global__ void __launch_bounds__(kTeamThreads, kTeamCtasPerSm)
 
 bool launch_team_power(int ctas, cudaStream_t st, const PowDev &d, const StripMat<double> &A,
                        const StripMat<double> &AT, const TeamBar &bar, int maxit) {
-  return team_launch(ctas, team_power, st, TeamPower{d, A, AT}, bar, maxit);
+  return A.p.nwide + AT.p.nwide > 0
+             ? team_launch(ctas, team_power<true>, st, TeamPower<true>{d, A, AT}, bar, maxit)
+             : team_launch(ctas, team_power<false>, st, TeamPower<false>{d, A, AT}, bar, maxit);
 }
 
-long long team_wait_cycles() {
-  const char *e = getenv("PDLP_TEAM_WAIT_CYCLES");
-  const long long v = e ? atoll(e) : 0;
-  return v > 0 ? v : kBulkWaitCycles;
+void team_reset(unsigned *count, cudaStream_t st) {
+  const char *e = getenv("PDLP_TEAM_FAIL");
+  // 0xC0C0C0C0 arrivals are 1.06e9 short of 0
+  PDLP_CUDA(cudaMemsetAsync(count, e && e[0] == '1' ? 0xC0 : 0, sizeof(unsigned), st));
 }
 
 namespace {

@@ -884,10 +884,10 @@ void Solve<T, M>::power_method() {
 
 template <class T, class M>
 bool Solve<T, M>::power_method_team() {
-  PDLP_CUDA(cudaMemsetAsync(team_count_, 0, sizeof(unsigned), st_));
+  team_reset(team_count_, st_);
   const bool launched =
       launch_team_power(team_, st_, pw_, strip_mat(A64_), strip_mat(AT64_),
-                        {team_count_, team_err_, team_wait_cycles()}, p_.sv_max_iter);
+                        {team_count_, team_err_}, p_.sv_max_iter);
   launches_ += launched;
   if (!team_finished(launched)) return false;
   Ctl c;
@@ -914,8 +914,7 @@ bool Solve<T, M>::team_finished(bool launched) {
 // when a barrier's wait ran out: the state is then again that of iteration t.
 template <class T, class M>
 bool Solve<T, M>::run_team(int t, int t1) {
-  const TeamRun r{{team_count_, team_err_, team_wait_cycles()}, snapshot_ ? 1 : 0};
-  const TeamData<T, M> data{d_, strip_mat(A_), strip_mat(AT_), strip_mat(A64_), strip_mat(AT64_)};
+  const TeamRun r{{team_count_, team_err_}, snapshot_ ? 1 : 0};
   auto copy = [&](void *dst, const void *src, size_t bytes) {
     if (bytes) PDLP_CUDA(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToDevice, st_));
   };
@@ -924,8 +923,15 @@ bool Solve<T, M>::run_team(int t, int t1) {
   char *const snap_save = (char *)snap_mem_ + snap_bytes_;
   copy(team_save_, d_.x[0], state_bytes_);
   copy(snap_save, snap_mem_, snap);
-  PDLP_CUDA(cudaMemsetAsync(team_count_, 0, sizeof(unsigned), st_));
-  const bool launched = team_launch(team_, team_loop<T, M>, st_, data, r, t, t1);
+  team_reset(team_count_, st_);
+  auto go = [&](auto wide) {
+    constexpr bool W = decltype(wide)::value;
+    const TeamData<T, M, W> data{d_, strip_mat(A_), strip_mat(AT_), strip_mat(A64_),
+                                 strip_mat(AT64_)};
+    return team_launch(team_, team_loop<T, M, W>, st_, data, r, t, t1);
+  };
+  const bool launched = P_.A.strip.nwide + P_.AT.strip.nwide > 0 ? go(std::true_type{})
+                                                                 : go(std::false_type{});
   launches_ += launched;
   if (team_finished(launched)) return true;
   copy(d_.x[0], team_save_, state_bytes_);

@@ -507,14 +507,17 @@ __device__ __forceinline__ float strip_segments(const Epi &epi, const int *col, 
   return all;
 }
 
-// Strip s, by a warp; `head` as strip_head loaded it.  NARROW: of a narrow matrix.
-template <bool STREAM, bool PAIR, bool NARROW = false, class Epi, class M>
+// Strip s, by a warp; `head` as strip_head loaded it.  NARROW: of a narrow matrix;
+// WIDE: of a matrix that may have wide strips.
+template <bool STREAM, bool PAIR, bool NARROW = false, bool WIDE = !NARROW, class Epi, class M>
 __device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi, double *acc,
                                            int s, const StripHead<M> &head) {
   const int lane = threadIdx.x & 31, o0 = head.o0, n = head.n;
   StripQuad<M> q = head.q;
   // the row of this lane, and whether it is the lane that ends the row
-  const StripPlace place = strip_place(A.p, A.rows, s);
+  const StripPlace place =
+      WIDE ? strip_place(A.p, A.rows, s)
+           : StripPlace{A.p.lg, A.p.nfront + s * (32 >> A.p.lg), A.rows};
   const int lg = NARROW ? 0 : place.lg, row = place.row + (lane >> lg);
   const bool ends = row < place.end && (lane & ((1 << lg) - 1)) == 0;
   const int *col = A.col + (size_t)o0 * 32 + lane;
@@ -524,7 +527,7 @@ __device__ __forceinline__ void strip_rows(const StripMat<M> &A, const Epi &epi,
     if (ends) epi.preload(row, pre);
   int how = 0;
   if constexpr (sizeof(M) == 4) how = row < A.rows ? __ldg(A.p.sums + row) : 8 << 4;
-  if constexpr (sizeof(M) == 4 && !PAIR && !NARROW)
+  if constexpr (sizeof(M) == 4 && !PAIR && WIDE)
     if (s < A.p.nwide) {
       const int up = lane & ((1 << lg) - 1);
       const bool strided = how >= kSumStrided;

@@ -37,7 +37,6 @@ constexpr int kTeamCtasPerSm = 2;
 struct TeamBar {
   unsigned *count;  // arrivals so far (0 at launch)
   int *err;         // set when a wait ran out
-  long long wait;   // its limit in cycles
 };
 
 struct TeamSmem {
@@ -47,7 +46,8 @@ struct TeamSmem {
 };
 
 // Barrier over the team: writes before it are visible after it.  False, in
-// every thread of the CTA, when the wait ran out (TeamBar::wait): the caller
+// every thread of the CTA, when the wait ran out (kBulkWaitCycles, a constant: read
+// from memory the limit costs a 40k x 100k LP 1.5 us an iteration): the caller
 // returns, and the other CTAs' waits run out too.  The host then takes the
 // launch's work back and repeats it with a kernel per product.
 __device__ __forceinline__ bool team_sync(const TeamBar &b, TeamSmem &sm) {
@@ -63,7 +63,7 @@ __device__ __forceinline__ bool team_sync(const TeamBar &b, TeamSmem &sm) {
       unsigned seen;
       asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(b.count) : "memory");
       if ((int)(seen - target) >= 0) break;
-      if (clock64() - t0 > b.wait) {
+      if (clock64() - t0 > kBulkWaitCycles) {
         atomicOr(b.err, 1);
         ok = 0;
         break;
@@ -111,7 +111,7 @@ __device__ __forceinline__ void team_phase(const Data &data, Mat mat, Make make,
     double acc[NF > 0 ? NF : 1];
 #pragma unroll
     for (int f = 0; f < (NF > 0 ? NF : 1); ++f) acc[f] = 0.0;
-    strip_rows<false, false>(mat(here), make(here), acc, s, x);
+    strip_rows<false, false, false, Data::kWide>(mat(here), make(here), acc, s, x);
     if constexpr (NF > 0) strip_partials<NF, MAXMASK>(acc, part, s, mat(here).p.nstrip);
     s += W;
     if (s >= mat(here).p.nstrip) return;
@@ -172,10 +172,10 @@ inline int team_ctas(long nnz, const StripPlan &A, const StripPlan &AT, int nsm)
   return work <= nsm * kTeamWarps ? std::max(1, std::min(work, nsm)) : nsm * kTeamCtasPerSm;
 }
 
-// Limit of a barrier's wait: that of the mbarrier waits, or
-// PDLP_TEAM_WAIT_CYCLES.  It runs out when the CTAs stop running at the same
-// time, as on a GPU whose time slices are longer.
-long long team_wait_cycles();
+// Sets a team's arrival counter for a launch: to 0, or, with PDLP_TEAM_FAIL=1, to
+// a number from which no barrier completes, so that every wait runs out (as where
+// the CTAs do not run at the same time for longer than that).
+void team_reset(unsigned *count, cudaStream_t st);
 
 // False when the device cannot hold the team's CTAs at once (an SM limit on
 // the process, say): nothing was launched.

@@ -65,9 +65,12 @@ struct TeamRun {
   int snapshot;
 };
 
-// What a team reads throughout; the kernel keeps a copy in shared memory.
-template <class T, class M>
+// What a team reads throughout; the kernel keeps a copy in shared memory.  WIDE: one
+// of the matrices has wide strips (without them the kernels are 2% faster on small
+// LPs, whose time is a few chains of instructions an iteration).
+template <class T, class M, bool WIDE>
 struct TeamData {
+  static constexpr bool kWide = WIDE;
   Dev<T> d;
   StripMat<M> A, AT;
   StripMat<double> A64, AT64;
@@ -93,10 +96,10 @@ __device__ __forceinline__ void team_blocks(int ew_grid, Body &&body) {
 }
 
 // KKT evaluation of iteration t; false when a barrier wait ran out.
-template <class T, class M>
-__device__ __noinline__ bool team_eval(const TeamData<T, M> &sd, const TeamRun r, TeamSmem &sm,
+template <class T, class M, bool WIDE>
+__device__ __noinline__ bool team_eval(const TeamData<T, M, WIDE> &sd, const TeamRun r, TeamSmem &sm,
                                        int t, bool infeas, bool restart_check) {
-  using Data = TeamData<T, M>;
+  using Data = TeamData<T, M, WIDE>;
   const Dev<T> &d = sd.d;
   auto on_A = [](const Data &x) -> const auto & { return x.A64; };
   auto on_AT = [](const Data &x) -> const auto & { return x.AT64; };
@@ -161,8 +164,8 @@ __device__ __noinline__ bool team_eval(const TeamData<T, M> &sd, const TeamRun r
 }
 
 // Restart of iteration t: the copies and the primal-weight update.
-template <class T, class M>
-__device__ __noinline__ bool team_restart(const TeamData<T, M> &sd, const TeamRun r, TeamSmem &sm,
+template <class T, class M, bool WIDE>
+__device__ __noinline__ bool team_restart(const TeamData<T, M, WIDE> &sd, const TeamRun r, TeamSmem &sm,
                                           int t) {
   const Dev<T> &d = sd.d;
   team_blocks(d.ew_grid, [&](int b, long first, long stride) {
@@ -185,11 +188,11 @@ __device__ __noinline__ bool team_restart(const TeamData<T, M> &sd, const TeamRu
 
 // An iteration that needs dx, dy and their norms, up to the barrier that ends
 // it, and its fixed-point error.
-template <class T, class M>
-__device__ __noinline__ bool team_step_fpe(const TeamData<T, M> &sd, const TeamRun r, TeamSmem &sm,
+template <class T, class M, bool WIDE>
+__device__ __noinline__ bool team_step_fpe(const TeamData<T, M, WIDE> &sd, const TeamRun r, TeamSmem &sm,
                                            T tau, T sigma, T inv_sigma, T w, T omw, int par,
                                            bool major, bool fpe) {
-  using Data = TeamData<T, M>;
+  using Data = TeamData<T, M, WIDE>;
   const Dev<T> &d = sd.d;
   auto on_A = [](const Data &x) -> const auto & { return x.A; };
   auto on_AT = [](const Data &x) -> const auto & { return x.AT; };
@@ -250,11 +253,11 @@ static __device__ __noinline__ unsigned team_flags(int t, int F, bool polish) {
 // Solve::enqueue_iteration.  What one iteration hands to the next, other than
 // its number, is in shared memory: registers that live across the calls below
 // would be spilled, also by the iterations that make none.
-template <class T, class M>
+template <class T, class M, bool WIDE>
 __global__ void __launch_bounds__(kTeamThreads, kTeamCtasPerSm)
-    team_loop(const __grid_constant__ TeamData<T, M> data, const __grid_constant__ TeamRun run,
+    team_loop(const __grid_constant__ TeamData<T, M, WIDE> data, const __grid_constant__ TeamRun run,
               int t0, int t1) {
-  using Data = TeamData<T, M>;
+  using Data = TeamData<T, M, WIDE>;
   __shared__ TeamSmem sm;
   __shared__ Data sd;
   __shared__ TeamRun r;

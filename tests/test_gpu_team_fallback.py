@@ -1,7 +1,7 @@
 """A resident team whose barrier waits run out: the solve takes the launch's work
-back, goes on with a kernel per product, and returns the same bits.  The wait
-limit is set to one cycle, so that every CTA but the last to arrive gives up at
-its first barrier."""
+back, goes on with a kernel per product, and returns the same bits.  The arrival
+counter starts where no barrier completes, so that every CTA gives up at its
+first one after the wait's limit (2 s)."""
 import numpy as np
 import pytest
 
@@ -17,7 +17,7 @@ def test_solve_goes_on_without_the_team(oracle, monkeypatch, precision):
     prob = cp.Problem.generated("random", 2000, 5000, 20000, 7)
     p = params(oracle, eps=1e-12, iteration_limit=1700)
     team = cp.solve(prob, p, precision=precision)
-    monkeypatch.setenv("PDLP_TEAM_WAIT_CYCLES", "1")
+    monkeypatch.setenv("PDLP_TEAM_FAIL", "1")
     alone = cp.solve(prob, p, precision=precision)
     # the second one really ran as single launches
     assert alone.info["kernel_launches"] > 2000 > team.info["kernel_launches"]

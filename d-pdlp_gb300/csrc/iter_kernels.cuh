@@ -430,16 +430,15 @@ inline size_t spmv_long_rows(const DevCsrT<V> &M) {
   if (M.strip.on) return (size_t)M.strip.nlong;
   return use_pipe(M) ? (size_t)M.pipe.nlong : (size_t)M.plan.nlong;
 }
-// partial buffers large enough for either kernel
+// partial buffers large enough for either CSR kernel
 template <class V>
 inline size_t spmv_partials_max(const DevCsrT<V> &M) {
-  if (M.strip.on)
-    return (size_t)(M.strip.unit_parts ? M.strip.nitem + M.strip.nstrip : M.strip.grid);
+  if (M.strip.on) return spmv_partials(M);
   return (size_t)(M.pipe.grid > M.plan.nblk ? M.pipe.grid : M.plan.nblk);
 }
 template <class V>
 inline size_t spmv_long_rows_max(const DevCsrT<V> &M) {
-  if (M.strip.on) return (size_t)M.strip.nlong;
+  if (M.strip.on) return spmv_long_rows(M);
   return (size_t)(M.pipe.nlong > M.plan.nlong ? M.pipe.nlong : M.plan.nlong);
 }
 

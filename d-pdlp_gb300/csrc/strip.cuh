@@ -7,7 +7,8 @@
 //
 // The upload orders the rows of A and of A^T (the constraints and the
 // variables) by decreasing length, stably, and the solve works in that order
-// throughout; only its inputs and results are permuted.  Then
+// throughout; only its inputs and results are permuted (the layout is SELL-C-sigma,
+// Kreutzer et al. 2014, with slices of 32 and all rows sorted).  Then
 //   * rows of at most kStripRow non-zeros form strips of 32 consecutive rows
 //     of (nearly) one length, stored element-major: element k of the strip's
 //     rows is 32 consecutive columns and values.  A warp takes a strip, a
@@ -41,7 +42,7 @@
 // by the lengths of all rows, so that one long row changes nothing for the
 // others): a row's elements are folded in segments that end at
 // fixed distances from the start of the row's tile of that kernel's plan, and
-// the segments are added in order.  StripHost::sums holds, per row, the
+// the segments are added in order.  StripPlan::sums holds, per row, the
 // segment length and the row's phase in it, or the number of lanes that the
 // kernel strides a long row with.
 #pragma once
@@ -783,7 +784,7 @@ __device__ __forceinline__ void strip_block_partials(const double (&acc)[NA], do
 // Bound by FP64 issue (16 cycles per warp instruction and SM) and by the
 // gathers' L2 requests.  20M non-zeros, ms per launch inside a solve, before (the
 // faster of the CSR kernels), with a block's warps far apart in the list, and
-// now: power-law primal step 0.155, 0.147, 0.120 (FP32 0.106, 0.123, 0.102), dual
+// now: power-law primal step 0.155, 0.147, 0.120 (FP32 0.106, 0.123, 0.105), dual
 // step 0.128, 0.089, 0.084 (FP32 0.104, 0.057, 0.051); transport primal step
 // 0.185, 0.206, 0.204 (FP32 0.132, 0.118, 0.118), dual step 0.108, 0.112, 0.096
 // (FP32 0.084, 0.104, 0.074).  5 blocks per SM: 6 spill more (FP32 power-law

@@ -155,9 +155,9 @@ class TeamTurn {
 };
 
 // CTAs of the team for an LP's matrices; 0: no team.  A matrix with a front (rows
-// of more than 256 entries) has none: its items and their sums need a barrier
-// more per product and leave most warps of a team idle (an LP with such rows:
-// 25 ms against 17 ms with a kernel per product).  Nor has one with more than
+// of more than 256 entries) has none: its items have not been tried in a team as
+// it is (an earlier one, with a barrier of their own for their sums, took 25 ms on
+// a small LP of long rows, against 17 with a kernel per product).  Nor has one with more than
 // two strips for a warp: the barriers no longer show beside the strips, but every
 // CTA folds every strip's partial sums itself.  FP64, 600 iterations with set-up,
 // team and single launches: 65k x 22k with 2 entries a row 15.1 and 17.2 ms, 131k

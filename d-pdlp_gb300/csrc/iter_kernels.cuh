@@ -468,6 +468,12 @@ void launch_spmv(const DevCsrT<V> &M, const Epi &epi, double *part, double *lpar
               <<<M.strip.grid, kThreads, 0, st>>>(strip_mat(M), part, lpart, epi);
           return;
         }
+      if constexpr (has_preload<Epi>::value && sizeof(typename Epi::val_t) == 4 && !P)
+        if (M.strip.nwide == 0) {
+          spmv_strip<Epi, S, P, false, false>
+              <<<M.strip.grid, kThreads, 0, st>>>(strip_mat(M), part, lpart, epi);
+          return;
+        }
       spmv_strip<Epi, S, P><<<M.strip.grid, kThreads, 0, st>>>(strip_mat(M), part, lpart, epi);
     };
     using Yes = std::true_type;

@@ -795,7 +795,9 @@ __device__ __forceinline__ void strip_block_partials(const double (&acc)[NA], do
 // blocks fit an SM, and their vectors' loads are what such a step is: transport
 // primal step 0.204 -> 0.201 ms (6 blocks 0.207), FP32 0.118 -> 0.096, FP32
 // matrix 0.218 -> 0.181 (before the strips 0.185, 0.132 and 0.201).
-template <class Epi, bool STREAM, bool PAIR, bool NARROW = false>
+// WIDE: the matrix has wide strips; without them the plain FP32 kernels are spared
+// their code, which takes registers from the other rows'.
+template <class Epi, bool STREAM, bool PAIR, bool NARROW = false, bool WIDE = !NARROW>
 __global__ void __launch_bounds__(kThreads, NARROW ? 8
                                             : sizeof(typename Epi::val_t) == 8 || !PAIR ? 5
                                                                                         : 6)
@@ -829,7 +831,7 @@ __global__ void __launch_bounds__(kThreads, NARROW ? 8
     if (i >= A.p.nitem) {
       StripHead<M> head;
       strip_head<STREAM>(A, i - A.p.nitem, head);
-      strip_rows<STREAM, PAIR>(A, epi, acc, i - A.p.nitem, head);
+      strip_rows<STREAM, PAIR, false, WIDE>(A, epi, acc, i - A.p.nitem, head);
       return;
     }
     strip_front<STREAM, PAIR>(A, epi, acc, i, [&](int at, const int4 &b, double sum) {

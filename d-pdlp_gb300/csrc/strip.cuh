@@ -784,7 +784,7 @@ __device__ __forceinline__ void strip_block_partials(const double (&acc)[NA], do
 // Bound by FP64 issue (16 cycles per warp instruction and SM) and by the
 // gathers' L2 requests.  20M non-zeros, ms per launch inside a solve, before (the
 // faster of the CSR kernels), with a block's warps far apart in the list, and
-// now: power-law primal step 0.155, 0.147, 0.120 (FP32 0.106, 0.123, 0.105), dual
+// now: power-law primal step 0.155, 0.147, 0.120 (FP32 0.106, 0.123, 0.107), dual
 // step 0.128, 0.089, 0.084 (FP32 0.104, 0.057, 0.051); transport primal step
 // 0.185, 0.206, 0.204 (FP32 0.132, 0.118, 0.118), dual step 0.108, 0.112, 0.096
 // (FP32 0.084, 0.104, 0.074).  5 blocks per SM: 6 spill more (FP32 power-law
@@ -795,12 +795,19 @@ __device__ __forceinline__ void strip_block_partials(const double (&acc)[NA], do
 // blocks fit an SM, and their vectors' loads are what such a step is: transport
 // primal step 0.204 -> 0.201 ms (6 blocks 0.207), FP32 0.118 -> 0.096, FP32
 // matrix 0.218 -> 0.181 (before the strips 0.185, 0.132 and 0.201).
+// Blocks per SM the kernel's registers must allow.  Plain FP32 with wide strips
+// spills 200 bytes at 5: 4 where the matrix stays in L2 (3M power-law non-zeros, FP32
+// primal step 33 -> 24 us), 5 where it streams from HBM (20M: 107 us, 110 at 4).
+template <bool FP64, bool STREAM, bool PAIR, bool NARROW, bool WIDE>
+constexpr int strip_blocks() {
+  return NARROW ? 8 : FP64 ? 5 : PAIR ? 6 : WIDE && !STREAM ? 4 : 5;
+}
+
 // WIDE: the matrix has wide strips; without them the plain FP32 kernels are spared
 // their code, which takes registers from the other rows'.
 template <class Epi, bool STREAM, bool PAIR, bool NARROW = false, bool WIDE = !NARROW>
-__global__ void __launch_bounds__(kThreads, NARROW ? 8
-                                            : sizeof(typename Epi::val_t) == 8 || !PAIR ? 5
-                                                                                        : 6)
+__global__ void __launch_bounds__(
+    kThreads, (strip_blocks<sizeof(typename Epi::val_t) == 8, STREAM, PAIR, NARROW, WIDE>()))
     spmv_strip(const __grid_constant__ StripMat<typename Epi::val_t> A,
                double *__restrict__ part, double *__restrict__ lpart, Epi epi) {
   using M = typename Epi::val_t;
